@@ -5,7 +5,7 @@
 // thread per bunch refits its mesh and writes its arguments on the device, one pass
 // deposits every bunch into its own quad grid, then each group of bunches with the same
 // grid shape is solved by the batched pipeline (Green spectra of all members from batched
-// corner blocks and even/odd line transforms; the stacked FFT passes with the members as
+// cell integrals and even/odd line transforms; the stacked FFT passes with the members as
 // extra rows, planes and columns) on one of four streams, and one pass interpolates E for
 // every particle.  Nothing in the step waits for the host, so a call whose signature
 // (grids, particle counts and offsets, pointers, options) repeats replays the step as one
@@ -66,7 +66,7 @@ int check_bunches(osc_ctx *ctx, int nb, const osc_bunch *bs, const double *x, co
 // ---- one FP32 batched step, issued without host synchronisation -----------------------
 // The host fills each bunch's mesh and charge into pinned staging (BunchIn); the step copies
 // it to the device, computes the bounding boxes and charges, and k_batch_setup refits the
-// meshes and writes every bunch's deposit, gather and Green-corner arguments on the device,
+// meshes and writes every bunch's deposit and gather arguments and its cell geometry on the device,
 // so nothing in the step waits for the host: the whole step can be captured in one CUDA
 // graph.  The results come back through pinned staging (BunchOut, counters).
 
@@ -77,21 +77,21 @@ struct BunchOut {
     double stats[8];  // bounding box (xmin, xmax, ymin, ymax, zmin, zmax), non-finite, sum q
     double min[3], max[3], delta[3], charge;
 };
-// Static placement of a bunch: its first corner block (component 1) in the batch's corner
-// array, the members of its group (blocks of one component), its grid.
+// Static placement of a bunch: its geometry in the batch's array (members of a group are
+// adjacent), its grid.
 struct BunchMap {
-    int ca0, cstride;
+    int geom;
     int n[3], nlo[3], nhi[3];
     int64_t np;
 };
 
-// Mesh refit (apply_refit), deposit / gather arguments (deposit_args, interp_args) and Green
-// corner arguments (green_corner_args with zero offset) of every bunch, with every product,
+// Mesh refit (apply_refit), deposit / gather arguments (deposit_args, interp_args) and the
+// cell geometry of the Green function of every bunch, with every product,
 // sum and quotient rounded separately as the host evaluates them, so the meshes and
 // arguments are bit-identical to those of a single step.
 __global__ void k_batch_setup(int nb, const BunchMap *__restrict__ map, const BunchIn *__restrict__ in,
                               const double *__restrict__ stats, int resize, int has_q, BunchArgs *ba,
-                              CornerArgs *ca, BunchOut *out) {
+                              CellGeom *cg, BunchOut *out) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     const BunchMap m = map[b];
@@ -134,25 +134,11 @@ __global__ void k_batch_setup(int nb, const BunchMap *__restrict__ map, const Bu
         ia.delta[d] = dl[d];
         ia.hinv[d] = __ddiv_rn(1.0, dl[d]);
     }
-    const double dz = __dmul_rn(dl[2], bi.gamma);
-    const double vol = __dmul_rn(__dmul_rn(dl[0], dl[1]), dz);
-    for (int comp = 1; comp <= 3; ++comp) {
-        CornerArgs &c = ca[m.ca0 + (comp - 1) * m.cstride];
-        c.cdx = m.n[0] + 1;
-        c.cdy = m.n[1] + 1;
-        c.cdz = m.n[2] + 1;
-        c.c0x = m.n[0] - 1;
-        c.c0y = m.n[1] - 1;
-        c.c0z = m.n[2] - 1;
-        c.dx = dl[0];
-        c.dy = dl[1];
-        c.dz = dz;
-        c.factor = (comp == 1 || comp == 2) ? __ddiv_rn(bi.gamma, vol) : __ddiv_rn(1.0, vol);
-        c.umin = __dadd_rn(__dmul_rn((double)__fsub_rn(0.5f, (float)m.n[0]), dl[0]), 0.0);
-        c.vmin = __dadd_rn(__dmul_rn((double)__fsub_rn(0.5f, (float)m.n[1]), dl[1]), 0.0);
-        c.wmin = __dadd_rn(__dmul_rn((double)__fsub_rn(0.5f, (float)m.n[2]), dz), __dmul_rn(0.0, bi.gamma));
-        c.icomp = comp;
-    }
+    CellGeom &g = cg[m.geom];
+    g.hx = dl[0];
+    g.hy = dl[1];
+    g.hz = __dmul_rn(dl[2], bi.gamma);
+    g.gamma = bi.gamma;
     BunchOut &o = out[b];
     for (int i = 0; i < 8; ++i) o.stats[i] = st[i];
     for (int d = 0; d < 3; ++d) {
@@ -170,12 +156,12 @@ struct BatchPlan {
     std::string key;
     int nb = 0, njobs = 0, resize = 0, has_q = 0;
     int64_t nodes = 0;
-    size_t max_f = 0, max_g = 0;
+    size_t max_g = 0;
     std::vector<Group> groups;
     std::vector<int> slot_of;      // auxiliary stream slot of each group
-    std::vector<size_t> ca_off;    // first corner block of each group
+    std::vector<size_t> geom_off;  // first cell geometry of each group
     std::vector<int> issue_order;  // groups, largest first
-    DevBuf d_ba, d_jobs, d_job0, d_ca, d_map, d_in, d_out;
+    DevBuf d_ba, d_jobs, d_job0, d_geom, d_map, d_in, d_out;
     BunchIn *h_in = nullptr;
     BunchOut *h_out = nullptr;
     unsigned long long *h_cnt = nullptr;
@@ -185,7 +171,7 @@ struct BatchPlan {
     int64_t step_launches = 0;  // kernels of one step, counted while capturing
     ~BatchPlan() {
         if (exec) cudaGraphExecDestroy(exec);
-        for (DevBuf *b : {&d_ba, &d_jobs, &d_job0, &d_ca, &d_map, &d_in, &d_out})
+        for (DevBuf *b : {&d_ba, &d_jobs, &d_job0, &d_geom, &d_map, &d_in, &d_out})
             if (b->p) cudaFree(b->p);
         if (h_in) cudaFreeHost(h_in);
         if (h_out) cudaFreeHost(h_out);
@@ -252,12 +238,12 @@ int make_plan(osc_ctx *ctx, BatchPlan &P, int nb, const osc_bunch *bs, const dou
     std::vector<BunchArgs> ba(nb);
     std::memset(ba.data(), 0, sizeof(BunchArgs) * nb);
     std::vector<BunchMap> map(nb);
-    size_t nca = 0;
+    size_t ngeom = 0;
     for (Group &g : P.groups) {
         const int64_t N = (int64_t)g.n[0] * g.n[1] * g.n[2];
         const int B = (int)g.members.size();
         g.node0 = P.nodes;
-        P.ca_off.push_back(nca);
+        P.geom_off.push_back(ngeom);
         for (int i = 0; i < B; ++i) {
             const int b = g.members[i];
             const int64_t o = bs[b].offset;
@@ -268,8 +254,7 @@ int make_plan(osc_ctx *ctx, BatchPlan &P, int nb, const osc_bunch *bs, const dou
             ba[b].node_off = P.nodes + (int64_t)i * N;
             ba[b].E = E + 3 * o;
             BunchMap &m = map[b];
-            m.ca0 = (int)(nca + i);
-            m.cstride = B;
+            m.geom = (int)(ngeom + i);
             for (int d = 0; d < 3; ++d) {
                 m.n[d] = g.n[d];
                 m.nlo[d] = bs[b].mesh.nlo[d];
@@ -277,14 +262,13 @@ int make_plan(osc_ctx *ctx, BatchPlan &P, int nb, const osc_bunch *bs, const dou
             }
             m.np = bs[b].np;
         }
-        nca += 3 * (size_t)B;
+        ngeom += (size_t)B;
         P.nodes += N * B;
-        P.max_f = std::max(P.max_f, 3 * (size_t)B * (g.n[0] + 1) * (g.n[1] + 1) * (g.n[2] + 1));
         const int zp = green_zpitch(g.n[2] + 1, sizeof(float));
         P.max_g = std::max(P.max_g, 3 * (size_t)B * (g.n[0] + 1) * (g.n[1] + 1) * zp);
     }
     // largest groups first, each on the stream with the least work queued so far, so the
-    // streams finish together (cost ~ members x corner-block nodes)
+    // streams finish together (cost ~ members x kernel nodes)
     auto gcost = [](const Group &g) {
         return (double)g.members.size() * (g.n[0] + 1) * (double)(g.n[1] + 1) * (double)(g.n[2] + 1);
     };
@@ -303,7 +287,7 @@ int make_plan(osc_ctx *ctx, BatchPlan &P, int nb, const osc_bunch *bs, const dou
     TRY(dev_alloc(ctx, P.d_ba, sizeof(BunchArgs) * nb));
     TRY(dev_alloc(ctx, P.d_jobs, sizeof(BatchJob) * jobs.size()));
     TRY(dev_alloc(ctx, P.d_job0, sizeof(int) * job0.size()));
-    TRY(dev_alloc(ctx, P.d_ca, sizeof(CornerArgs) * nca));
+    TRY(dev_alloc(ctx, P.d_geom, sizeof(CellGeom) * ngeom));
     TRY(dev_alloc(ctx, P.d_map, sizeof(BunchMap) * nb));
     TRY(dev_alloc(ctx, P.d_in, sizeof(BunchIn) * nb));
     TRY(dev_alloc(ctx, P.d_out, sizeof(BunchOut) * nb));
@@ -341,10 +325,9 @@ int batch_workspaces(osc_ctx *ctx, const BatchPlan &P) {
         TRY(ws_get(ctx, "fs_x2", sizeof(float2) * x2, &p));
         TRY(ws_get(ctx, "fs_x3", sizeof(float2) * x3, &p));
         TRY(ws_get(ctx, "fs_x4", sizeof(float2) * x4, &p));
-        TRY(ws_get(ctx, "green_h", sizeof(double) * h, &p));
-        TRY(ws_get(ctx, "green_hx", sizeof(double) * hx, &p));
-        TRY(ws_get(ctx, "green_hy", sizeof(double) * hy, &p));
-        TRY(ws_get(ctx, "batch_F", sizeof(double) * P.max_f, &p));
+        TRY(ws_get(ctx, "green_h", sizeof(float) * h, &p));
+        TRY(ws_get(ctx, "green_hx", sizeof(float) * hx, &p));
+        TRY(ws_get(ctx, "green_hy", sizeof(float) * hy, &p));
         TRY(ws_get(ctx, "batch_green", sizeof(float) * P.max_g, &p));
     }
     TRY(ws_get(ctx, "batch_keys", sizeof(unsigned long long) * 7 * (size_t)std::max(P.njobs, 1), &p));
@@ -362,7 +345,7 @@ int batch_issue(osc_ctx *ctx, BatchPlan &P) {
     const int nb = P.nb;
     BunchArgs *d_ba = reinterpret_cast<BunchArgs *>(P.d_ba.p);
     const BatchJob *d_jobs = reinterpret_cast<const BatchJob *>(P.d_jobs.p);
-    CornerArgs *d_ca = reinterpret_cast<CornerArgs *>(P.d_ca.p);
+    CellGeom *d_geom = reinterpret_cast<CellGeom *>(P.d_geom.p);
     unsigned long long *keys, *cnt;
     double *qsum, *stats;
     float *quad, *e8;
@@ -382,11 +365,12 @@ int batch_issue(osc_ctx *ctx, BatchPlan &P) {
             return set_err(ctx, OSC_E_CUDA, "batch stats");
     }
     {
-        Launch L_(ctx, "batch_setup");
+        Launch L_(ctx, "batch_setup", 2);
         k_batch_setup<<<(nb + 127) / 128, 128, 0, ctx->stream>>>(
             nb, reinterpret_cast<const BunchMap *>(P.d_map.p), reinterpret_cast<const BunchIn *>(P.d_in.p), stats,
-            P.resize, P.has_q, d_ba, d_ca, reinterpret_cast<BunchOut *>(P.d_out.p));
+            P.resize, P.has_q, d_ba, d_geom, reinterpret_cast<BunchOut *>(P.d_out.p));
         CK(cudaGetLastError(), "batch setup");
+        if (launch_cell_series(d_geom, nb, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "batch cell series");
     }
     // deposit every bunch into its quad grid
     CK(cudaMemsetAsync(quad, 0, sizeof(float) * 4 * (size_t)P.nodes, ctx->stream), "memset quad");
@@ -403,25 +387,32 @@ int batch_issue(osc_ctx *ctx, BatchPlan &P) {
     for (int gi : P.issue_order) {
         const Group &g = P.groups[gi];
         SlotGuard sg(ctx, P.slot_of[gi]);
-        float *gbuf;
-        double *F;
-        TRY(ws_get(ctx, "batch_F", sizeof(double) * P.max_f, (void **)&F));
+        float *gbuf, *h;
         TRY(ws_get(ctx, "batch_green", sizeof(float) * P.max_g, (void **)&gbuf));
         const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
         const int B = (int)g.members.size();
         const int zinner = zconv_warp_ok(2 * nz, nz, 4) ? 1 : 0;
         const int zp = zinner ? green_zpitch(nz + 1, sizeof(float)) : nz + 1;
         const int64_t per = (int64_t)(nx + 1) * (ny + 1) * zp;
-        const int64_t fstride = (int64_t)(nx + 1) * (ny + 1) * (nz + 1);
+        TRY(ws_get(ctx, "green_h", sizeof(float) * 3 * (size_t)B * nx * ny * nz, (void **)&h));
         if (zinner) CK(cudaMemsetAsync(gbuf, 0, sizeof(float) * 3 * B * per, ctx->stream), "memset spectra");
         // Green spectra of the three E components of every member: members m = comp*B + i
         {
-            Launch L_(ctx, "green_corners");
-            if (launch_igf_corners_batch(F, d_ca + P.ca_off[gi], 3 * B, fstride, fstride, ctx->stream))
-                return set_err(ctx, OSC_E_CUDA, "batch corners");
+            CellArgs ca;
+            ca.nx = nx;
+            ca.ny = ny;
+            ca.nz = nz;
+            ca.zwrap = 0;
+            ca.ncomp = 3;
+            for (int q = 0; q < 3; ++q) ca.comps[q] = q + 1;
+            ca.nmem = B;
+            ca.hstride = (int64_t)nx * ny * nz;
+            Launch L_(ctx, "green_cells");
+            if (launch_green_cells_batch(h, ca, d_geom + P.geom_off[gi], ctx->stream))
+                return set_err(ctx, OSC_E_CUDA, "batch cells");
         }
         const int odd[3][2] = {{0, B}, {B, 2 * B}, {2 * B, 3 * B}};
-        TRY(green_sym_lines3<float>(ctx, F, 3 * B, nx, ny, nz, odd, zinner, zp, gbuf, per));
+        TRY(green_sym_lines3<float>(ctx, h, 3 * B, nx, ny, nz, odd, zinner, zp, gbuf, per));
         GSpecDev spec[3];
         for (int comp = 1; comp <= 3; ++comp) {
             GSpecDev &s = spec[comp - 1];

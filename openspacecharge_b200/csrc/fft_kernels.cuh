@@ -157,12 +157,12 @@ struct SymArgs {
     FFTPlan p;  // length L = 2n
     int n;
     int odd_lo, odd_hi;  // members b in [odd_lo, odd_hi) are odd (par -1), the others even
-    int64_t nlines;
+    int nb;              // members
     int nq;
     int64_t in_ps, in_qs, in_es;
     int64_t out_ps, out_qs, out_es;
     double scale;
-    // batches: lines of member b are the lines [b*npq, (b+1)*npq), offset by b*in_bs, b*out_bs
+    // npq lines per member, member b's offset by b*in_bs, b*out_bs
     int64_t npq, in_bs, out_bs;
     int nl_div = 0;  // autotuner: 2 or 4 divides the line pairs per CTA of a static engine
 };

@@ -560,11 +560,12 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
     const int64_t r0 = (int64_t)blockIdx.x * (2 * NL);
     const int n = a.n;
     for (int t = tid; t < 2 * NL; t += nthreads) {  // line start offsets, once per line
-        const int64_t r = r0 + t;
+        // members start on even lines, so that no two of them (phi and E differ by orders of
+        // magnitude) share a complex line
+        const int64_t r = r0 + t, npq2 = (a.npq + 1) & ~(int64_t)1, bi = r / npq2, rl = r - bi * npq2;
         int64_t oi = -1, oo = -1;
         int odd = 0;
-        if (r < a.nlines) {
-            const int64_t bi = r / a.npq, rl = r - bi * a.npq;
+        if (bi < a.nb && rl < a.npq) {
             const int64_t pi = rl / a.nq, qi = rl - pi * a.nq;
             oi = bi * a.in_bs + pi * a.in_ps + qi * a.in_qs;
             oo = bi * a.out_bs + pi * a.out_ps + qi * a.out_qs;
@@ -1034,7 +1035,7 @@ int launch_sym_lines(const TI *in, TO *out, const SymArgs &a, const TwPair<cplx<
             const int nt = fft_threads(L, NL, E::kEPT);
             if (nt < 1 || nt > E::kMaxThreads || (L * NL) % E::kEPT) return OSC_E_FFT_SIZE;
             const size_t sm = sizeof(cplx<TC>) * ((size_t)L + (size_t)L * (NL + 1));
-            const unsigned nblk = (unsigned)ceil_div(a.nlines, 2 * NL);
+            const unsigned nblk = (unsigned)ceil_div(((a.npq + 1) & ~(int64_t)1) * a.nb, 2 * NL);
             auto go = [&](auto kern) -> int {
                 int rc = set_smem(kern, sm);
                 if (rc) return rc;

@@ -1,5 +1,4 @@
 // grid_kernels.cu -- Green-function construction (FP64) and grid elementwise kernels.
-#include <algorithm>
 #include "grid_kernels.cuh"
 #include "osc_igf.cuh"
 
@@ -102,106 +101,6 @@ __global__ void k_green_center(const double *__restrict__ F, double2 *__restrict
 int launch_green_center(const double *F, double2 *cg, const CenterArgs &a, cudaStream_t st) {
     const int64_t n = (int64_t)8 * a.nx * a.ny * a.nz;
     k_green_center<<<nblocks(n, 256), 256, 0, st>>>(F, cg, a);
-    return ok();
-}
-
-// Octant of the centred kernel for all-symmetric geometries: h[c][b][a] = g at displacement
-// (a, b, c) >= 0, the 8-corner difference of the cell whose corners are a, a+1 (the corner
-// block starts at index n-1 of the doubled grid, so cell a uses corners a and a+1).
-template <typename TH>
-__global__ void k_green_octant(const double *__restrict__ F, TH *__restrict__ h, int nx, int ny, int nz) {
-    const int cdx = nx + 1, cdy = ny + 1;
-    const int n = nx * ny * nz;  // one member's octant (< 2^31 nodes)
-    F += blockIdx.y * ((int64_t)cdx * cdy * (nz + 1));  // batch member
-    h += blockIdx.y * (int64_t)n;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const int i = idx % nx, r = idx / nx;
-        const int j = r % ny, k = r / ny;
-        const double *f0 = F + i + cdx * (j + cdy * k);
-        const int sy = cdx, sz = cdx * cdy;
-        double g = +f0[1 + sy + sz];
-        g = g - f0[sy + sz];
-        g = g - f0[1 + sz];
-        g = g - f0[1 + sy];
-        g = g - f0[0];
-        g = g + f0[sz];
-        g = g + f0[sy];
-        g = g + f0[1];
-        h[idx] = (TH)g;
-    }
-}
-template <typename TH>
-int launch_green_octant(const double *F, TH *h, int nx, int ny, int nz, int nbatch, cudaStream_t st) {
-    const dim3 grid(nblocks((int64_t)nx * ny * nz, 256), (unsigned)nbatch);
-    k_green_octant<TH><<<grid, 256, 0, st>>>(F, h, nx, ny, nz);
-    return ok();
-}
-template int launch_green_octant<double>(const double *, double *, int, int, int, int, cudaStream_t);
-template int launch_green_octant<float>(const double *, float *, int, int, int, int, cudaStream_t);
-
-// Corner blocks of several geometries: member blockIdx.y uses args[blockIdx.y] and writes
-// F + blockIdx.y * fstride.
-__global__ void k_igf_corners_batch(double *__restrict__ F, const CornerArgs *__restrict__ args, int64_t fstride) {
-    const CornerArgs a = args[blockIdx.y];
-    F += blockIdx.y * fstride;
-    const int64_t n = (int64_t)a.cdx * a.cdy * a.cdz;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    auto at = [&](int64_t idx) {
-        const int cx = (int)(idx % a.cdx);
-        const int64_t r = idx / a.cdx;
-        const int cy = (int)(r % a.cdy);
-        const int cz = (int)(r / a.cdy);
-        const double u = (a.c0x + cx) * a.dx + a.umin;
-        const double v = (a.c0y + cy) * a.dy + a.vmin;
-        const double w = (a.c0z + cz) * a.dz + a.wmin;
-        return igf_primitive(a.icomp, u, v, w) * a.factor;
-    };
-    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 2 * stride) {
-        const int64_t i1 = i0 + stride;  // two points per thread and trip, as k_igf_corners_set
-        const double f0 = at(i0);
-        const double f1 = i1 < n ? at(i1) : 0.0;
-        F[i0] = f0;
-        if (i1 < n) F[i1] = f1;
-    }
-}
-__global__ void k_igf_corners_set(double *__restrict__ F, CornerSet s, int64_t fstride) {
-    const CornerArgs a = s.a[blockIdx.y];
-    F += blockIdx.y * fstride;
-    const int64_t n = (int64_t)a.cdx * a.cdy * a.cdz;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    auto at = [&](int64_t idx) {
-        const int cx = (int)(idx % a.cdx);
-        const int64_t r = idx / a.cdx;
-        const int cy = (int)(r % a.cdy);
-        const int cz = (int)(r / a.cdy);
-        const double u = (a.c0x + cx) * a.dx + a.umin;
-        const double v = (a.c0y + cy) * a.dy + a.vmin;
-        const double w = (a.c0z + cz) * a.dz + a.wmin;
-        return igf_primitive(a.icomp, u, v, w) * a.factor;
-    };
-    // two points per thread and trip: the two dependency chains of log/atan evaluations
-    // interleave
-    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 2 * stride) {
-        const int64_t i1 = i0 + stride;
-        const double f0 = at(i0);
-        const double f1 = i1 < n ? at(i1) : 0.0;
-        F[i0] = f0;
-        if (i1 < n) F[i1] = f1;
-    }
-}
-int launch_igf_corners_set(double *F, const CornerSet &s, int64_t fstride, cudaStream_t st) {
-    if (s.n < 1 || s.n > 4) return 1;
-    int64_t npts = 0;
-    for (int i = 0; i < s.n; ++i) npts = std::max(npts, (int64_t)s.a[i].cdx * s.a[i].cdy * s.a[i].cdz);
-    const dim3 grid(nblocks((npts + 1) / 2, 256), (unsigned)s.n);  // two points per thread
-    k_igf_corners_set<<<grid, 256, 0, st>>>(F, s, fstride);
-    return ok();
-}
-
-int launch_igf_corners_batch(double *F, const CornerArgs *args_dev, int nbatch, int64_t fstride, int64_t npts,
-                             cudaStream_t st) {
-    const dim3 grid(nblocks((npts + 1) / 2, 256), (unsigned)nbatch);  // two points per thread
-    k_igf_corners_batch<<<grid, 256, 0, st>>>(F, args_dev, fstride);
     return ok();
 }
 

@@ -16,13 +16,6 @@ struct CornerArgs {
     int icomp;
 };
 int launch_igf_corners(double *F, const CornerArgs &a, cudaStream_t st);
-// Corner blocks of up to four components of one geometry in one launch (arguments by
-// value): component i writes F + i * fstride, a[i] cdx*cdy*cdz points each.
-struct CornerSet {
-    CornerArgs a[4];
-    int n;
-};
-int launch_igf_corners_set(double *F, const CornerSet &s, int64_t fstride, cudaStream_t st);
 
 // Reference layout: cgrn(i,j,k) = 8-corner difference for i<N-1.., raw corner value on the
 // last faces, as complex128 over the full (Nx,Ny,Nz) grid (code/open_spacecharge_mod.f90:697-705).
@@ -38,16 +31,6 @@ struct CenterArgs {
     int c0x, c0y, c0z, cdx, cdy;
 };
 int launch_green_center(const double *F, double2 *cg, const CenterArgs &a, cudaStream_t st);
-
-// All-symmetric geometries: the non-negative octant h[c][b][a] (a < nx, b < ny, c < nz) of
-// the centred kernel from corners F of extent (n+1) per axis starting at index n-1.
-// nbatch members: corner blocks (n+1)^3 apart in F, octants n^3 apart in h.
-// h = the 8-corner differences of F (FP64), rounded once to TH.
-template <typename TH>
-int launch_green_octant(const double *F, TH *h, int nx, int ny, int nz, int nbatch, cudaStream_t st);
-// Corner blocks of nbatch geometries (args_dev: device array), fstride apart, npts each.
-int launch_igf_corners_batch(double *F, const CornerArgs *args_dev, int nbatch, int64_t fstride, int64_t npts,
-                             cudaStream_t st);
 
 // Stored half-spectrum extraction: kx in [0,nx], ky in [0,dimy), kz in [0,dimz), times scale;
 // layout [kz][ky][kx], or [ky][kx][kz] with columns zpitch elements apart when zpitch > 0

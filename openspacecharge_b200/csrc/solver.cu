@@ -99,28 +99,22 @@ CornerArgs green_corner_args(const int n[3], const double delta[3], double gamma
 }
 
 // ------------------------------------------------------------------------------------
-// Stored spectra of all-symmetric kernels (offset 0 on every axis) of nb geometries with
-// equal grids, from their corner blocks F ((n+1)^3 apart): octant differences, then even/
-// odd transforms along x, y and z; the last pass applies fpei/M and writes the stored
+// Stored spectra of all-symmetric kernels (offset 0 on every axis) of nb members with equal
+// grids, from their cell integrals h ([z][y][x] each, nx*ny*nz apart): even/odd transforms
+// along x, y and z; the last pass applies fpei/M and writes the stored
 // layout (zinner: [ky][kx][kz] with columns zpitch apart, else [kz][ky][kx]) of member b at
 // out + b * out_bstride.  Equals the extraction of the FP64 doubled-grid FFT
 // (osc_get_cgrn_freespace + ccfft3d, code/open_spacecharge_mod.f90:633-705,
-// code/fft_interface_mod.f90:96-143) up to rounding.  The corner primitives and their
-// 8-corner differences, whose log/atan terms cancel catastrophically at large offsets,
-// are always FP64; the line transforms run in T: FP64 for FP64 spectra, FP32 (from the
-// octant values rounded once) for the FP32 path, whose stored spectrum is FP32 anyway.
+// code/fft_interface_mod.f90:96-143) up to rounding.  The cell integrals are FP64, rounded
+// once to T; the line transforms run in T: FP64 for FP64 spectra, FP32 for the FP32 path,
+// whose stored spectrum is FP32 anyway.
 template <typename T>
-int green_sym_lines3(osc_ctx *c, const double *F, int nb, int nx, int ny, int nz, const int odd[3][2], int zinner,
+int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, const int odd[3][2], int zinner,
                      int zpitch, T *out, int64_t out_bstride) {
     const int nxh = nx + 1, nyh = ny + 1;
-    T *h, *hx, *hy;
-    TRY(ws_get(c, "green_h", sizeof(T) * (size_t)nb * nx * ny * nz, (void **)&h));
+    T *hx, *hy;
     TRY(ws_get(c, "green_hx", sizeof(T) * (size_t)nb * nxh * ny * nz, (void **)&hx));
     TRY(ws_get(c, "green_hy", sizeof(T) * (size_t)nb * nxh * nyh * nz, (void **)&hy));
-    {
-        Launch L_(c, "green_octant");
-        TRY(kerr(c, launch_green_octant<T>(F, h, nx, ny, nz, nb, c->stream), "green octant"));
-    }
     FFTPlan px, py, pz;
     if (!make_fft_plan(2 * nx, px) || !make_fft_plan(2 * ny, py) || !make_fft_plan(2 * nz, pz))
         return set_err(c, OSC_E_FFT_SIZE, "doubled grid lengths must be 2^a 3^b 5^c");
@@ -133,7 +127,7 @@ int green_sym_lines3(osc_ctx *c, const double *F, int nb, int nx, int ny, int nz
     const std::string tp = sizeof(T) == 4 ? "f32" : "f64";
     // x: rows h[c][b][0..nx) -> hx[c][b][0..nx]
     a.p = px; a.n = nx; a.odd_lo = odd[0][0]; a.odd_hi = odd[0][1]; a.nq = ny;
-    a.npq = (int64_t)ny * nz; a.nlines = nb * a.npq;
+    a.npq = (int64_t)ny * nz; a.nb = nb;
     a.in_ps = (int64_t)ny * nx; a.in_qs = nx; a.in_es = 1; a.in_bs = (int64_t)nx * ny * nz;
     a.out_ps = (int64_t)ny * nxh; a.out_qs = nxh; a.out_es = 1; a.out_bs = (int64_t)nxh * ny * nz;
     a.scale = 1.0;
@@ -141,14 +135,14 @@ int green_sym_lines3(osc_ctx *c, const double *F, int nb, int nx, int ny, int nz
     TRY(kerr(c, launch_sym_lines<T, T, T>(h, hx, a, twx, true, true, c->stream), "green x"));
     // y: lines (c, kx) of hx -> hy[c][ky][kx]
     a.p = py; a.n = ny; a.odd_lo = odd[1][0]; a.odd_hi = odd[1][1]; a.nq = nxh;
-    a.npq = (int64_t)nz * nxh; a.nlines = nb * a.npq;
+    a.npq = (int64_t)nz * nxh; a.nb = nb;
     a.in_ps = (int64_t)ny * nxh; a.in_qs = 1; a.in_es = nxh; a.in_bs = (int64_t)nxh * ny * nz;
     a.out_ps = (int64_t)nyh * nxh; a.out_qs = 1; a.out_es = nxh; a.out_bs = (int64_t)nxh * nyh * nz;
     a.nl_div = tune_get(c, "sym_nl_div:" + tp + ":L" + std::to_string(2 * ny));
     TRY(kerr(c, launch_sym_lines<T, T, T>(hx, hy, a, twy, false, false, c->stream), "green y"));
     // z: lines (ky, kx) of hy -> stored spectrum, scaled by fpei/M
     a.p = pz; a.n = nz; a.odd_lo = odd[2][0]; a.odd_hi = odd[2][1]; a.nq = nxh;
-    a.npq = (int64_t)nyh * nxh; a.nlines = nb * a.npq;
+    a.npq = (int64_t)nyh * nxh; a.nb = nb;
     a.in_ps = nxh; a.in_qs = 1; a.in_es = (int64_t)nyh * nxh; a.in_bs = (int64_t)nxh * nyh * nz;
     if (zinner) {
         a.out_ps = (int64_t)nxh * zpitch; a.out_qs = zpitch; a.out_es = 1;
@@ -161,30 +155,35 @@ int green_sym_lines3(osc_ctx *c, const double *F, int nb, int nx, int ny, int nz
     TRY(kerr(c, launch_sym_lines<T, T, T>(hy, out, a, twz, false, zinner != 0, c->stream), "green z"));
     return OSC_OK;
 }
-template int green_sym_lines3<float>(osc_ctx *, const double *, int, int, int, int, const int (*)[2], int, int,
+template int green_sym_lines3<float>(osc_ctx *, const float *, int, int, int, int, const int (*)[2], int, int,
                                      float *, int64_t);
 template int green_sym_lines3<double>(osc_ctx *, const double *, int, int, int, int, const int (*)[2], int, int,
                                       double *, int64_t);
 
 // All components of a geometry with zero offset (even or odd along every axis) at once:
-// the corner blocks of every component in one launch, then the octant differences and the
+// the cell integrals of every component in one launch, then the
 // three even/odd line passes with the components as batch members (per axis, the member of
 // that axis' E component is the odd one); one buffer holds the stored spectra of all
 // components, in gs.buf[0], and gs.spec[i] points at component comps[i].
 template <typename T>
 static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[3], double gamma, const int *comps,
                          int ncomp, GreenSet &gs) {
-    const int n[3] = {nx, ny, nz};
-    const double off0[3] = {0.0, 0.0, 0.0};
-    const int64_t fstride = (int64_t)(nx + 1) * (ny + 1) * (nz + 1);
-    double *F;
-    TRY(ws_get(c, "green_F", sizeof(double) * (size_t)ncomp * fstride, (void **)&F));
-    CornerSet cs;
-    cs.n = ncomp;
-    for (int i = 0; i < ncomp; ++i) cs.a[i] = green_corner_args(n, delta, gamma, off0, comps[i]);
+    T *h;
+    TRY(ws_get(c, "green_h", sizeof(T) * (size_t)ncomp * nx * ny * nz, (void **)&h));
     {
-        Launch L_(c, "green_corners");
-        TRY(kerr(c, launch_igf_corners_set(F, cs, fstride, c->stream), "green corners"));
+        CellArgs ca;
+        ca.nx = nx;
+        ca.ny = ny;
+        ca.nz = nz;
+        ca.zwrap = 0;
+        ca.ncomp = ncomp;
+        for (int i = 0; i < ncomp; ++i) ca.comps[i] = comps[i];
+        ca.nmem = 1;
+        ca.hstride = (int64_t)nx * ny * nz;
+        Launch L_(c, "green_cells");
+        TRY(kerr(c, launch_green_cells<T>(h, ca, cell_geom(delta[0], delta[1], delta[2] * gamma, gamma, 0.0,
+                                                           kSerRatio), c->stream),
+                 "green cells"));
     }
     const int zinner = zconv_warp_ok(2 * nz, nz, (int)sizeof(T)) ? 1 : 0;
     const int zp = zinner ? green_zpitch(nz + 1, sizeof(T)) : nz + 1;
@@ -198,7 +197,7 @@ static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[
             odd[comps[i] - 1][1] = i + 1;
         }
     int rc = zinner ? cuda_check(c, cudaMemsetAsync(store.p, 0, store.bytes, c->stream), "memset spectra") : OSC_OK;
-    if (!rc) rc = green_sym_lines3<T>(c, F, ncomp, nx, ny, nz, odd, zinner, zp, reinterpret_cast<T *>(store.p), per);
+    if (!rc) rc = green_sym_lines3<T>(c, h, ncomp, nx, ny, nz, odd, zinner, zp, reinterpret_cast<T *>(store.p), per);
     if (rc) {
         green_release(c, store);
         return rc;

@@ -3,6 +3,7 @@
 
 #include "../../include/opensc_gpu.h"
 #include "context.cuh"
+#include "green_cells.cuh"
 #include "grid_kernels.cuh"
 #include "particle_kernels.cuh"
 
@@ -62,11 +63,11 @@ struct FreeSpaceJob {
 
 // Corner block arguments of the IGF primitive of component icomp (0 phi, 1..3 E).
 CornerArgs green_corner_args(const int n[3], const double delta[3], double gamma, const double off[3], int icomp);
-// Stored spectra of all-symmetric kernels of nb members with equal grids from their corner
-// blocks F ((n+1)^3 each, corner index n-1 first): member b written at out + b*out_bstride.
+// Stored spectra of all-symmetric kernels of nb members with equal grids from their cell
+// integrals h (nx*ny*nz each): member b written at out + b*out_bstride.
 // Along axis d the members in [odd[d][0], odd[d][1]) are odd, the others even.
 template <typename T>
-int green_sym_lines3(osc_ctx *c, const double *F, int nb, int nx, int ny, int nz, const int odd[3][2], int zinner,
+int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, const int odd[3][2], int zinner,
                      int zpitch, T *out, int64_t out_bstride);
 
 // Optimised IGF convolution (cached half-spectra, pruned transforms) in precision T.
