@@ -3,7 +3,8 @@
 Every ``csrc/*.cu`` file is compiled by ``nvcc -gencode arch=compute_100a,code=sm_100a
 -lineinfo -O3`` into an object under ``_build/`` and the objects are linked into
 ``openspacecharge_b200/libopensc_b200.so`` in the source tree, so the library travels with
-the repository snapshot.  Objects are rebuilt when their source or any header is newer.
+the repository snapshot.  Objects are rebuilt when their source or a header that it includes
+(nvcc's dependency file) is newer.
 
 Usage: ``python -m openspacecharge_b200.build [--force] [--jobs N] [--verbose]``.
 """
@@ -46,26 +47,31 @@ def _host_cxx() -> list[str]:
     return []
 
 
-def _newest_header() -> float:
+def _newest_input(src: str, dep: str) -> float:
+    """Newest of the source and the project headers its dependency file names (all headers
+    when there is no dependency file)."""
     hdrs = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
-    return max((os.path.getmtime(h) for h in hdrs), default=0.0)
+    if os.path.exists(dep):
+        with open(dep) as f:
+            named = {os.path.realpath(t) for t in f.read().replace("\\\n", " ").split()}
+        hdrs = [h for h in hdrs if os.path.realpath(h) in named] or hdrs  # of this tree, not a copy's
+    return max(os.path.getmtime(p) for p in [src] + hdrs)
 
 
 def build(force: bool = False, jobs: int = 8, verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     nvcc = _nvcc()
-    hdr_t = _newest_header()
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     objs, todo = [], []
     for src in sources:
         obj = os.path.join(BUILD, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
-        if force or not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(src), hdr_t):
+        if force or not os.path.exists(obj) or os.path.getmtime(obj) < _newest_input(src, obj[:-2] + ".d"):
             todo.append((src, obj))
 
     def compile_one(so):
         src, obj = so
-        cmd = [nvcc] + _host_cxx() + NVCC_FLAGS + ["-c", src, "-o", obj]
+        cmd = [nvcc] + _host_cxx() + NVCC_FLAGS + ["-MD", "-MF", obj[:-2] + ".d", "-c", src, "-o", obj]
         if verbose:
             cmd += ["-Xptxas", "-v"]
         r = subprocess.run(cmd, capture_output=True, text=True)

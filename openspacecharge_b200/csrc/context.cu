@@ -112,8 +112,8 @@ template <typename T> static std::vector<cplx<T>> stage_table(int L, const int *
     return h;
 }
 
-// Keys of the table map: L runtime table, -L static-engine stages, L + kWarpKey warp-engine
-// stages (a null entry when the length has no such engine).
+// Keys of the table map: L whole circle, -L static-engine or runtime-plan stages, L + kWarpKey
+// warp-engine stages (a null entry when the length has no such engine).
 static constexpr int kWarpKey = 1 << 20;
 
 template <typename T> int twiddles(osc_ctx *c, int L, TwPair<cplx<T>> *out) {
@@ -132,6 +132,8 @@ template <typename T> int twiddles(osc_ctx *c, int L, TwPair<cplx<T>> *out) {
         if (rc) return rc;
         tab[L] = b;
     }
+    FFTPlan plan;
+    if (!make_fft_plan(L, plan)) return set_err(c, OSC_E_FFT_SIZE, "FFT length %d unsupported", L);
     for (int which = 0; which < 2; ++which) {
         const int key = which == 0 ? -L : L + kWarpKey;
         if (tab.find(key) != tab.end()) continue;
@@ -139,6 +141,7 @@ template <typename T> int twiddles(osc_ctx *c, int L, TwPair<cplx<T>> *out) {
         auto make = [&](auto eng) -> int {
             using E = decltype(eng);
             if constexpr (E::kLen > 0) h = stage_table<T>(L, E::kRad, E::kNst);
+            else if (which == 0) h = stage_table<T>(L, plan.radix, plan.nst);
             return 0;
         };
         if (which == 0) dispatch_fft_len<T>(L, make);

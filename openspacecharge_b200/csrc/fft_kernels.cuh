@@ -188,6 +188,6 @@ bool zconv_warp_ok(int L, int nz, int elem_bytes);
 bool zconv_img_ok(int L, int nz, int elem_bytes);
 template <typename T>
 int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPair<cplx<T>> &tw,
-                 int nl, cudaStream_t st);
+                 cudaStream_t st);
 
 }  // namespace osc

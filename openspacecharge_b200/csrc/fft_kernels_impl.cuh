@@ -23,40 +23,17 @@
 
 namespace osc {
 
-#ifdef OSC_FFT_DEFINE_PLAN
-bool make_fft_plan(int L, FFTPlan &p) {
-    if (L < 2 || L > FFT_MAX_LEN || (L % 2) != 0) return false;
-    p.L = L;
-    p.nst = 0;
-    int m = L;
-    while (m % 8 == 0) { p.radix[p.nst++] = 8; m /= 8; }
-    while (m % 4 == 0) { p.radix[p.nst++] = 4; m /= 4; }
-    while (m % 2 == 0) { p.radix[p.nst++] = 2; m /= 2; }
-    while (m % 3 == 0) { p.radix[p.nst++] = 3; m /= 3; }
-    while (m % 5 == 0) { p.radix[p.nst++] = 5; m /= 5; }
-    return m == 1 && p.nst <= FFT_MAX_STAGES;
-}
-// The warp-per-column z pass (FP32 and FP64) for the lengths of the warp registry.
-bool zconv_warp_ok(int L, int nz, int elem_bytes) {
-    if ((elem_bytes != 4 && elem_bytes != 8) || 2 * nz != L) return false;
-    return dispatch_warp_len(L, [](auto eng) -> int { return decltype(eng)::kLen > 0 ? 1 : 0; }) != 0;
-}
-bool zconv_img_ok(int L, int nz, int elem_bytes) {
-    if (!zconv_warp_ok(L, nz, elem_bytes)) return false;
-    return dispatch_warp_len(L, [](auto eng) -> int {
-               using E = decltype(eng);
-               if constexpr (E::kLen > 0) {
-                   constexpr int nb = E::kLen / E::kRad[0];
-                   return nb % 32 == 0 || nb < 32 ? 1 : 0;
-               }
-               return 0;
-           }) != 0;
-}
-#endif
+// Line buffers of a kernel that transforms in shared memory (FftRuntime alternates between two).
+template <class E> constexpr int eng_bufs() { return E::kLen > 0 ? 1 : 2; }
 
-// Engine-specific twiddle table in global memory.
-template <class E, typename V> __host__ __device__ inline const V *eng_tw(const TwPair<V> &t) {
-    return E::kLen > 0 ? t.st : t.rt;
+// f(row, e) for e < len of rows [0, nrows): whole warps walk a row, so that no index is divided
+// by a length known only at run time.
+template <class F> __device__ __forceinline__ void for_rows(int nrows, int len, F &&f) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll 2
+    for (int r = threadIdx.x >> 5; r < nrows; r += nw)
+#pragma unroll 2
+        for (int e = lane; e < len; e += 32) f(r, e);
 }
 
 // ------------------------------------------------------------------------------------
@@ -81,6 +58,27 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_lines(const cplx<T> *in, cpl
         __syncthreads();
         const bool flip = (a.flip_mask >> blockIdx.z) & 1u;
         const T sc = (T)a.scale;
+        if constexpr (E::kLen == 0) {
+            // a thread stays on one line: its pointers once, flat or plane by plane
+            const int l0 = tid % NL;
+            int pl = a.flat_lines > 0 ? col0 / a.ncols : (int)blockIdx.y, c = a.flat_lines > 0 ? col0 - pl * a.ncols + l0 : col0 + l0;
+            const bool live = a.flat_lines > 0 ? col0 + l0 < a.flat_lines : c < a.ncols;
+            if (a.flat_lines > 0 && c >= a.ncols) {
+                c -= a.ncols;
+                ++pl;
+            }
+            const V *sp = in + (int64_t)blockIdx.z * a.in_zstride + (int64_t)pl * a.in_pstride + (int64_t)c * a.in_cstride;
+            V *dp = out + (int64_t)blockIdx.z * a.out_zstride + (int64_t)pl * a.out_pstride + (int64_t)c * a.out_cstride;
+            auto ld = [&](int e, int) -> V {
+                return live && e < a.in_len ? sp[(int64_t)e * a.in_estride] : mk<T>(0, 0);
+            };
+            auto st = [&](int p, int, const V &v) {
+                const int e = (flip && p > 0 ? L - p : p) - a.out_lo;
+                if (live && e >= 0 && e < a.out_len) dp[(int64_t)e * a.out_estride] = cscale(v, sc);
+            };
+            E::template run_io<V, NL, false, false>(buf, a.p, tw, a.sign, ld, st);
+            return;
+        }
         if (a.flat_lines > 0) {
             // tile over the flat line sequence: line col0 + l is column (c0 + l) of plane pl0,
             // or column (c0 + l - ncols) of plane pl0 + 1 (NL <= ncols, so at most one wrap)
@@ -121,45 +119,40 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_lines(const cplx<T> *in, cpl
         E::template run_io<V, NL, MODE == 1, MODE == 2>(buf, a.p, tw, a.sign, ld, st);
         return;
     }
-    // the static first stage skips the zero half (MODE 1 launches only with in_len == L/2)
-    const int ld_len = (E::kLen > 0 && MODE == 1) ? E::kLen / 2 : L;
-    const int nld = NL * ld_len;
-    for (int idx = tid; idx < nld; idx += nthreads) {
-        int e, c;
-        if (ROW) { c = idx / ld_len; e = idx - c * ld_len; }
-        else { e = idx / NL; c = idx - e * NL; }
+    // rows (blocks of contiguous lines); every element of a line is loaded, zeros past in_len
+    static_assert(!ROW || E::kLen * NL / E::kEPT % 32 == 0, "for_rows needs whole warps");
+    auto put = [&](int c, int e) {
         V v = mk<T>(0, 0);
         const int col = col0 + c;
         if (e < a.in_len && col < a.ncols) v = src[(int64_t)col * a.in_cstride + (int64_t)e * a.in_estride];
         buf[e * lstr + c] = v;
-    }
+    };
+    if constexpr (E::kLen > 0)
+        for (int idx = tid; idx < NL * E::kLen; idx += nthreads) put(idx / E::kLen, idx % E::kLen);
+    else
+        for_rows(NL, L, put);
     __syncthreads();
-    E::template run<V, NL, MODE == 1, MODE == 2>(buf, a.p, tw, a.sign);
-    const int nst = NL * a.out_len;
+    const V *res = E::template run<V, NL, false, false>(buf, a.p, tw, a.sign);
     const T sc = (T)a.scale;
-    for (int idx = tid; idx < nst; idx += nthreads) {
-        int e, c;
-        if (ROW) { c = idx / a.out_len; e = idx - c * a.out_len; }
-        else { e = idx / NL; c = idx - e * NL; }
+    for_rows(NL, a.out_len, [&](int c, int e) {
         const int col = col0 + c;
-        const int src_e = ((a.flip_mask >> blockIdx.z) & 1u) ? (L - (e + a.out_lo)) % L : e + a.out_lo;
+        const int p = e + a.out_lo, src_e = ((a.flip_mask >> blockIdx.z) & 1u) && p > 0 ? L - p : p;
         if (col < a.ncols)
-            dst[(int64_t)col * a.out_cstride + (int64_t)e * a.out_estride] = cscale(buf[src_e * lstr + c], sc);
-    }
+            dst[(int64_t)col * a.out_cstride + (int64_t)e * a.out_estride] = cscale(res[src_e * lstr + c], sc);
+    });
 }
 
 // ------------------------------------------------------------------------------------
-// Element e of real input row `row` (row < nrows, e < nin).
+// Element e of the real input row at p (jn: a quad-grid row with a y neighbour below it).
 template <typename TIn>
-__device__ __forceinline__ TIn r2c_in(const TIn *__restrict__ in, const R2CArgs &a, int64_t row, int e) {
-    return in[row * a.in_rstride + e];
+__device__ __forceinline__ TIn r2c_in(const TIn *__restrict__ p, const R2CArgs &, bool, int e) {
+    return p[e];
 }
 // Quad-grid input of the FP32 deposit: node (i,j) of a plane is the sum of the four
 // contributions held at (i,j).x, (i-1,j).y, (i,j-1).z and (i-1,j-1).w, added in that
 // fixed order (the order of k_quad_to_nodes, so rho is the same to the bit).
-__device__ __forceinline__ float r2c_in(const float4 *__restrict__ in, const R2CArgs &a, int64_t row, int e) {
-    const float4 *q = in + row * a.in_rstride + e;
-    const bool jn = (row % a.qny) > 0;
+__device__ __forceinline__ float r2c_in(const float4 *__restrict__ p, const R2CArgs &a, bool jn, int e) {
+    const float4 *q = p + e;
     float s = __ldg(&q->x);
     if (e > 0) s += __ldg(&q[-1].y);
     if (jn) s += __ldg(&q[-a.in_rstride].z);
@@ -185,8 +178,18 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
     // static engines launch with L*NL/E::kEPT threads: compile-time trip counts below
     const int nthreads = E::kLen ? E::kLen * NL / E::kEPT : (int)blockDim.x, tid = threadIdx.x;
     const int64_t row0 = (int64_t)blockIdx.x * (2 * NL);
+    // whether a quad-grid row has a y neighbour: one division per row, not per element
+    __shared__ bool jns[2 * NL];
+    if (std::is_same<TIn, float4>::value) {
+        for (int t = tid; t < 2 * NL; t += nthreads) jns[t] = (row0 + t) % a.qny > 0;
+        __syncthreads();
+    }
     load_twiddles(tw, twg, L);
-    const int ld_len = (E::kLen > 0 && HIN) ? E::kLen / 2 : L;  // HIN launches only with nin == L/2
+    auto elem = [&](int rr, int e) -> T {
+        const int64_t row = row0 + rr;
+        if (row >= a.nrows || e >= a.nin) return (T)0;
+        return (T)r2c_in(in + row * a.in_rstride, a, std::is_same<TIn, float4>::value ? jns[rr] : false, e);
+    };
     if constexpr (E::kLen > 0) {
         // all of a thread's loads are issued before any is stored to shared memory
         constexpr int LDL = HIN ? E::kLen / 2 : E::kLen, NT = E::kLen * NL / E::kEPT;
@@ -195,9 +198,8 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
             const int idx = tid + it * NT, rr = idx / LDL, e = idx - rr * LDL;
-            const int64_t row = row0 + rr;
             v[it] = 0;
-            if (idx < 2 * NL * LDL && row < a.nrows && e < a.nin) v[it] = (T)r2c_in(in, a, row, e);
+            if (idx < 2 * NL * LDL) v[it] = elem(rr, e);
         }
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
@@ -205,25 +207,18 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
             if (idx < 2 * NL * LDL) reinterpret_cast<T *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = v[it];
         }
     } else {
-        for (int idx = tid; idx < 2 * NL * ld_len; idx += nthreads) {
-            const int rr = idx / ld_len, e = idx - rr * ld_len;
-            const int64_t row = row0 + rr;
-            T v = 0;
-            if (row < a.nrows && e < a.nin) v = (T)r2c_in(in, a, row, e);
-            T *slot = reinterpret_cast<T *>(&buf[e * lstr + (rr >> 1)]);
-            slot[rr & 1] = v;
-        }
+        for_rows(2 * NL, L, [&](int rr, int e) {
+            reinterpret_cast<T *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = elem(rr, e);
+        });
     }
     __syncthreads();
-    E::template run<V, NL, HIN, false>(buf, a.p, tw, +1);
-    const int nh = L / 2 + 1;
-    for (int idx = tid; idx < 2 * NL * nh; idx += nthreads) {
-        const int rr = idx / nh, k = idx - rr * nh;
+    const V *res = E::template run<V, NL, HIN, false>(buf, a.p, tw, +1);
+    auto put = [&](int rr, int k) {
         const int64_t row = row0 + rr;
-        if (row >= a.nrows) continue;
+        if (row >= a.nrows) return;
         const int line = rr >> 1;
-        const V Z = buf[k * lstr + line];
-        const V Zm = buf[((L - k) % L) * lstr + line];
+        const V Z = res[k * lstr + line];
+        const V Zm = res[(k > 0 ? L - k : 0) * lstr + line];
         V r;
         if ((rr & 1) == 0) {  // (Z + conj Zm)/2
             r.x = (T)0.5 * (Z.x + Zm.x);
@@ -233,6 +228,12 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
             r.y = (T)0.5 * (Zm.x - Z.x);
         }
         out[row * a.out_rstride + k] = r;
+    };
+    if constexpr (E::kLen > 0) {
+        constexpr int nh = E::kLen / 2 + 1;
+        for (int idx = tid; idx < 2 * NL * nh; idx += nthreads) put(idx / nh, idx % nh);
+    } else {
+        for_rows(2 * NL, L / 2 + 1, put);
     }
 }
 
@@ -294,7 +295,8 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
     const int nthreads = blockDim.x, tid = threadIdx.x;
     const int64_t row0 = (int64_t)blockIdx.x * (2 * NL);
     const int half = L / 2;
-    T *res = reinterpret_cast<T *>(buf + L * lstr);  // [3][2*NL][nout] when a.e8 is set
+    static_assert(E::kLen * NL / E::kEPT % 32 == 0, "for_rows needs whole warps");
+    T *res = reinterpret_cast<T *>(buf + eng_bufs<E>() * L * lstr);  // [3][2*NL][nout] when a.e8 is set
     __shared__ int64_t rin[2 * NL], rout[2 * NL];
     for (int t = tid; t < 2 * NL; t += nthreads) row_bases(a, row0 + t, rin[t], rout[t]);
     const int64_t ies = a.zin ? a.zin_nz : 1;
@@ -302,15 +304,7 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
     __syncthreads();
     for (int c = 0; c < a.ncomp; ++c) {
         const V *src = in + (int64_t)c * a.in_cstride;
-        for (int idx = tid; idx < NL * L; idx += nthreads) {
-            int line, k;
-            if (a.zin) {  // adjacent lines (adjacent z) fastest for the kz-innermost spectra
-                k = idx / NL;
-                line = idx - k * NL;
-            } else {
-                line = idx / L;
-                k = idx - line * L;
-            }
+        auto put = [&](int line, int k) {
             const int64_t ra = row0 + 2 * line, rb = ra + 1;
             const int kk = k <= half ? k : L - k;
             V A = mk<T>(0, 0), B = mk<T>(0, 0);
@@ -319,15 +313,18 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
             if (k == 0 || k == half) { A.y = 0; B.y = 0; }
             if (k > half) { A.y = -A.y; B.y = -B.y; }
             buf[k * lstr + line] = mk<T>(A.x - B.y, A.y + B.x);
-        }
+        };
+        if (a.zin)  // adjacent lines (adjacent z) fastest for the kz-innermost spectra
+            for (int idx = tid; idx < NL * L; idx += nthreads) put(idx % NL, idx / NL);
+        else
+            for_rows(NL, L, put);
         __syncthreads();
-        E::template run<V, NL, false, HOUT>(buf, a.p, tw, -1);
-        for (int idx = tid; idx < 2 * NL * a.nout; idx += nthreads) {
-            const int rr = idx / a.nout, x = idx - rr * a.nout;
+        const V *fb = E::template run<V, NL, false, HOUT>(buf, a.p, tw, -1);
+        for_rows(2 * NL, a.nout, [&](int rr, int x) {
             const int64_t row = row0 + rr;
-            if (row >= a.nrows) continue;
-            const int xs = ((a.flip_mask >> c) & 1u) ? (L - x) % L : x;
-            const V z = buf[xs * lstr + (rr >> 1)];
+            if (row >= a.nrows) return;
+            const int xs = ((a.flip_mask >> c) & 1u) && x > 0 ? L - x : x;
+            const V z = fb[xs * lstr + (rr >> 1)];
             const T val = (rr & 1) ? z.y : z.x;
             const int64_t gidx = rout[rr] * a.nout + x;
             for (int d = 0; d < a.ndest[c]; ++d) write_dest<T>(a.dest[c][d], gidx, x, val);
@@ -336,17 +333,16 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
                 for (int q = 0; q < 3; ++q)
                     if (a.e8_comp[q] == c) res[(q * 2 * NL + rr) * a.nout + x] = val;
             }
-        }
+        });
         __syncthreads();
     }
     if (a.e8) {
         // x-pair grid rows: node n gets (E(n), E(n+1)), the row's last node (E(n), 0)
         typedef vec4<T> V4;
         V4 *g = reinterpret_cast<V4 *>(a.e8);
-        for (int idx = tid; idx < 2 * NL * a.nout; idx += nthreads) {
-            const int rr = idx / a.nout, x = idx - rr * a.nout;
+        for_rows(2 * NL, a.nout, [&](int rr, int x) {
             const int64_t row = row0 + rr;
-            if (row >= a.nrows) continue;
+            if (row >= a.nrows) return;
             const int64_t gidx = rout[rr] * a.nout + x;
             const T *r0 = res + rr * a.nout + x;
             const int64_t cs = (int64_t)2 * NL * a.nout;
@@ -369,67 +365,100 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
                 g[2 * gidx] = lo;
                 g[2 * gidx + 1] = hi;
             }
-        }
+        });
     }
 }
 
 // ------------------------------------------------------------------------------------
-// HALF: nz == L/2, so the static engine's forward first stage skips the zero half and
-// its inverse last stage skips the upper half, which is never stored.  The forward
-// transform reads the column straight from global memory into its first stage; each
-// inverse transform computes its input (spectrum times Green spectrum, plus the image term)
-// inside its first stage and writes its last stage straight to global memory.
-template <typename T, int NL, class E, bool HALF>
-__global__ void __launch_bounds__(E::kMaxThreads) k_zconv(const cplx<T> *__restrict__ in, cplx<T> *__restrict__ out,
-                                                          ZConvArgs a, const cplx<T> *__restrict__ twg,
-                                                          const cplx<T> *__restrict__ tw_rt) {
+// One (kx, ky) column of a stored Green spectrum: g_lookup with everything that does not depend
+// on kz worked out once.
+template <typename T> struct GColumn {
+    const void *p;
+    int64_t zs;
+    bool realv, iu, symz, neg, zneg;
+    __device__ __forceinline__ GColumn(const GSpecDev &g, int kx, int ky, int nxh, int Ny, int ny, int64_t goff) {
+        const bool my = g.sym_y && ky > ny;
+        const int yy = my ? Ny - ky : ky;
+        realv = g.real_valued;
+        iu = g.imag_unit;
+        symz = g.sym_z;
+        neg = my && g.par_y < 0;
+        zneg = g.par_z < 0;
+        const int64_t at = goff + (int64_t)yy * nxh + kx;
+        zs = (int64_t)g.dimy * nxh;
+        p = realv ? (const void *)(reinterpret_cast<const T *>(g.data) + at)
+                  : (const void *)(reinterpret_cast<const cplx<T> *>(g.data) + at);
+    }
+    __device__ __forceinline__ cplx<T> times(const cplx<T> &x, int kz, int Nz, int nz) const {
+        const bool mz = symz && kz > nz;
+        const int64_t at = (int64_t)(mz ? Nz - kz : kz) * zs;
+        const bool sg = neg != (mz && zneg);
+        if (realv) {
+            T s = __ldg(reinterpret_cast<const T *>(p) + at);
+            if (sg) s = -s;
+            return iu ? mk<T>(-x.y * s, x.x * s) : mk<T>(x.x * s, x.y * s);
+        }
+        cplx<T> v = __ldg(reinterpret_cast<const cplx<T> *>(p) + at);
+        if (sg) { v.x = -v.x; v.y = -v.y; }
+        return cmul(x, v);
+    }
+};
+
+// The z pass of the lengths without a warp engine, NL columns per CTA on the runtime-plan
+// engine.  The forward transform reads its columns straight from global memory into its first
+// stage; each inverse transform forms its input (spectrum times Green spectrum, plus the image
+// term) inside its first stage and writes its last stage straight to global memory.  A thread
+// stays on one column, whose Green column and pointers it works out once.
+template <typename T, int NL>
+__global__ void __launch_bounds__(FftRuntime::kMaxThreads) k_zconv(const cplx<T> *__restrict__ in, cplx<T> *__restrict__ out,
+                                                                   ZConvArgs a, const cplx<T> *__restrict__ twg,
+                                                                   const cplx<T> *__restrict__ tw_rt) {
     typedef cplx<T> V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     V *tw = reinterpret_cast<V *>(smem_raw);
-    const int L = E::kLen ? E::kLen : a.p.L;
+    const int L = a.p.L;
     V *rhat = tw + L;
     constexpr int lstr = NL + 1;
     V *buf = rhat + L * lstr;
-    const int col0 = blockIdx.x * NL;
-    in += blockIdx.y * a.in_bstride;
-    out += blockIdx.y * a.out_bstride;
+    const int l0 = threadIdx.x % NL, col = blockIdx.x * NL + l0, colc = min(col, a.ncols - 1);
+    const bool live = col < a.ncols;
+    const int ky = colc / a.nxh, kx = colc - ky * a.nxh;
+    in += blockIdx.y * a.in_bstride + colc;
+    out += blockIdx.y * a.out_bstride + (int64_t)colc * a.out_colstride;
     const int64_t goff = blockIdx.y * a.g_bstride;
     load_twiddles(tw, twg, L);
     __syncthreads();
-    auto ld_in = [&](int e, int l) -> V {
-        const int col = col0 + l;
-        V v = mk<T>(0, 0);
-        if (e < a.nz && col < a.ncols) v = in[(int64_t)e * a.in_estride + col];
-        return v;
-    };
+    auto ld_in = [&](int e, int) -> V { return live && e < a.nz ? in[(int64_t)e * a.in_estride] : mk<T>(0, 0); };
     auto st_rhat = [&](int e, int l, const V &v) { rhat[e * lstr + l] = v; };
-    E::template run_io<V, NL, HALF, false>(rhat, a.p, tw, +1, ld_in, st_rhat);
+    FftRuntime::template run_io<V, NL, false, false>(buf, a.p, tw, +1, ld_in, st_rhat);
     for (int o = 0; o < a.nout; ++o) {
         const int gd = a.gdir[o], gi = a.gimg[o];
-        const T icoef = (T)a.img_coef[o];
-        auto ld_mul = [&](int e, int l) -> V {
-            const int col = min(col0 + l, a.ncols - 1);
-            const int ky = col / a.nxh, kx = col - ky * a.nxh;
-            V S = mk<T>(0, 0);
-            if (gd >= 0)
-                S = cmul(rhat[e * lstr + l], g_lookup<T>(a.g[gd], kx, ky, e, a.nxh, a.Ny, a.ny, L, a.nz, goff));
-            if (gi >= 0) {
+        const GColumn<T> cd(a.g[gd >= 0 ? gd : 0], kx, ky, a.nxh, a.Ny, a.ny, goff);
+        V *dst = out + (int64_t)o * a.out_cstride;
+        auto st_out = [&](int e, int, const V &v) {
+            if (e < a.nz && live) dst[(int64_t)e * a.out_estride] = v;
+        };
+        if (gi < 0) {
+            auto ld_mul = [&](int e, int l) -> V {
+                return gd >= 0 ? cd.times(rhat[e * lstr + l], e, L, a.nz) : mk<T>(0, 0);
+            };
+            FftRuntime::template run_io<V, NL, false, false>(buf, a.p, tw, -1, ld_mul, st_out);
+        } else {
+            const GColumn<T> ci(a.g[gi], kx, ky, a.nxh, a.Ny, a.ny, goff);
+            const T icoef = (T)a.img_coef[o];
+            auto ld_mul = [&](int e, int l) -> V {
+                V S = gd >= 0 ? cd.times(rhat[e * lstr + l], e, L, a.nz) : mk<T>(0, 0);
                 // spectrum of -rho flipped in z: -w^((nz-1) kz) * rho_hat(-kz)
-                const V rm = rhat[((L - e) % L) * lstr + l];
-                const V ph = __ldg(tw_rt + (int)(((int64_t)a.img_phase_mul * e) % L));
+                const V rm = rhat[(e > 0 ? L - e : 0) * lstr + l];
+                // (nz-1)*kz < 2^21: 32-bit index arithmetic
+                const V ph = __ldg(tw_rt + (int)(((unsigned)a.img_phase_mul * (unsigned)e) % (unsigned)L));
                 V ri = cmul(ph, rm);
                 ri.x = -ri.x * icoef;
                 ri.y = -ri.y * icoef;
-                S = cadd(S, cmul(ri, g_lookup<T>(a.g[gi], kx, ky, e, a.nxh, a.Ny, a.ny, L, a.nz, goff)));
-            }
-            return S;
-        };
-        V *dst = out + (int64_t)o * a.out_cstride;
-        auto st_out = [&](int e, int l, const V &v) {
-            const int col = col0 + l;
-            if (e < a.nz && col < a.ncols) dst[(int64_t)e * a.out_estride + (int64_t)col * a.out_colstride] = v;
-        };
-        E::template run_io<V, NL, false, HALF>(buf, a.p, tw, -1, ld_mul, st_out);
+                return cadd(S, ci.times(ri, e, L, a.nz));
+            };
+            FftRuntime::template run_io<V, NL, false, false>(buf, a.p, tw, -1, ld_mul, st_out);
+        }
     }
 }
 
@@ -542,6 +571,61 @@ __global__ void __launch_bounds__(E::kLen * 3 * NLC / E::kEPT, sizeof(T) == 4 ? 
     }
 }
 
+// The same on the runtime-plan engine, for the lengths without a static one.
+template <typename T, int NLC>
+__global__ void __launch_bounds__(FftRuntime::kMaxThreads) k_c2r_e8_rt(const cplx<T> *__restrict__ in, C2RArgs a,
+                                                                       const cplx<T> *__restrict__ twg) {
+    typedef cplx<T> V;
+    constexpr int NLT = 3 * NLC, lstr = NLT + 1;
+    const int L = a.p.L, half = L / 2, nout = half;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V *tw = reinterpret_cast<V *>(smem_raw);
+    V *buf = tw + L;
+    const int tid = threadIdx.x;
+    const int64_t row0 = (int64_t)blockIdx.x * (2 * NLC);
+    __shared__ int64_t rin[2 * NLC], rout[2 * NLC];
+    for (int t = tid; t < 2 * NLC; t += blockDim.x) row_bases(a, row0 + t, rin[t], rout[t]);
+    const int64_t ies = a.zin ? a.zin_nz : 1;
+    load_twiddles(tw, twg, L);
+    __syncthreads();
+    auto put = [&](int ln, int k) {  // ln = c * NLC + line
+        const int c = ln / NLC, line = ln - c * NLC;
+        const V *src = in + (int64_t)a.e8_comp[c] * a.in_cstride;
+        const int64_t ra = row0 + 2 * line, rb = ra + 1;
+        V A = mk<T>(0, 0), B = mk<T>(0, 0);
+        if (ra < a.nrows) A = src[rin[2 * line] + k * ies];
+        if (rb < a.nrows) B = src[rin[2 * line + 1] + k * ies];
+        if (k == 0 || k == half) { A.y = 0; B.y = 0; }
+        buf[k * lstr + ln] = mk<T>(A.x - B.y, A.y + B.x);
+        if (k > 0 && k < half) buf[(L - k) * lstr + ln] = mk<T>(A.x + B.y, B.x - A.y);
+    };
+    if (a.zin)
+#pragma unroll 4
+        for (int idx = tid; idx < NLT * (half + 1); idx += blockDim.x) put(idx % NLT, idx / NLT);
+    else
+        for_rows(NLT, half + 1, put);
+    __syncthreads();
+    const V *res = FftRuntime::template run<V, NLT, false, true>(buf, a.p, tw, -1);
+    for_rows(2 * NLC, nout, [&](int rr, int x) {
+        const int64_t row = row0 + rr;
+        if (row >= a.nrows) return;
+        const int ln = rr >> 1;
+        const bool odd = rr & 1;
+        T e0[3], e1[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const V z0 = res[x * lstr + c * NLC + ln], z1 = res[(x + 1) * lstr + c * NLC + ln];
+            e0[c] = odd ? z0.y : z0.x;
+            e1[c] = x + 1 < nout ? (odd ? z1.y : z1.x) : (T)0;
+        }
+        if constexpr (sizeof(T) == 4)
+            st_pair(reinterpret_cast<float4 *>(a.e8) + 2 * (rout[rr] * nout + x),
+                    make_float4(e0[0], e0[1], e0[2], 0.f), make_float4(e1[0], e1[1], e1[2], 0.f));
+        else
+            st_node(reinterpret_cast<double4 *>(a.e8) + rout[rr] * nout + x, e0[0], e0[1], e0[2]);
+    });
+}
+
 // Even/odd real line transforms (Green spectra): two real lines per complex line, the
 // parity extension formed in the load, the halves separated after the transform.  TC is
 // the arithmetic type (and that of the twiddles), TI the input's, TO the output's.
@@ -610,39 +694,41 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
             }
         }
     } else {
-        for (int idx = tid; idx < 2 * NL * L; idx += nthreads) {
-            int rr, e;
-            if (LDE) { rr = idx / L; e = idx - rr * L; }
-            else { e = idx / (2 * NL); rr = idx - e * (2 * NL); }
+        // each of the n+1 distinct values is read once and written at e and at L - e
+        auto put = [&](int rr, int e) {
             const int64_t o = bin[rr];
             TC v = (TC)0;
-            if (o >= 0 && e != n) {
-                const int src = e < n ? e : L - e;
-                v = (TC)in[o + (int64_t)src * a.in_es];
-                if (e > n && podd[rr]) v = -v;
-            }
-            TC *slot = reinterpret_cast<TC *>(&buf[e * lstr + (rr >> 1)]);
-            slot[rr & 1] = v;
-        }
+            if (o >= 0 && e != n) v = (TC)in[o + (int64_t)e * a.in_es];
+            reinterpret_cast<TC *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = v;
+            if (e > 0 && e < n) reinterpret_cast<TC *>(&buf[(L - e) * lstr + (rr >> 1)])[rr & 1] = podd[rr] ? -v : v;
+        };
+        if (LDE) for_rows(2 * NL, n + 1, put);
+        else
+#pragma unroll 4
+            for (int idx = tid; idx < 2 * NL * (n + 1); idx += nthreads) put(idx % (2 * NL), idx / (2 * NL));
     }
     __syncthreads();
-    E::template run<V, NL, false, false>(buf, a.p, tw, +1);
+    const V *res = E::template run<V, NL, false, false>(buf, a.p, tw, +1);
     const int nk = n + 1;
-    for (int idx = tid; idx < 2 * NL * nk; idx += nthreads) {
-        int rr, k;
-        if (STK) { rr = idx / nk; k = idx - rr * nk; }
-        else { k = idx / (2 * NL); rr = idx - k * (2 * NL); }
+    auto fin = [&](int rr, int k) {
         const int64_t o = bout[rr];
-        if (o < 0) continue;
-        const V Z = buf[k * lstr + (rr >> 1)];
-        const V Zm = buf[((L - k) % L) * lstr + (rr >> 1)];
+        if (o < 0) return;
+        const V Z = res[k * lstr + (rr >> 1)];
+        const V Zm = res[(k > 0 ? L - k : 0) * lstr + (rr >> 1)];
         const bool odd = podd[rr];
         TC sv;
         const TC hf = (TC)0.5;
         if ((rr & 1) == 0) sv = !odd ? hf * (Z.x + Zm.x) : hf * (Z.y - Zm.y);
         else sv = !odd ? hf * (Z.y + Zm.y) : hf * (Zm.x - Z.x);
         out[o + (int64_t)k * a.out_es] = (TO)(sv * (TC)a.scale);
-    }
+    };
+    if (!STK)
+        for (int idx = tid; idx < 2 * NL * nk; idx += nthreads) fin(idx % (2 * NL), idx / (2 * NL));
+    else if constexpr (E::kLen > 0)
+        for (int idx = tid; idx < 2 * NL * (E::kLen / 2 + 1); idx += nthreads)
+            fin(idx / (E::kLen / 2 + 1), idx % (E::kLen / 2 + 1));
+    else
+        for_rows(2 * NL, nk, fin);
 }
 
 // ------------------------------------------------------------------------------------
@@ -670,40 +756,45 @@ template <typename K> inline int set_smem(K kern, size_t bytes) {
 }
 inline int launch_ok() { return cudaGetLastError() == cudaSuccess ? OSC_OK : OSC_E_CUDA; }
 
-// Runtime-engine NL: a whole number of threads, <= 256 threads, buffers within budget.
-inline int pick_nl_rt(int L, int nl_max, size_t elem, int nbuf) {
-    for (int nl = nl_max; nl >= 2; nl /= 2) {
-        if ((L * nl) % FFT_EPT != 0 || fft_threads(L, nl) > FftRuntime::kMaxThreads) continue;
-        if ((size_t)nbuf * L * (nl + 1) * elem + L * elem > 110 * 1024 && nl > 2) continue;
-        return nl;
-    }
+// Lines per CTA of a runtime-plan kernel: the widest of nl (descending) whose nbuf line buffers of
+// L (nl + 1) elements, twiddles and `extra` bytes a line leave several CTAs per SM, else the
+// widest that fits (8 at most); 0 when none does.
+inline int pick_nl_rt(int L, const int *nl, int nnl, size_t elem, int nbuf, size_t extra = 0) {
+    auto need = [&](int n) { return (size_t)nbuf * L * (n + 1) * elem + L * elem + extra * n; };
+    for (int i = 0; i < nnl; ++i)
+        if (need(nl[i]) <= 56 * 1024) return nl[i];
+    for (int i = 0; i < nnl; ++i)
+        if (nl[i] <= 8 && need(nl[i]) <= 226 * 1024) return nl[i];
     return 0;
 }
+// Threads and dynamic shared memory of a kernel on engine E with NL lines.
+template <class E> inline int eng_threads(const FFTPlan &p, int NL) {
+    return E::kLen > 0 ? fft_threads(p.L, NL, E::kEPT) : mix_threads(p, NL);
+}
+template <class E, typename T> inline size_t eng_smem(int L, int NL) {
+    return sizeof(cplx<T>) * ((size_t)L + (size_t)eng_bufs<E>() * L * (NL + 1));
+}
 
-// Calls f(std::integral_constant<int, NL>) for the engine's lines-per-CTA.  Static engines
-// use a compile-time NL: the widest that fits (one line buffer) or, for the two-buffer
-// z-pass, at most 4 lines in ~48 KB so several CTAs share an SM.
-template <typename T, class E, class F>
-inline int with_nl(int L, int nbuf, int nl_max, int nl_req, F &&f, int nl_div = 0) {
+// Calls f(std::integral_constant<int, NL>) for the engine's lines per CTA.  Static engines use a
+// compile-time NL, the widest that fits; runtime plans MAXNL, 8 or MINNL (pick_nl_rt).
+template <typename T, class E, int MAXNL, int MINNL, bool HALVES, class F>
+inline int with_nl(int L, F &&f, int nl_div = 0, size_t extra = 0) {
     if constexpr (E::kLen > 0) {
         (void)L;
-        (void)nl_req;
-        (void)nl_max;
+        (void)extra;
         constexpr int NL1 = nl_static(E::kLen, sizeof(T) == 4 ? 16 : 8, (int)sizeof(cplx<T>), 1, 100 * 1024, E::kEPT);
-        constexpr int NL2 = nl_static(E::kLen, 4, (int)sizeof(cplx<T>), 2, 64 * 1024, E::kEPT);
-        if (nbuf >= 2) return f(std::integral_constant<int, NL2>{});
         // the autotuner's alternative tile: half the lines per CTA (more, smaller CTAs)
         constexpr int NLH = NL1 >= 4 && ((E::kLen * (NL1 / 2)) % E::kEPT) == 0 ? NL1 / 2 : NL1;
-        if (nl_div == 2 && NLH != NL1) return f(std::integral_constant<int, NLH>{});
+        if constexpr (HALVES && NLH != NL1)
+            if (nl_div == 2) return f(std::integral_constant<int, NLH>{});
         return f(std::integral_constant<int, NL1>{});
     } else {
-        int nl = nl_req > 0 ? nl_req : pick_nl_rt(L, nl_max, sizeof(cplx<T>), nbuf);
-        switch (nl) {
-        case 16: return f(std::integral_constant<int, 16>{});
-        case 8: return f(std::integral_constant<int, 8>{});
-        case 4: return f(std::integral_constant<int, 4>{});
-        case 2: return f(std::integral_constant<int, 2>{});
-        default: return OSC_E_FFT_SIZE;
+        constexpr int nls[3] = {MAXNL, 8, MINNL};
+        switch (pick_nl_rt(L, nls, 3, sizeof(cplx<T>), eng_bufs<E>(), extra)) {
+        case MAXNL: return f(std::integral_constant<int, MAXNL>{});
+        case MINNL: return f(std::integral_constant<int, MINNL>{});
+        case 0: return OSC_E_FFT_SIZE;
+        default: return f(std::integral_constant<int, 8>{});
         }
     }
 }
@@ -712,9 +803,8 @@ template <typename T, int NL, bool ROW, class E, int MODE>
 inline int launch_lines_k(const cplx<T> *in, cplx<T> *out, const LineArgs &a, int nplanes, int ncomp, const cplx<T> *tw,
                           cudaStream_t st) {
     const int L = a.p.L;
-    const int nt = fft_threads(L, NL, E::kEPT);
-    if (nt < 1 || nt > E::kMaxThreads || (L * NL) % E::kEPT) return OSC_E_FFT_SIZE;
-    const size_t sm = sizeof(cplx<T>) * ((size_t)L + (size_t)L * (NL + 1));
+    const int nt = eng_threads<E>(a.p, NL);
+    const size_t sm = eng_smem<E, T>(L, NL);
     auto kern = k_lines<T, NL, ROW, E, MODE>;
     int rc = set_smem(kern, sm);
     if (rc) return rc;
@@ -734,10 +824,11 @@ int launch_lines(const cplx<T> *in, cplx<T> *out, const LineArgs &a, int nplanes
     const int L = a.p.L;
     return dispatch_fft_len<T>(L, [&](auto eng) -> int {
         using E = decltype(eng);
-        const cplx<T> *twe = eng_tw<E>(tw);
-        return with_nl<T, E>(L, 1, sizeof(T) == 4 ? 16 : 8, 0, [&](auto nlc) -> int {
+        const cplx<T> *twe = tw.st;
+        return with_nl<T, E, sizeof(T) == 4 ? 16 : 8, 2, true>(L, [&](auto nlc) -> int {
             constexpr int NL = decltype(nlc)::value;
-            if (row_mode) return launch_lines_k<T, NL, true, E, 0>(in, out, a, nplanes, ncomp, twe, st);
+            if constexpr (E::kLen * NL / E::kEPT % 32 == 0)  // whole warps (the widest tile always is)
+                if (row_mode) return launch_lines_k<T, NL, true, E, 0>(in, out, a, nplanes, ncomp, twe, st);
             if constexpr (E::kLen > 0) {
                 if (2 * a.in_len == L && a.out_len == L && a.out_lo == 0)
                     return launch_lines_k<T, NL, false, E, 1>(in, out, a, nplanes, ncomp, twe, st);
@@ -761,12 +852,11 @@ int launch_r2c_rows(const TIn *in, cplx<T> *out, const R2CArgs &a, const TwPair<
     };
     return dispatch([&](auto eng) -> int {
         using E = decltype(eng);
-        const cplx<T> *twe = eng_tw<E>(tw);
-        return with_nl<T, E>(L, 1, sizeof(T) == 4 ? 16 : 8, 0, [&](auto nlc) -> int {
+        const cplx<T> *twe = tw.st;
+        return with_nl<T, E, 8, 2, true>(L, [&](auto nlc) -> int {
             constexpr int NL = decltype(nlc)::value;
-            const int nt = fft_threads(L, NL, E::kEPT);
-            if (nt < 1 || nt > E::kMaxThreads || (L * NL) % E::kEPT) return OSC_E_FFT_SIZE;
-            const size_t sm = sizeof(cplx<T>) * ((size_t)L + (size_t)L * (NL + 1));
+            const int nt = eng_threads<E>(a.p, NL);
+            const size_t sm = eng_smem<E, T>(L, NL);
             const unsigned nblk = (unsigned)ceil_div(a.nrows, 2 * NL);
             if (E::kLen > 0 && 2 * a.nin == L) {
                 auto kern = k_r2c_rows<T, TIn, NL, E, true>;
@@ -812,19 +902,31 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
                     if (a.nl_div == 2 && NLH != NLC) return go(std::integral_constant<int, NLH>{});
                     return go(std::integral_constant<int, NLC>{});
                 }
-                return -1;  // no static engine: generic kernel
+                else {
+                    auto go = [&](auto nlcc) -> int {
+                        constexpr int NLC = decltype(nlcc)::value;
+                        const size_t sm = eng_smem<E, T>(L, 3 * NLC);
+                        auto kern = k_c2r_e8_rt<T, NLC>;
+                        int r = set_smem(kern, sm);
+                        if (r) return r;
+                        kern<<<(unsigned)ceil_div(a.nrows, 2 * NLC), mix_threads(a.p, 3 * NLC), sm, st>>>(in, a, tw.st);
+                        return launch_ok();
+                    };
+                    if (eng_smem<E, T>(L, 12) <= 75 * 1024) return go(std::integral_constant<int, 4>{});
+                    if (eng_smem<E, T>(L, 3) <= 200 * 1024) return go(std::integral_constant<int, 1>{});
+                    return -1;  // too long for three lines at once: the generic kernel
+                }
             });
             if (rc != -1) return rc;
         }
     }
     return dispatch_fft_len<T>(L, [&](auto eng) -> int {
         using E = decltype(eng);
-        const cplx<T> *twe = eng_tw<E>(tw);
-        return with_nl<T, E>(L, 1, sizeof(T) == 4 ? 16 : 8, 0, [&](auto nlc) -> int {
+        const cplx<T> *twe = tw.st;
+        return with_nl<T, E, 8, 1, false>(L, [&](auto nlc) -> int {
             constexpr int NL = decltype(nlc)::value;
-            const int nt = fft_threads(L, NL, E::kEPT);
-            if (nt < 1 || nt > E::kMaxThreads || (L * NL) % E::kEPT) return OSC_E_FFT_SIZE;
-            const size_t sm = sizeof(cplx<T>) * ((size_t)L + (size_t)L * (NL + 1)) +
+            const int nt = eng_threads<E>(a.p, NL);
+            const size_t sm = eng_smem<E, T>(L, NL) +
                               (a.e8 ? sizeof(T) * 3 * 2 * NL * (size_t)a.nout : 0);
             const unsigned nblk = (unsigned)ceil_div(a.nrows, 2 * NL);
             if (E::kLen > 0 && 2 * a.nout == L && a.flip_mask == 0) {
@@ -839,7 +941,7 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
                 kern<<<nblk, nt, sm, st>>>(in, a, twe);
             }
             return launch_ok();
-        });
+        }, 0, a.e8 ? sizeof(T) * 3 * 2 * (size_t)a.nout : 0);
     });
 }
 
@@ -928,7 +1030,7 @@ inline int launch_zconv_w512(const float2 *in, float2 *out, const ZConvArgs &a, 
 }
 
 template <typename T>
-int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPair<cplx<T>> &tw, int nl,
+int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPair<cplx<T>> &tw,
                  cudaStream_t st) {
     const int L = a.p.L;
     // a column range of a z slab (col_base > 0) runs on the radix warp engine only
@@ -981,29 +1083,22 @@ int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPa
     if (a.nsum > 0) return OSC_E_UNSUPPORTED;  // summed inputs: warp engine lengths only
     for (int i = 0; i < a.ng; ++i)
         if (a.g[i].zinner) return OSC_E_INVALID;
-    return dispatch_fft_len<T>(L, [&](auto eng) -> int {
-        using E = decltype(eng);
-        const cplx<T> *twe = eng_tw<E>(tw);
-        return with_nl<T, E>(L, 2, sizeof(T) == 4 ? 8 : 4, nl, [&](auto nlc) -> int {
-            constexpr int NL = decltype(nlc)::value;
-            const int nt = fft_threads(L, NL, E::kEPT);
-            if (nt < 1 || nt > E::kMaxThreads || (L * NL) % E::kEPT) return OSC_E_FFT_SIZE;
-            const size_t sm = sizeof(cplx<T>) * ((size_t)L + 2 * (size_t)L * (NL + 1));
-            const dim3 nblk((unsigned)ceil_div(a.ncols, NL), (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
-            if (E::kLen > 0 && 2 * a.nz == L) {
-                auto kern = k_zconv<T, NL, E, true>;
-                int rc = set_smem(kern, sm);
-                if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, out, a, twe, tw.rt);
-            } else {
-                auto kern = k_zconv<T, NL, E, false>;
-                int rc = set_smem(kern, sm);
-                if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, out, a, twe, tw.rt);
-            }
-            return launch_ok();
-        });
-    });
+    auto go = [&](auto nlc) -> int {
+        constexpr int NL = decltype(nlc)::value;
+        const size_t sm = sizeof(cplx<T>) * ((size_t)L + (size_t)(a.p.nst > 2 ? 3 : 2) * L * (NL + 1));
+        auto kern = k_zconv<T, NL>;
+        int rc = set_smem(kern, sm);
+        if (rc) return rc;
+        const dim3 nblk((unsigned)ceil_div(a.ncols, NL), (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
+        kern<<<nblk, mix_threads(a.p, NL), sm, st>>>(in, out, a, tw.st, tw.rt);
+        return launch_ok();
+    };
+    const int nls[2] = {8, 1};
+    switch (pick_nl_rt(L, nls, 2, sizeof(cplx<T>), a.p.nst > 2 ? 3 : 2)) {
+    case 8: return go(std::integral_constant<int, 8>{});
+    case 1: return go(std::integral_constant<int, 1>{});
+    default: return OSC_E_FFT_SIZE;
+    }
 }
 
 template <typename TC, typename TI, typename TO>
@@ -1013,7 +1108,7 @@ int launch_sym_lines(const TI *in, TO *out, const SymArgs &a, const TwPair<cplx<
     if (L != 2 * a.n) return OSC_E_INVALID;
     return dispatch_fft_len<TC>(L, [&](auto eng) -> int {
         using E = decltype(eng);
-        const cplx<TC> *twe = eng_tw<E>(tw);
+        const cplx<TC> *twe = tw.st;
         // static engines: up to 16 line pairs per CTA, so the short lines of small batch
         // groups still give CTAs of several warps
         auto with_sym_nl = [&](auto &&f) -> int {
@@ -1027,14 +1122,13 @@ int launch_sym_lines(const TI *in, TO *out, const SymArgs &a, const TwPair<cplx<
                 if (a.nl_div >= 2 && NL2 != NL1) return f(std::integral_constant<int, NL2>{});
                 return f(std::integral_constant<int, NL1>{});
             } else {
-                return with_nl<TC, E>(L, 1, 8, 0, f);
+                return with_nl<TC, E, 8, 2, false>(L, f);
             }
         };
         return with_sym_nl([&](auto nlc) -> int {
             constexpr int NL = decltype(nlc)::value;
-            const int nt = fft_threads(L, NL, E::kEPT);
-            if (nt < 1 || nt > E::kMaxThreads || (L * NL) % E::kEPT) return OSC_E_FFT_SIZE;
-            const size_t sm = sizeof(cplx<TC>) * ((size_t)L + (size_t)L * (NL + 1));
+            const int nt = eng_threads<E>(a.p, NL);
+            const size_t sm = eng_smem<E, TC>(L, NL);
             const unsigned nblk = (unsigned)ceil_div(((a.npq + 1) & ~(int64_t)1) * a.nb, 2 * NL);
             auto go = [&](auto kern) -> int {
                 int rc = set_smem(kern, sm);

@@ -1,0 +1,7 @@
+// fft_sym_f64.cu -- FP64 even/odd line transforms of the Green build (fft_kernels_impl.cuh).
+#include "fft_kernels_impl.cuh"
+
+namespace osc {
+template int launch_sym_lines<double, double, double>(const double *, double *, const SymArgs &,
+                                                      const TwPair<cplx<double>> &, bool, bool, cudaStream_t);
+}  // namespace osc

@@ -446,7 +446,7 @@ static int pipe_phi_opt(osc_ctx *c, const LGeom &g, const double *rho, double *p
     }
     {
         Launch L_(c, "fft_z_conv");
-        TRY(kchk(c, launch_zconv<T>(X2, X3, za, twz, 0, c->stream), "z conv"));
+        TRY(kchk(c, launch_zconv<T>(X2, X3, za, twz, c->stream), "z conv"));
     }
     // inverse sign +1 along an axis = standard inverse read at the mirrored index
     LineArgs li = ly;

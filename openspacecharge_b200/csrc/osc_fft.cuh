@@ -15,7 +15,10 @@
 // Its first stage can skip the zero upper half of the input (forward transforms of the
 // zero-padded doubled grid) and its last stage can skip the upper half of the output
 // (inverse transforms whose physical window is the lower half).  FftRuntime follows a
-// runtime radix plan for any other 2^a 3^b 5^c length with the table tw[m]=exp(2 pi i m/L).
+// runtime radix plan for any other 2^a 3^b 5^c length: radices up to 16, so that the lengths
+// up to 240 take two stages and most others three, the same per-stage twiddle table, and two
+// line buffers that the stages alternate between (one barrier per stage).  A step on 45 x 36 x 50
+// (lengths 90, 72, 100) took 339 us on radices 8, 4, 2, 3, 5 in place, and takes 211.
 //
 // Twiddles are computed on the host in FP64 and rounded once for FP32; sign -1 uses the
 // conjugate.  Convention: X[k] = sum_j x[j] exp(sign*2*pi*i*j*k/L), unnormalised -- the sign
@@ -36,7 +39,8 @@ struct FFTPlan {
     int radix[FFT_MAX_STAGES];
 };
 
-// Host: radix plan for L = 2^a 3^b 5^c (radix 8 first, then 4, 2, 3, 5).  Returns false
+// Host: radix plan for L = 2^a 3^b 5^c with the fewest stages, and of those the smallest sum
+// of radices, an even radix first (its upper half of zero-padded input is zero).  Returns false
 // for other lengths, odd lengths or L > FFT_MAX_LEN.
 bool make_fft_plan(int L, FFTPlan &p);
 // Threads of a CTA that transforms NL lines of length L.
@@ -187,63 +191,114 @@ template <> struct Dft<5> {
     }
 };
 
-// ---- runtime-plan engine ----------------------------------------------------------------
-// One Stockham stage over NL interleaved lines; all threads of the CTA must call it.
-template <typename V, int R, int NL>
-__device__ __forceinline__ void stockham_stage(V *buf, int lstr, int L, int Ns, const V *tw, int sign) {
-    constexpr int MAXB = (FFT_EPT + R - 1) / R;
-    const int nthreads = blockDim.x * blockDim.y;
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    const int nb = L / R;
-    const int total = nb * NL;
-    const int tstep = L / (Ns * R);
-    V v[MAXB][R];
-#pragma unroll
-    for (int q = 0; q < MAXB; ++q) {
-        const int b = tid + q * nthreads;
-        if (b < total) {
-            const int line = b % NL;
-            const int j = b / NL;
-            const int k = j % Ns;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                V x = buf[(j + r * nb) * lstr + line];
-                if (r) x = cmul(x, tw_get(tw, r * k * tstep, sign));
-                v[q][r] = x;
-            }
-            Dft<R>::run(v[q], sign);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < MAXB; ++q) {
-        const int b = tid + q * nthreads;
-        if (b < total) {
-            const int line = b % NL;
-            const int j = b / NL;
-            const int k = j % Ns;
-            const int idxD = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int r = 0; r < R; ++r) buf[(idxD + r * Ns) * lstr + line] = v[q][r];
-        }
-    }
-    __syncthreads();
+// N = N1 N2 coprime by the prime-factor map, without twiddles: input N2 n1 + N1 n2, output the k
+// with k = k1 mod N1 and k = k2 mod N2.
+constexpr int crt_index(int n1, int n2, int k1, int k2) {
+    int k = 0;
+    while (k % n1 != k1 || k % n2 != k2) ++k;
+    return k;
 }
-
-// Full transform of the NL interleaved lines in buf.  Caller synchronises before.
-template <typename V, int NL>
-__device__ __forceinline__ void fft_smem(V *buf, int lstr, const FFTPlan &p, const V *tw, int sign) {
-    int Ns = 1;
-    for (int s = 0; s < p.nst; ++s) {
-        const int R = p.radix[s];
-        switch (R) {
-        case 8: stockham_stage<V, 8, NL>(buf, lstr, p.L, Ns, tw, sign); break;
-        case 4: stockham_stage<V, 4, NL>(buf, lstr, p.L, Ns, tw, sign); break;
-        case 2: stockham_stage<V, 2, NL>(buf, lstr, p.L, Ns, tw, sign); break;
-        case 3: stockham_stage<V, 3, NL>(buf, lstr, p.L, Ns, tw, sign); break;
-        default: stockham_stage<V, 5, NL>(buf, lstr, p.L, Ns, tw, sign); break;
+template <int N1, int N2> struct DftPfa {
+    template <typename V> __device__ __forceinline__ static void run(V *v, int s) {
+        V t[N1][N2];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) {
+            V a[N1];
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) a[n1] = v[(N2 * n1 + N1 * n2) % (N1 * N2)];
+            Dft<N1>::run(a, s);
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) t[n1][n2] = a[n1];
         }
-        Ns *= R;
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            Dft<N2>::run(t[k1], s);
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) v[crt_index(N1, N2, k1, k2)] = t[k1][k2];
+        }
+    }
+};
+template <> struct Dft<6> : DftPfa<2, 3> {};
+template <> struct Dft<10> : DftPfa<2, 5> {};
+template <> struct Dft<12> : DftPfa<4, 3> {};
+template <> struct Dft<15> : DftPfa<3, 5> {};
+
+template <> struct Dft<9> {
+    template <typename V> __device__ __forceinline__ static void run(V *v, int s) {
+        typedef decltype(v[0].x) T;
+        // cos and sin of 2 pi m / 9, m = 1, 2, 4
+        const T c1 = (T)0.76604444311897803520239265055542, s1 = (T)0.64278760968653932632264340990726;
+        const T c2 = (T)0.17364817766693034885171662676931, s2 = (T)0.98480775301220805936674302458952;
+        const T c4 = (T)-0.93969262078590838405410927732473, s4 = (T)0.34202014332566873304409961468226;
+        const T sg = (T)s;
+        V t[3][3];
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            t[n][0] = v[n];
+            t[n][1] = v[n + 3];
+            t[n][2] = v[n + 6];
+            Dft<3>::run(t[n], s);
+        }
+        auto rot = [&](V &x, T cr, T sr) {
+            const V u = x;
+            x.x = cr * u.x - sg * sr * u.y;
+            x.y = cr * u.y + sg * sr * u.x;
+        };
+        rot(t[1][1], c1, s1);
+        rot(t[1][2], c2, s2);
+        rot(t[2][1], c2, s2);
+        rot(t[2][2], c4, s4);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            V a[3] = {t[0][k], t[1][k], t[2][k]};
+            Dft<3>::run(a, s);
+            v[k] = a[0];
+            v[k + 3] = a[1];
+            v[k + 6] = a[2];
+        }
+    }
+};
+
+// ---- runtime-plan engine ----------------------------------------------------------------
+// One Stockham stage over NL interleaved lines from ld(e, line) to st(e, line, v), which must
+// not overlap unless a butterfly's inputs are its outputs.  A thread takes butterfly after
+// butterfly; with blockDim a multiple of NL its line is threadIdx.x % NL in all of them.
+template <typename V, int R, int NL, bool FIRST, class LD, class ST>
+__device__ __forceinline__ void mix_stage_r(int L, int Ns, const V *tw, int sign, const LD &ld, const ST &st) {
+    const int nb = L / R, total = nb * NL;
+    // j / Ns by multiplication: exact while j Ns < 2^20 (j < L / R <= 1024)
+    const unsigned magic = FIRST ? 0u : ((1u << 20) + (unsigned)Ns - 1u) / (unsigned)Ns;
+    for (int b = threadIdx.x; b < total; b += blockDim.x) {
+        const int line = b % NL, j = b / NL;
+        const int q = FIRST ? j : (int)(((unsigned)j * magic) >> 20), k = FIRST ? 0 : j - q * Ns;
+        V v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = ld(j + r * nb, line);
+        if (!FIRST) {
+            const V *t = tw + (Ns - 1) + k * (R - 1) - 1;
+#pragma unroll
+            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw_get(t, r, sign));
+        }
+        Dft<R>::run(v, sign);
+        const int d = q * Ns * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) st(d + r * Ns, line, v[r]);
+    }
+}
+template <typename V, int NL, bool FIRST, class LD, class ST>
+__device__ __forceinline__ void mix_stage(int R, int L, int Ns, const V *tw, int sign, const LD &ld, const ST &st) {
+    switch (R) {
+    case 2: mix_stage_r<V, 2, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 3: mix_stage_r<V, 3, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 4: mix_stage_r<V, 4, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 5: mix_stage_r<V, 5, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 6: mix_stage_r<V, 6, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 8: mix_stage_r<V, 8, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 9: mix_stage_r<V, 9, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 10: mix_stage_r<V, 10, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 12: mix_stage_r<V, 12, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    case 15: mix_stage_r<V, 15, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
+    default: mix_stage_r<V, 16, NL, FIRST>(L, Ns, tw, sign, ld, st); break;
     }
 }
 
@@ -371,13 +426,15 @@ __device__ __forceinline__ void fft_io_rec(Radices<R, Rest...>, V *buf, const V 
     if constexpr (!last) fft_io_rec<V, NL, L, Ns * R, HIN, HOUT, EPT>(Radices<Rest...>{}, buf, tw, sign, ld, st);
 }
 
-// FFT engines.  FftRuntime CTAs are capped at 256 threads so the generic stage code keeps
-// its registers; FftStatic CTAs at 512.  HIN/HOUT only change the static engine.
+// FFT engines.  FftRuntime CTAs are capped at 256 threads so the radix-16 stages keep their
+// registers; FftStatic CTAs at 512.  HIN/HOUT only change the static engine.
 //
 // run_io(buf, plan, tw, sign, ld, st): transform with input ld(e, line) (asked only for
 // e < L/2 when HIN) and output st(e, line, v) (called only for e < L/2 when HOUT; storers
 // must themselves ignore indices outside their window).  buf is the working buffer; ld may
-// read another shared buffer.
+// read another shared buffer.  run(buf, ...): transform of the lines in buf, returns the buffer
+// that holds the result.  FftRuntime's working buffer is two line buffers, the second after
+// the first (one is enough for run_io with at most two stages).
 struct FftRuntime {
     static constexpr int kLen = 0;
     static constexpr int kEPT = FFT_EPT;
@@ -385,27 +442,61 @@ struct FftRuntime {
     static constexpr int kNst = 0;
     static constexpr int kRad[1] = {0};
     template <typename V, int NL, bool HIN, bool HOUT>
-    __device__ __forceinline__ static void run(V *buf, const FFTPlan &p, const V *tw, int sign) {
-        fft_smem<V, NL>(buf, NL + 1, p, tw, sign);
+    __device__ __forceinline__ static V *run(V *buf, const FFTPlan &p, const V *tw, int sign) {
+        constexpr int lstr = NL + 1;
+        V *a = buf, *b = buf + p.L * lstr;
+        int Ns = 1;
+        for (int s = 0; s < p.nst; ++s) {
+            auto ld = [a](int e, int l) -> V { return a[e * lstr + l]; };
+            auto st = [b](int e, int l, const V &x) { b[e * lstr + l] = x; };
+            if (s == 0) mix_stage<V, NL, true>(p.radix[s], p.L, Ns, tw, sign, ld, st);
+            else mix_stage<V, NL, false>(p.radix[s], p.L, Ns, tw, sign, ld, st);
+            __syncthreads();
+            Ns *= p.radix[s];
+            V *t = a;
+            a = b;
+            b = t;
+        }
+        return a;
     }
     template <typename V, int NL, bool HIN, bool HOUT, class LD, class ST>
     __device__ __forceinline__ static void run_io(V *buf, const FFTPlan &p, const V *tw, int sign, const LD &ld,
                                                   const ST &st) {
-        const int L = p.L, nthreads = blockDim.x, tid = threadIdx.x;
         constexpr int lstr = NL + 1;
-        for (int idx = tid; idx < NL * L; idx += nthreads) {
-            const int e = idx / NL, l = idx - e * NL;
-            buf[e * lstr + l] = ld(e, l);
+        V *a = buf, *b = buf + p.L * lstr;
+        {
+            auto sst = [a](int e, int l, const V &x) { a[e * lstr + l] = x; };
+            mix_stage<V, NL, true>(p.radix[0], p.L, 1, tw, sign, ld, sst);
         }
         __syncthreads();
-        fft_smem<V, NL>(buf, lstr, p, tw, sign);
-        for (int idx = tid; idx < NL * L; idx += nthreads) {
-            const int e = idx / NL, l = idx - e * NL;
-            st(e, l, buf[e * lstr + l]);
+        int Ns = p.radix[0];
+        for (int s = 1; s + 1 < p.nst; ++s) {
+            auto sld = [a](int e, int l) -> V { return a[e * lstr + l]; };
+            auto sst = [b](int e, int l, const V &x) { b[e * lstr + l] = x; };
+            mix_stage<V, NL, false>(p.radix[s], p.L, Ns, tw, sign, sld, sst);
+            __syncthreads();
+            Ns *= p.radix[s];
+            V *t = a;
+            a = b;
+            b = t;
+        }
+        auto sld = [a](int e, int l) -> V { return a[e * lstr + l]; };
+        if (p.nst > 1) {
+            mix_stage<V, NL, false>(p.radix[p.nst - 1], p.L, Ns, tw, sign, sld, st);
+        } else {
+            for (int idx = threadIdx.x; idx < NL * p.L; idx += blockDim.x) st(idx / NL, idx % NL, sld(idx / NL, idx % NL));
         }
         __syncthreads();
     }
 };
+// Threads of a runtime-plan CTA for `lines` lines: about one butterfly each in the stage with the
+// most, whole warps, at most 256.
+inline int mix_threads(const FFTPlan &p, int lines) {
+    int r = p.radix[0];
+    for (int s = 1; s < p.nst; ++s) r = p.radix[s] < r ? p.radix[s] : r;
+    const int n = (p.L / r * lines + 31) / 32 * 32;
+    return n < 64 ? 64 : (n > FftRuntime::kMaxThreads ? FftRuntime::kMaxThreads : n);
+}
 // Static engine with EPT_ complex values per thread and stage (L*NL/EPT_ threads per CTA).
 template <int EPT_, int L_, int... Rs> struct FftStaticT {
     static constexpr int kLen = L_;
@@ -414,8 +505,9 @@ template <int EPT_, int L_, int... Rs> struct FftStaticT {
     static constexpr int kNst = sizeof...(Rs);
     static constexpr int kRad[sizeof...(Rs)] = {Rs...};
     template <typename V, int NL, bool HIN, bool HOUT>
-    __device__ __forceinline__ static void run(V *buf, const FFTPlan &, const V *tw, int sign) {
+    __device__ __forceinline__ static V *run(V *buf, const FFTPlan &, const V *tw, int sign) {
         fft_ct<V, NL, L_, 1, HIN, HOUT, EPT_, Rs...>(buf, tw, sign);
+        return buf;
     }
     template <typename V, int NL, bool HIN, bool HOUT, class LD, class ST>
     __device__ __forceinline__ static void run_io(V *buf, const FFTPlan &, const V *tw, int sign, const LD &ld,
@@ -484,6 +576,8 @@ struct WarpNone {
 };
 template <class F> inline int dispatch_warp_len(int L, F &&f) {
     switch (L) {
+    case 32: return f(WarpFft<32, 4, 2, 4>{});
+    case 64: return f(WarpFft<64, 4, 4, 4>{});
     case 96: return f(WarpFft<96, 4, 2, 3, 4>{});
     case 128: return f(WarpFft<128, 4, 8, 4>{});
     case 192: return f(WarpFft<192, 4, 4, 3, 4>{});
@@ -494,9 +588,9 @@ template <class F> inline int dispatch_warp_len(int L, F &&f) {
     }
 }
 
-// Twiddle tables of one length: rt[m] = exp(2 pi i m/L) for the runtime engine; st is the
-// per-stage table of the static engine ([stage][k][r-1], L-1 entries), or rt when the
-// length has no static engine; wt the same for the warp engine of the z pass (or rt).
+// Twiddle tables of one length: rt[m] = exp(2 pi i m/L); st is the per-stage table
+// ([stage][k][r-1], L-1 entries) of the static engine, or of the runtime plan when the length
+// has no static engine; wt the same for the warp engine of the z pass (or rt).
 template <typename V> struct TwPair {
     const V *rt;
     const V *st;

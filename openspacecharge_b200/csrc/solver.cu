@@ -521,7 +521,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     for (int i = 0; i < gs->nspec; ++i) za.g[i] = gs->spec[i];
     {
         Launch L_(c, "fft_z_conv");
-        TRY(kerr(c, launch_zconv<T>(X2, X3, za, twz, 0, c->stream), "z convolution"));
+        TRY(kerr(c, launch_zconv<T>(X2, X3, za, twz, c->stream), "z convolution"));
     }
     // y inverse, window [0,ny)
     LineArgs li = ly;
@@ -614,7 +614,7 @@ int slab_forward(osc_ctx *c, int nx, int ny, int nzl, const float4 *quad, cplx<f
 
 int slab_zpass(osc_ctx *c, const FreeSpaceJob &j, int col0, int ncols, const cplx<float> *in, cplx<float> *out) {
     const int nx = j.nx, ny = j.ny, nz = j.nz, nxh = nx + 1, Ny = 2 * ny, Nz = 2 * nz;
-    if (!zconv_warp_ok(Nz, nz, 4))
+    if (!zconv_warp_ok(Nz, nz, 4) || Nz < 96)
         return set_err(c, OSC_E_UNSUPPORTED, "z slabs: doubled z length %d has no warp-per-column z pass", Nz);
     if (col0 < 0 || ncols < 0 || (int64_t)col0 + ncols > (int64_t)nxh * Ny)
         return set_err(c, OSC_E_INVALID, "z slabs: columns [%d, %d) outside the %d columns", col0, col0 + ncols,
@@ -651,7 +651,7 @@ int slab_zpass(osc_ctx *c, const FreeSpaceJob &j, int col0, int ncols, const cpl
     za.fault = c->d_fault;
     za.nbatch = 1;
     Launch L_(c, "fft_z_conv");
-    return kerr(c, launch_zconv<float>(in, out, za, twz, 0, c->stream), "z convolution");
+    return kerr(c, launch_zconv<float>(in, out, za, twz, c->stream), "z convolution");
 }
 
 int slab_inverse(osc_ctx *c, int nx, int ny, int nzl, const cplx<float> *X3, float4 *e8) {
