@@ -566,12 +566,8 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
         }
         j.E4 = E8;
         j.e4_pairs = 1;
-        j.B = nullptr;
-        if (B) {
-            double *Bg;
-            TRY(ws_get(ctx, "st_Bg", sizeof(double) * 3 * N, (void **)&Bg));
-            j.B = Bg;
-        }
+        if (B && at_cathode) TRY(ws_get(ctx, "st_B8", sizeof(float4) * 2 * N, &j.B4));
+        else j.calc_b = 0;
         TRY(freespace_opt<float, float>(ctx, j, rho));
         if (!at_cathode) {  // the E grid of this free-space step, for the adjoint
             osc_ctx::FwdRecord &f = ctx->fwd;
@@ -598,18 +594,16 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
             TRY(ws_get(ctx, "st_sE", sizeof(double) * 3 * (size_t)np, (void **)&Eo));
             if (B) TRY(ws_get(ctx, "st_sB", sizeof(double) * 3 * (size_t)np, (void **)&Bo));
         }
-        {
+        auto gather = [&](const void *g8, double *Eg, double *Bg, unsigned long long *ncl) -> int {
             Launch L_(ctx, order == OSC_ORDER_ANY ? "interp_f32" : "interp_f32_runs");
-            if ((order == OSC_ORDER_ANY
-                     ? launch_interp_pairs(ia, reinterpret_cast<const float4 *>(E8), Eo, ctx->d_small + 2, ctx->stream)
-                     : launch_interp_pairs_runs(ia, reinterpret_cast<const float4 *>(E8), Eo, ctx->d_small + 2,
-                                                ctx->stream)))
+            const float4 *g = reinterpret_cast<const float4 *>(g8);
+            if ((order == OSC_ORDER_ANY ? launch_interp_pairs(ia, g, Eg, ncl, ctx->stream, Bg, j.bcoef)
+                                        : launch_interp_pairs_runs(ia, g, Eg, ncl, ctx->stream, Bg, j.bcoef)))
                 return set_err(ctx, OSC_E_CUDA, "interp");
-        }
-        if (B) {
-            Launch L_(ctx, "interp_f64");
-            if (launch_interp_planes(ia, j.B, Bo, ctx->d_small + 3, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "interp");
-        }
+            return OSC_OK;
+        };
+        TRY(gather(E8, Eo, at_cathode ? nullptr : Bo, ctx->d_small + 2));
+        if (j.B4) TRY(gather(j.B4, nullptr, Bo, ctx->d_small + 3));
         if (inv) {
             Launch L_(ctx, "unpermute", B ? 2 : 1);
             if (launch_unpermute_rows3(np, inv, Eo, E, ctx->stream) ||
@@ -625,19 +619,18 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
     TRY(ws_get(ctx, "st_E4d", sizeof(double4) * N, &E4));
     TRY(deposit_rho<double>(ctx, da, rho, N, 1.0, ctx->particle_order == OSC_ORDER_CELL_SORTED));
     j.E4 = E4;
-    if (B) {
-        double *Bg;
-        TRY(ws_get(ctx, "st_Bg", sizeof(double) * 3 * N, (void **)&Bg));
-        j.B = Bg;
-    }
+    if (B && at_cathode) TRY(ws_get(ctx, "st_B4d", sizeof(double4) * N, &j.B4));
+    else j.calc_b = 0;
     TRY(freespace_opt<double, double>(ctx, j, rho));
     {
         Launch L_(ctx, "interp_f64");
-        if (launch_interp_vec4<double>(ia, E4, E, ctx->d_small + 2, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "interp");
+        if (launch_interp_vec4<double>(ia, E4, E, ctx->d_small + 2, ctx->stream, at_cathode ? nullptr : B, j.bcoef))
+            return set_err(ctx, OSC_E_CUDA, "interp");
     }
-    if (B) {
+    if (j.B4) {
         Launch L_(ctx, "interp_f64");
-        if (launch_interp_planes(ia, j.B, B, ctx->d_small + 3, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "interp");
+        if (launch_interp_vec4<double>(ia, j.B4, nullptr, ctx->d_small + 3, ctx->stream, B, j.bcoef))
+            return set_err(ctx, OSC_E_CUDA, "interp");
     }
     return OSC_OK;
 }

@@ -879,7 +879,7 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
     const int L = a.p.L;
     // FP32 x-pairs or FP64 nodes: the specialised kernel; other combinations: generic
     if (a.e8 && (a.e8_node != 0) == (sizeof(T) == 8)) {
-        bool e8_only = a.e8 && a.ncomp == 3 && a.flip_mask == 0 && 2 * a.nout == L &&
+        bool e8_only = a.e8 && a.ncomp <= 3 && a.flip_mask == 0 && 2 * a.nout == L &&
                        reinterpret_cast<uintptr_t>(a.e8) % 32 == 0;
         for (int c = 0; c < a.ncomp && e8_only; ++c) e8_only = a.ndest[c] == 0;
         if (e8_only) {

@@ -508,7 +508,7 @@ int pipe_solve(osc_ctx *c, int precision, const double delta[3], double gam0, co
             TRY(conv_extract(c, g, crho, ct, PIPE_INV[t], PIPE_SIGN[t] * factr, phi, t > 0));
         }
     }
-    if (e8 && !E && !B) {  // E only as the x-pair grid of the FP32 gather
+    if (e8) {  // E only as the x-pair grid of the FP32 gather
         Launch L_(c, "fd_efield");
         return kchk(c, launch_fd_efield_pairs(phi, e8, g.n[0], g.n[1], g.n[2], delta[0], delta[1], delta[2], gam0,
                                               c->stream),
@@ -519,10 +519,6 @@ int pipe_solve(osc_ctx *c, int precision, const double delta[3], double gam0, co
         Launch L_(c, "fd_efield");
         TRY(kchk(c, launch_fd_efield(phi, E, g.n[0], g.n[1], g.n[2], delta[0], delta[1], delta[2], gam0, c->stream),
                  "fd"));
-    }
-    if (e8) {
-        Launch L_(c, "planes_to_pairs");
-        TRY(kchk(c, launch_planes_to_pairs(E, e8, g.n[0], g.N, c->stream), "E pairs"));
     }
     if (!B) return OSC_OK;
     const double beta0 = std::sqrt(1 - 1 / (gam0 * gam0));

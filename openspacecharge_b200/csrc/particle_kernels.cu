@@ -234,6 +234,27 @@ __device__ __forceinline__ bool locate(const InterpArgs &a, double x, double y, 
     return flag;
 }
 
+// A warp's 32 staged field vectors ws (row 0 is particle m0 of np) as contiguous rows: E as they
+// are, and/or B = bcoef (-v_y, v_x, 0), the magnetic field of the moving charges whose
+// field is v (space_charge_3d, code/open_spacecharge_mod.f90:456-461): B on the grid is
+// proportional to E there, so gathering it would only repeat the gather of E (FP64 step, 128^3 and
+// 4e6 particles: 998 us with B planes and their gather, 655 without).
+template <typename TO>
+__device__ __forceinline__ void store_rows(const TO *ws, int64_t m0, int64_t np, int lane, TO *__restrict__ E,
+                                           TO *__restrict__ B, double bcoef) {
+    const int64_t o0 = 3 * m0, n3 = 3 * np;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        const int e = 32 * t + lane;
+        if (o0 + e >= n3) continue;
+        if (E) E[o0 + e] = ws[e];
+        if (B) {
+            const int c = e % 3;
+            B[o0 + e] = c == 0 ? (TO)(-bcoef * ws[e + 1]) : (c == 1 ? (TO)(bcoef * ws[e - 1]) : (TO)0);
+        }
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void load_node(const vec4<T> *g, int64_t n, double &a, double &b, double &c) {
     if constexpr (sizeof(T) == 8) {  // one 256-bit read-only load per node
@@ -249,6 +270,7 @@ __device__ __forceinline__ void load_node(const vec4<T> *g, int64_t n, double &a
 
 template <typename T, typename TO>
 __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T> *__restrict__ g, TO *__restrict__ E,
+                                                     TO *__restrict__ B, double bcoef,
                                                      unsigned long long *__restrict__ nclamp) {
     // E goes through a per-warp shared-memory stage and is stored as contiguous rows (as in
     // k_interp_pairs); the loop runs while the warp's first particle exists
@@ -284,39 +306,21 @@ __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T>
         }
         count_one(nclamp, fl);
         __syncwarp();
-        const int64_t o0 = 3 * (m - lane), n3 = 3 * a.np;
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int e = 32 * t + lane;
-            if (o0 + e < n3) E[o0 + e] = ws[e];
-        }
+        store_rows(ws, m - lane, a.np, lane, E, B, bcoef);
         __syncwarp();
     }
 }
 
 template <typename T>
-int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp, cudaStream_t st) {
+int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp, cudaStream_t st,
+                       double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
     k_interp_vec4<T, double><<<nblocks(a.np, 256, 148 * 64), 256, 0, st>>>(a, reinterpret_cast<const vec4<T> *>(E4),
-                                                                            E, nclamp);
+                                                                            E, B, bcoef, nclamp);
     return ok();
 }
-template <typename T>
-int launch_interp_vec4_any(const InterpArgs &a, const void *E4, void *E, int out_f32, unsigned long long *nclamp,
-                           cudaStream_t st) {
-    if (a.np <= 0) return OSC_OK;
-    if (out_f32)
-        k_interp_vec4<T, float><<<nblocks(a.np, 256, 148 * 64), 256, 0, st>>>(
-            a, reinterpret_cast<const vec4<T> *>(E4), reinterpret_cast<float *>(E), nclamp);
-    else
-        k_interp_vec4<T, double><<<nblocks(a.np, 256, 148 * 64), 256, 0, st>>>(
-            a, reinterpret_cast<const vec4<T> *>(E4), reinterpret_cast<double *>(E), nclamp);
-    return ok();
-}
-template int launch_interp_vec4<float>(const InterpArgs &, const void *, double *, unsigned long long *, cudaStream_t);
-template int launch_interp_vec4<double>(const InterpArgs &, const void *, double *, unsigned long long *, cudaStream_t);
-template int launch_interp_vec4_any<float>(const InterpArgs &, const void *, void *, int, unsigned long long *, cudaStream_t);
-template int launch_interp_vec4_any<double>(const InterpArgs &, const void *, void *, int, unsigned long long *, cudaStream_t);
+template int launch_interp_vec4<double>(const InterpArgs &, const void *, double *, unsigned long long *, cudaStream_t,
+                                        double *, double);
 
 // Three double planes [3][N], reference order of the 8-term sum per component.
 __global__ void __launch_bounds__(256) k_interp_planes(InterpArgs a, const double *__restrict__ F,
@@ -394,7 +398,8 @@ __device__ __forceinline__ bool interp_pair_one(const InterpArgs &a, const float
 // warp instead of 18 for three strided 8-byte stores per lane, on a kernel whose limit is the
 // L1's request port to L2.
 __global__ void __launch_bounds__(256) k_interp_pairs(InterpArgs a, const float4 *__restrict__ g8,
-                                                      double *__restrict__ E, unsigned long long *__restrict__ nclamp) {
+                                                      double *__restrict__ E, double *__restrict__ B, double bcoef,
+                                                      unsigned long long *__restrict__ nclamp) {
     __shared__ double stage[256 * 3];
     const int lane = threadIdx.x & 31;
     double *ws = stage + (threadIdx.x - lane) * 3;
@@ -422,12 +427,7 @@ __global__ void __launch_bounds__(256) k_interp_pairs(InterpArgs a, const float4
         if (live) fl = interp_pair_one(a, g8, plane, xm, ym, zm, ws + 3 * lane);
         count_one(nclamp, fl);
         __syncwarp();
-        const int64_t o0 = 3 * (m - lane), n3 = 3 * a.np;
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int e = 32 * t + lane;
-            if (o0 + e < n3) E[o0 + e] = ws[e];
-        }
+        store_rows(ws, m - lane, a.np, lane, E, B, bcoef);
         __syncwarp();
     }
 }
@@ -443,7 +443,7 @@ __device__ __forceinline__ void ldg_v4(const double *p, double *v) {
 }
 template <int RUN>
 __global__ void __launch_bounds__(256, RUN == 4 ? 3 : 2) k_interp_pairs_runs(InterpArgs a, const float4 *__restrict__ g8, bool vec,
-                                                           double *__restrict__ E,
+                                                           double *__restrict__ E, double *__restrict__ B, double bcoef,
                                                            unsigned long long *__restrict__ nclamp) {
     static_assert(RUN % 4 == 0, "runs of whole 256-bit vectors");
     const int64_t plane = (int64_t)a.nx * a.ny;
@@ -492,17 +492,29 @@ __global__ void __launch_bounds__(256, RUN == 4 ? 3 : 2) k_interp_pairs_runs(Int
             out[3 * t + 1] = ey;
             out[3 * t + 2] = ez;
         }
-        double *dst = E + 3 * m0;
-        if (full) {
+        auto rows = [&](double *dst) {
+            if (full) {
 #pragma unroll
-            for (int v = 0; v < 3 * RUN / 4; ++v)
-                asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(dst + 4 * v), "d"(out[4 * v]),
-                             "d"(out[4 * v + 1]), "d"(out[4 * v + 2]), "d"(out[4 * v + 3])
-                             : "memory");
-        } else {
+                for (int v = 0; v < 3 * RUN / 4; ++v)
+                    asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(dst + 4 * v), "d"(out[4 * v]),
+                                 "d"(out[4 * v + 1]), "d"(out[4 * v + 2]), "d"(out[4 * v + 3])
+                                 : "memory");
+            } else {
 #pragma unroll
-            for (int e = 0; e < 3 * RUN; ++e)
-                if (m0 + e / 3 < a.np) dst[e] = out[e];
+                for (int e = 0; e < 3 * RUN; ++e)
+                    if (m0 + e / 3 < a.np) dst[e] = out[e];
+            }
+        };
+        if (E) rows(E + 3 * m0);
+        if (B) {  // as store_rows
+#pragma unroll
+            for (int t = 0; t < RUN; ++t) {
+                const double vx = out[3 * t];
+                out[3 * t] = -bcoef * out[3 * t + 1];
+                out[3 * t + 1] = bcoef * vx;
+                out[3 * t + 2] = 0.0;
+            }
+            rows(B + 3 * m0);
         }
         ncl = __reduce_add_sync(0xffffffffu, ncl);
         if (lane == 0 && ncl) atomicAdd(nclamp, (unsigned long long)ncl);
@@ -510,27 +522,27 @@ __global__ void __launch_bounds__(256, RUN == 4 ? 3 : 2) k_interp_pairs_runs(Int
 }
 
 int launch_interp_pairs_runs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
-                             cudaStream_t st) {
+                             cudaStream_t st, double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(E8) % 32) return OSC_E_INVALID;
     auto al = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 32 == 0; };
-    const bool vec = al(a.x) && al(a.y) && al(a.z) && al(E);
+    const bool vec = al(a.x) && al(a.y) && al(a.z) && al(E) && al(B);
     const int run = a.tile == 8 ? 8 : 4;
     const int64_t chunks = (a.np + 32 * run - 1) / (32 * run);
     const unsigned nb = nblocks(chunks * 32, 256, 148 * (int64_t)(a.ctas > 0 ? a.ctas : 16));
     if (run == 8)
-        k_interp_pairs_runs<8><<<nb, 256, 0, st>>>(a, E8, vec, E, nclamp);
+        k_interp_pairs_runs<8><<<nb, 256, 0, st>>>(a, E8, vec, E, B, bcoef, nclamp);
     else
-        k_interp_pairs_runs<4><<<nb, 256, 0, st>>>(a, E8, vec, E, nclamp);
+        k_interp_pairs_runs<4><<<nb, 256, 0, st>>>(a, E8, vec, E, B, bcoef, nclamp);
     return ok();
 }
 
 int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
-                        cudaStream_t st) {
+                        cudaStream_t st, double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(E8) % 32) return OSC_E_INVALID;
     const int64_t cap = 148 * (int64_t)(a.ctas > 0 ? a.ctas : 64);
-    k_interp_pairs<<<nblocks(a.np, 256, cap), 256, 0, st>>>(a, E8, E, nclamp);
+    k_interp_pairs<<<nblocks(a.np, 256, cap), 256, 0, st>>>(a, E8, E, B, bcoef, nclamp);
     return ok();
 }
 

@@ -86,24 +86,21 @@ struct InterpArgs {
     int tile = 0;
     int ctas = 0;
 };
+// The gathers from a grid write E (when not null) and/or B = bcoef (-E_y, E_x, 0) (when not null).
 template <typename T>
 int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp,
-                       cudaStream_t st);
-// out_f32 != 0: E is float [np][3]
-template <typename T>
-int launch_interp_vec4_any(const InterpArgs &a, const void *E4, void *E, int out_f32,
-                           unsigned long long *nclamp, cudaStream_t st);
+                       cudaStream_t st, double *B = nullptr, double bcoef = 0);
 int launch_interp_planes(const InterpArgs &a, const double *F, double *out,
                          unsigned long long *nclamp, cudaStream_t st);
 // Gather from an x-pair grid: node n holds (E(n), E(n+1)) as two float4 in one 32-byte
 // sector, so the 8 nodes of a particle come from 4 sectors.
 int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
-                        cudaStream_t st);
+                        cudaStream_t st, double *B = nullptr, double bcoef = 0);
 // The same gather for particles in cell order: runs of consecutive particles in one cell
 // share their stencil's loads; coordinates and E move as 256-bit vectors.  Bit-identical
 // to launch_interp_pairs for any order.
 int launch_interp_pairs_runs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
-                             cudaStream_t st);
+                             cudaStream_t st, double *B = nullptr, double bcoef = 0);
 
 // Bounding box {xmin,xmax,ymin,ymax,zmin,zmax} of the particles, written to bb (device)
 // through order-preserving 64-bit keys; also counts non-finite coordinates.

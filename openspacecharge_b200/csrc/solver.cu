@@ -433,6 +433,12 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
             add_dest(add_out(2, -1.0), j.B, 1, 0, -j.bcoef);
         }
     }
+    if (j.B4) {  // outputs 3 and 4, after the three of E4
+        if (!j.E4 || !j.at_cathode || j.E || j.phi || j.B || j.comp_mask != 7)
+            return set_err(c, OSC_E_INVALID, "B grid: cathode solves to the E grid only");
+        add_out(1, -1.0);
+        add_out(2, -1.0);
+    }
     }  // summed solve or per-output destinations
     if (j.calc_b && j.B) TRY(cuda_check(c, cudaMemsetAsync(j.B + 2 * N, 0, sizeof(double) * N, c->stream), "memset B"));
 
@@ -555,11 +561,19 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     cr.zin = zin ? 1 : 0;
     cr.zin_nz = nz;
     cr.zin_ny = ny;
-    cr.ncomp = nout;
+    cr.ncomp = j.B4 ? 3 : nout;
     cr.nl_div = tune_get(c, "c2r_nl_div:" + tprec + ":L" + std::to_string(Nx));
     {
         Launch L_(c, "fft_x_c2r");
         TRY(kerr(c, launch_c2r_rows<T>(X4, cr, twx, c->stream), "x c2r"));
+    }
+    if (j.B4) {
+        cr.e8 = j.B4;
+        cr.ncomp = 2;
+        cr.e8_comp[0] = 0;
+        cr.e8_comp[1] = cr.e8_comp[2] = 1;  // the third slot is not used
+        Launch L_(c, "fft_x_c2r");
+        TRY(kerr(c, launch_c2r_rows<T>(X4 + 3 * cr.in_cstride, cr, twx, c->stream), "x c2r B"));
     }
     return OSC_OK;
 }

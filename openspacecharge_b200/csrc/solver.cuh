@@ -41,6 +41,9 @@ struct FreeSpaceJob {
     double *B = nullptr;    // device f64 [3][N]
     void *E4 = nullptr;     // device vec4<T> [N], or the x-pair grid vec4<T> [N][2]
     int e4_pairs = 0;       // 1: E4 is the x-pair grid read by launch_interp_pairs
+    // cathode steps with B (calc_b): a grid like E4 for the fields (direct - image) whose B is
+    // bcoef (-y, x, 0); without a cathode B follows from E4 itself
+    void *B4 = nullptr;
     // FP32 only: the deposit's quad grid (float4 [N]); when set, the x transform sums each
     // node from it and the rho argument is not read
     const float4 *quad = nullptr;
@@ -104,8 +107,8 @@ int legacy_cathode(osc_ctx *c, const int nlo[3], const int nhi[3], const int npa
 int pipe_green_build(osc_ctx *c, const int nlo[3], const int nhi[3], const int npad[3],
                      const double delta[3], const double umin[3], double gam, double a, double b);
 // Pipe potential phi from rho (or, FP32 with npad 1, from the deposit's quad grid), then
-// E = -grad phi as FP64 planes E and/or the FP32 x-pair grid e8 (E null: e8 only, written
-// straight from phi), and B from the planes when B is given.
+// E = -grad phi as the FP32 x-pair grid e8, written straight from phi, or as FP64 planes E with
+// B from the planes when B is given.
 int pipe_solve(osc_ctx *c, int precision, const double delta[3], double gam0, const double *rho,
                double *phi, double *E, double *B, const float4 *quad = nullptr, float *e8 = nullptr);
 // pipe_solve after checking that the pipe Green set was built for this mesh.
