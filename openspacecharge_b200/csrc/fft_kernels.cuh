@@ -166,6 +166,23 @@ struct SymArgs {
     int64_t npq, in_bs, out_bs;
     int nl_div = 0;  // autotuner: 2 or 4 divides the line pairs per CTA of a static engine
 };
+// z transforms of a Green function that is even or odd in x and y only: real columns q (nq per
+// member, q = ky (nx+1) + kx) of length L, element p of column q of member b at in[b*in_bs + p*nq
+// + q], to the complex spectrum k in [0, dimz), dimz <= L, times scale, times i for the members
+// whose bit is set in imag, and with fold >= 0 times -exp(2 pi i fold k / L) (the image z-flip
+// phase).  Written at out[b*out_bs + q*zpitch + k] (zpitch > 0) or out[b*out_bs + k*nq + q].
+struct ZLineArgs {
+    FFTPlan p;
+    int nb;
+    int64_t nq, in_bs, out_bs;
+    int dimz, zpitch, fold;
+    unsigned imag;
+    double scale;
+};
+template <typename TO>
+int launch_green_zlines(const double *in, cplx<TO> *out, const ZLineArgs &a, const TwPair<cplx<double>> &tw,
+                        cudaStream_t st);
+
 // row_load: elements of a line are contiguous in the input (load along the line);
 // k_fast_store: outputs of a line are contiguous (store along the line).
 // TC: arithmetic type of the transform (double, or float from octant values rounded once).

@@ -731,6 +731,60 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
         for_rows(2 * NL, nk, fin);
 }
 
+// z transforms of the Green columns that are not even or odd in z (ZLineArgs): two real columns per
+// complex line, FP64.  Reads and, with zpitch 0, writes walk adjacent columns; the kz-innermost
+// store walks k.
+template <typename TO, int NL, class E>
+__global__ void __launch_bounds__(E::kMaxThreads) k_green_zlines(const double *__restrict__ in, cplx<TO> *__restrict__ out,
+                                                                 ZLineArgs a, const double2 *__restrict__ twg,
+                                                                 const double2 *__restrict__ tw_rt) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int64_t bin[2 * NL], bout[2 * NL];
+    __shared__ bool bim[2 * NL];
+    double2 *tw = reinterpret_cast<double2 *>(smem_raw);
+    const int L = E::kLen ? E::kLen : a.p.L;
+    double2 *buf = tw + L;
+    constexpr int lstr = NL + 1;
+    const int nthreads = blockDim.x, tid = threadIdx.x;
+    for (int t = tid; t < 2 * NL; t += nthreads) {
+        // members start on even lines (as in k_sym_lines)
+        const int64_t r = (int64_t)blockIdx.x * (2 * NL) + t, nq2 = (a.nq + 1) & ~(int64_t)1;
+        const int64_t b = r / nq2, q = r - b * nq2;
+        const bool live = b < a.nb && q < a.nq;
+        bin[t] = live ? b * a.in_bs + q : -1;
+        bout[t] = b * a.out_bs + q * (a.zpitch > 0 ? a.zpitch : 1);
+        bim[t] = (a.imag >> b) & 1u;
+    }
+    load_twiddles(tw, twg, L);
+    __syncthreads();
+#pragma unroll 4
+    for (int idx = tid; idx < 2 * NL * L; idx += nthreads) {
+        const int rr = idx % (2 * NL), p = idx / (2 * NL);
+        const double v = bin[rr] >= 0 ? in[bin[rr] + (int64_t)p * a.nq] : 0.0;
+        reinterpret_cast<double *>(&buf[p * lstr + (rr >> 1)])[rr & 1] = v;
+    }
+    __syncthreads();
+    const double2 *res = E::template run<double2, NL, false, false>(buf, a.p, tw, +1);
+    auto put = [&](int rr, int k) {
+        if (bin[rr] < 0) return;
+        const double2 Z = res[k * lstr + (rr >> 1)], Zm = res[(k > 0 ? L - k : 0) * lstr + (rr >> 1)];
+        double2 v = (rr & 1) == 0 ? make_double2(0.5 * (Z.x + Zm.x), 0.5 * (Z.y - Zm.y))
+                                  : make_double2(0.5 * (Z.y + Zm.y), 0.5 * (Zm.x - Z.x));
+        if (bim[rr]) v = make_double2(-v.y, v.x);
+        if (a.fold >= 0) {  // fold, k < 2^11: 32-bit index arithmetic
+            const double2 ph = __ldg(tw_rt + (int)(((unsigned)a.fold * (unsigned)k) % (unsigned)L));
+            v = make_double2(-(v.x * ph.x - v.y * ph.y), -(v.x * ph.y + v.y * ph.x));
+        }
+        out[bout[rr] + (a.zpitch > 0 ? (int64_t)k : (int64_t)k * a.nq)] =
+            mk<TO>((TO)(v.x * a.scale), (TO)(v.y * a.scale));
+    };
+    if (a.zpitch > 0) {
+        for (int idx = tid; idx < 2 * NL * a.dimz; idx += nthreads) put(idx / a.dimz, idx % a.dimz);
+    } else {
+        for (int idx = tid; idx < 2 * NL * a.dimz; idx += nthreads) put(idx % (2 * NL), idx / (2 * NL));
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // Launchers.  Shared memory above 48 KB needs the opt-in attribute, set per kernel.
 // The attribute is set once per kernel, device and size (a lookup instead of a driver call
@@ -1140,6 +1194,25 @@ int launch_sym_lines(const TI *in, TO *out, const SymArgs &a, const TwPair<cplx<
                                               : go(k_sym_lines<TC, TI, TO, NL, E, true, false>);
             return k_fast_store ? go(k_sym_lines<TC, TI, TO, NL, E, false, true>)
                                 : go(k_sym_lines<TC, TI, TO, NL, E, false, false>);
+        });
+    });
+}
+
+template <typename TO>
+int launch_green_zlines(const double *in, cplx<TO> *out, const ZLineArgs &a, const TwPair<cplx<double>> &tw,
+                        cudaStream_t st) {
+    const int L = a.p.L;
+    return dispatch_fft_len<double>(L, [&](auto eng) -> int {
+        using E = decltype(eng);
+        return with_nl<double, E, 8, 2, false>(L, [&](auto nlc) -> int {
+            constexpr int NL = decltype(nlc)::value;
+            auto kern = k_green_zlines<TO, NL, E>;
+            const size_t sm = eng_smem<E, double>(L, NL);
+            int rc = set_smem(kern, sm);
+            if (rc) return rc;
+            const unsigned nblk = (unsigned)ceil_div(((a.nq + 1) & ~(int64_t)1) * a.nb, 2 * NL);
+            kern<<<nblk, eng_threads<E>(a.p, NL), sm, st>>>(in, out, a, tw.st, tw.rt);
+            return launch_ok();
         });
     });
 }

@@ -109,20 +109,18 @@ CornerArgs green_corner_args(const int n[3], const double delta[3], double gamma
 // once to T; the line transforms run in T: FP64 for FP64 spectra, FP32 for the FP32 path,
 // whose stored spectrum is FP32 anyway.
 template <typename T>
-int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, const int odd[3][2], int zinner,
-                     int zpitch, T *out, int64_t out_bstride) {
+static int green_sym_xy(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, const int odd[3][2], T **out) {
     const int nxh = nx + 1, nyh = ny + 1;
     T *hx, *hy;
     TRY(ws_get(c, "green_hx", sizeof(T) * (size_t)nb * nxh * ny * nz, (void **)&hx));
     TRY(ws_get(c, "green_hy", sizeof(T) * (size_t)nb * nxh * nyh * nz, (void **)&hy));
-    FFTPlan px, py, pz;
-    if (!make_fft_plan(2 * nx, px) || !make_fft_plan(2 * ny, py) || !make_fft_plan(2 * nz, pz))
+    FFTPlan px, py;
+    if (!make_fft_plan(2 * nx, px) || !make_fft_plan(2 * ny, py))
         return set_err(c, OSC_E_FFT_SIZE, "doubled grid lengths must be 2^a 3^b 5^c");
-    TwPair<cplx<T>> twx, twy, twz;
+    TwPair<cplx<T>> twx, twy;
     TRY(twiddles<T>(c, 2 * nx, &twx));
     TRY(twiddles<T>(c, 2 * ny, &twy));
-    TRY(twiddles<T>(c, 2 * nz, &twz));
-    Launch L_(c, "green_sym_lines", 3);
+    Launch L_(c, "green_sym_lines", 2);
     SymArgs a;
     const std::string tp = sizeof(T) == 4 ? "f32" : "f64";
     // x: rows h[c][b][0..nx) -> hx[c][b][0..nx]
@@ -140,6 +138,22 @@ int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, con
     a.out_ps = (int64_t)nyh * nxh; a.out_qs = 1; a.out_es = nxh; a.out_bs = (int64_t)nxh * nyh * nz;
     a.nl_div = tune_get(c, "sym_nl_div:" + tp + ":L" + std::to_string(2 * ny));
     TRY(kerr(c, launch_sym_lines<T, T, T>(hx, hy, a, twy, false, false, c->stream), "green y"));
+    *out = hy;
+    return OSC_OK;
+}
+
+template <typename T>
+int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, const int odd[3][2], int zinner,
+                     int zpitch, T *out, int64_t out_bstride) {
+    const int nxh = nx + 1, nyh = ny + 1;
+    FFTPlan pz;
+    if (!make_fft_plan(2 * nz, pz)) return set_err(c, OSC_E_FFT_SIZE, "doubled grid lengths must be 2^a 3^b 5^c");
+    TwPair<cplx<T>> twz;
+    TRY(twiddles<T>(c, 2 * nz, &twz));
+    T *hy;
+    TRY(green_sym_xy<T>(c, h, nb, nx, ny, nz, odd, &hy));
+    Launch L_(c, "green_sym_lines", 1);
+    SymArgs a;
     // z: lines (ky, kx) of hy -> stored spectrum, scaled by fpei/M
     a.p = pz; a.n = nz; a.odd_lo = odd[2][0]; a.odd_hi = odd[2][1]; a.nq = nxh;
     a.npq = (int64_t)nyh * nxh; a.nb = nb;
@@ -151,7 +165,7 @@ int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, con
     }
     a.out_bs = out_bstride;
     a.scale = fpei_solver2() / (8.0 * nx * ny * nz);
-    a.nl_div = tune_get(c, "sym_nl_div:" + tp + ":L" + std::to_string(2 * nz));
+    a.nl_div = tune_get(c, std::string("sym_nl_div:") + (sizeof(T) == 4 ? "f32" : "f64") + ":L" + std::to_string(2 * nz));
     TRY(kerr(c, launch_sym_lines<T, T, T>(hy, out, a, twz, false, zinner != 0, c->stream), "green z"));
     return OSC_OK;
 }
@@ -223,13 +237,97 @@ static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[
     return OSC_OK;
 }
 
+// All components of a geometry whose kernel is displaced along z only (the cathode image's, or a
+// user's z offset): even or odd along x and y, so the x and y passes are the even/odd line
+// transforms of the cells of the whole doubled z range, and the z pass transforms real columns
+// (two per complex line) in FP64 throughout.  image: where the image z pass runs, half of z
+// is stored with the flip phase applied (the value at Nz - kz is par_x par_y times the conjugate
+// of that at kz).  Before, each component filled the complex doubled grid and took a
+// full FP64 3D transform of it: eight times the values, most of them zeros or mirror images (the
+// 64^3 cathode step with a refit mesh: 548 us that way, 381 this way).
+template <typename T>
+static int green_zoff_set(osc_ctx *c, int nx, int ny, int nz, const double delta[3], double gamma, double zoff,
+                          bool image, const int *comps, int ncomp, GreenSet &gs) {
+    const int Nz = 2 * nz, nxh = nx + 1, nyh = ny + 1;
+    double *h, *hy;
+    TRY(ws_get(c, "green_h", sizeof(double) * (size_t)ncomp * nx * ny * Nz, (void **)&h));
+    {
+        CellArgs ca;
+        ca.nx = nx;
+        ca.ny = ny;
+        ca.nz = nz;
+        ca.zwrap = 1;
+        ca.ncomp = ncomp;
+        for (int i = 0; i < ncomp; ++i) ca.comps[i] = comps[i];
+        ca.nmem = 1;
+        ca.hstride = (int64_t)nx * ny * Nz;
+        Launch L_(c, "green_cells");
+        TRY(kerr(c, launch_green_cells<double>(h, ca, cell_geom(delta[0], delta[1], delta[2] * gamma, gamma,
+                                                                zoff * gamma, kSerRatio), c->stream),
+                 "green cells"));
+    }
+    int odd[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    ZLineArgs za;
+    za.imag = 0;
+    for (int i = 0; i < ncomp; ++i)
+        if (comps[i] >= 1) {
+            odd[comps[i] - 1][0] = i;
+            odd[comps[i] - 1][1] = i + 1;
+            if (comps[i] <= 2) za.imag |= 1u << i;  // odd in x or y: i times a real transform
+        }
+    TRY(green_sym_xy<double>(c, h, ncomp, nx, ny, Nz, odd, &hy));
+    GSpecDev s{};
+    s.sym_y = 1;
+    s.zinner = zconv_warp_ok(Nz, nz, (int)sizeof(T)) ? 1 : 0;
+    s.herm_img = image && zconv_img_ok(Nz, nz, (int)sizeof(T)) ? 1 : 0;
+    s.dimy = nyh;
+    s.dimz = s.herm_img ? nz + 1 : Nz;
+    s.zpitch = s.zinner ? green_zpitch(s.dimz, sizeof(cplx<T>)) : s.dimz;
+    s.par_z = 1;
+    const int64_t per = (int64_t)nxh * nyh * s.zpitch;
+    DevBuf store;
+    TRY(green_alloc(c, sizeof(cplx<T>) * (size_t)per * ncomp, store));
+    int rc = s.zpitch > s.dimz ? cuda_check(c, cudaMemsetAsync(store.p, 0, store.bytes, c->stream), "memset spectra") : OSC_OK;
+    TwPair<cplx<double>> twz;
+    if (!rc && !make_fft_plan(Nz, za.p)) rc = set_err(c, OSC_E_FFT_SIZE, "doubled grid lengths must be 2^a 3^b 5^c");
+    if (!rc) rc = twiddles<double>(c, Nz, &twz);
+    if (!rc) {
+        za.nq = (int64_t)nxh * nyh;
+        za.nb = ncomp;
+        za.in_bs = za.nq * Nz;
+        za.out_bs = per;
+        za.dimz = s.dimz;
+        za.zpitch = s.zinner ? s.zpitch : 0;
+        za.fold = s.herm_img ? nz - 1 : -1;
+        za.scale = fpei_solver2() / (8.0 * nx * ny * nz);
+        Launch L_(c, "green_zlines");
+        rc = kerr(c, launch_green_zlines<T>(hy, reinterpret_cast<cplx<T> *>(store.p), za, twz, c->stream), "green z lines");
+    }
+    if (rc) {
+        green_release(c, store);
+        return rc;
+    }
+    const int base = gs.nspec;
+    gs.buf[base] = store;
+    gs.bytes += store.bytes;
+    for (int i = 0; i < ncomp; ++i) {
+        GSpecDev &d = gs.spec[base + i];
+        d = s;
+        d.data = reinterpret_cast<cplx<T> *>(store.p) + i * per;
+        d.par_y = comps[i] == 2 ? -1 : 1;
+        d.par_h = comps[i] == 1 || comps[i] == 2 ? -1 : 1;
+    }
+    gs.nspec += ncomp;
+    return OSC_OK;
+}
+
 // ------------------------------------------------------------------------------------
 // Green spectrum of one component (icomp 0 phi, 1..3 E) of a kernel with a non-zero offset
-// on some axis (all-symmetric kernels go through green_sym_set): corners, the centred
+// along x or y (the others go through green_sym_set and green_zoff_set): corners, the centred
 // complex doubled grid, an FP64 3D FFT and the extraction into the stored layout.
 template <typename T>
 static int build_green_component(osc_ctx *c, int nx, int ny, int nz, const double delta[3], double gamma,
-                                 const double off[3], int icomp, bool image, DevBuf &store, GSpecDev &spec) {
+                                 const double off[3], int icomp, DevBuf &store, GSpecDev &spec) {
     const int n[3] = {nx, ny, nz};
     const int N[3] = {2 * nx, 2 * ny, 2 * nz};
     const int64_t M = (int64_t)N[0] * N[1] * N[2];
@@ -270,15 +368,6 @@ static int build_green_component(osc_ctx *c, int nx, int ny, int nz, const doubl
     spec.dimz = sym[2] ? nz + 1 : N[2];
     spec.zinner = zconv_warp_ok(N[2], nz, (int)sizeof(T)) ? 1 : 0;
     spec.zpitch = spec.zinner ? green_zpitch(spec.dimz, spec.real_valued ? sizeof(T) : sizeof(cplx<T>)) : spec.dimz;
-    // an image spectrum even/odd in x and y: half of z stored, flip phase applied, for the
-    // image z pass (its value at Nz - kz is par_x par_y times the conjugate of that at kz)
-    const bool herm = image && sym[0] && sym[1] && !sym[2] && zconv_img_ok(N[2], nz, (int)sizeof(T));
-    if (herm) {
-        spec.dimz = nz + 1;
-        spec.zpitch = green_zpitch(spec.dimz, sizeof(cplx<T>));
-        spec.herm_img = 1;
-        spec.par_h = par[0] * par[1];
-    }
     const size_t elems = (size_t)(nx + 1) * spec.dimy * spec.zpitch;
     const size_t bytes = elems * (spec.real_valued ? sizeof(T) : sizeof(cplx<T>));
     TRY(green_alloc(c, bytes, store));
@@ -286,8 +375,7 @@ static int build_green_component(osc_ctx *c, int nx, int ny, int nz, const doubl
     {
         Launch L_(c, "green_extract");
         TRY(kerr(c, launch_green_extract<T>(cg, store.p, nx, N[0], N[1], spec.dimy, spec.dimz, spec.real_valued,
-                                            spec.imag_unit, scale, spec.zinner ? spec.zpitch : 0, herm ? nz - 1 : -1,
-                                            N[2], c->stream),
+                                            spec.imag_unit, scale, spec.zinner ? spec.zpitch : 0, c->stream),
                  "green extract"));
     }
     spec.data = store.p;
@@ -326,9 +414,17 @@ static int green_set(osc_ctx *c, const FreeSpaceJob &j, const int *comps, int nc
             }
             continue;
         }
+        if (off[0] == 0.0 && off[1] == 0.0) {
+            const int rc = green_zoff_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off[2], s == 1, comps, ncomp, gs);
+            if (rc) {
+                for (int q = 0; q < gs.nspec; ++q) green_release(c, gs.buf[q]);
+                return rc;
+            }
+            continue;
+        }
         for (int i = 0; i < ncomp; ++i) {
             const int k = gs.nspec;
-            int rc = build_green_component<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off, comps[i], s == 1,
+            int rc = build_green_component<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off, comps[i],
                                                        gs.buf[k], gs.spec[k]);
             if (rc) {
                 for (int q = 0; q <= k; ++q) green_release(c, gs.buf[q]);
