@@ -9,6 +9,11 @@ using namespace osc;
 using namespace osc_abi;
 
 
+namespace {
+int step_queue(osc_ctx *ctx, const osc_mesh3d *mesh, const int n[3], int64_t np, const double *x, const double *y,
+               const double *z, const double *q, double charge1, int at_cathode, int precision, double *E, double *B);
+}
+
 extern "C" {
 
 const char *osc_version(void) { return "opensc_b200 0.1.0 (sm_100a)"; }
@@ -29,6 +34,8 @@ int osc_ctx_create(int device, osc_ctx **out) {
         cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc(&ctx->d_small, sizeof(unsigned long long) * 64) != cudaSuccess ||
         cudaMallocHost(&ctx->h_small, sizeof(unsigned long long) * 64) != cudaSuccess ||
+        cudaMemset(ctx->d_small, 0, sizeof(unsigned long long) * 64) != cudaSuccess ||
+        cudaEventCreateWithFlags(&ctx->charge_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(&ctx->d_partials, sizeof(double) * 1024) != cudaSuccess ||
         cudaHostAlloc((void **)&ctx->h_fault, sizeof(unsigned), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void **)&ctx->d_fault, ctx->h_fault, 0) != cudaSuccess) {
@@ -60,6 +67,7 @@ int osc_ctx_destroy(osc_ctx *ctx) {
     for (auto e : ctx->ev_pool) cudaEventDestroy(e);
     if (ctx->d_small) cudaFree(ctx->d_small);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
+    if (ctx->charge_ev) cudaEventDestroy(ctx->charge_ev);
     if (ctx->d_partials) cudaFree(ctx->d_partials);
     if (ctx->h_fault) cudaFreeHost(ctx->h_fault);
     for (auto s : ctx->aux) cudaStreamDestroy(s);
@@ -164,7 +172,7 @@ int osc_ctx_set_tuning(osc_ctx *ctx, const char *key, int value) {
 
 int osc_ctx_get_tuning(osc_ctx *ctx, const char *key, int *value) {
     if (!ctx || !key || !value) return OSC_E_INVALID;
-    *value = tune_get(ctx, key, 0);
+    *value = tune_get(ctx, key);
     return OSC_OK;
 }
 
@@ -496,15 +504,28 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
     if (!q && !total_charge) return set_err(ctx, OSC_E_NOCHARGE, "Error, must specify qa or total_charge");
     if (!(mesh->gamma >= 1.0)) return set_err(ctx, OSC_E_INVALID, "gamma must be >= 1");
     ++ctx->step_calls;  // any earlier step's kept E grid is out of date from here on
-    if (resize_mesh) TRY(refit_mesh(ctx, np, x, y, z, mesh));
     double charge1 = 0;
-    if (q) TRY(set_charge(ctx, np, q, total_charge, mesh, &charge1));
-    else {
+    if (q) {
+        TRY(charge_queue(ctx, np, q, kChargeWord, false));
+    } else {
         mesh->charge = *total_charge;
         charge1 = *total_charge / (double)np;
     }
+    if (resize_mesh) TRY(refit_mesh(ctx, np, x, y, z, mesh));
+    const int rc = step_queue(ctx, mesh, n, np, x, y, z, q, charge1, at_cathode, precision, E, B);
+    const int rq = q ? charge_wait(ctx, kChargeWord, &mesh->charge) : OSC_OK;
+    return rc ? rc : rq;
+}
+
+}  // extern "C"
+
+namespace {
+// The step on a mesh and charges that are settled: everything queued, nothing waited for.
+int step_queue(osc_ctx *ctx, const osc_mesh3d *mesh, const int n[3], int64_t np, const double *x, const double *y,
+               const double *z, const double *q, double charge1, int at_cathode, int precision, double *E, double *B) {
     const int64_t N = (int64_t)n[0] * n[1] * n[2];
-    TRY(counters_reset(ctx));
+    const bool quad_step = precision == OSC_PREC_FP32 && ctx->deposit_mode == OSC_DEPOSIT_ATOMIC;
+    if (!quad_step) TRY(counters_reset(ctx));  // else cleared with the quad grid
     DepositArgs da = deposit_args(mesh, n, np, x, y, z, q, charge1, ctx->check_finite);
     InterpArgs ia = interp_args(mesh, n, np, x, y, z);
     FreeSpaceJob j = fs_job(mesh, n, nullptr, at_cathode, B != nullptr);
@@ -555,9 +576,9 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
             TRY(deposit_rho<float>(ctx, da, rho, N, 1.0, order != OSC_ORDER_ANY));
         } else {
             TRY(ws_get(ctx, "st_quad", sizeof(float) * 4 * N, (void **)&quad));
-            CK(cudaMemsetAsync(quad, 0, sizeof(float) * 4 * N, ctx->stream), "memset quad");
             {
-                Launch L_(ctx, order == OSC_ORDER_ANY ? "deposit_f32" : "deposit_f32_runs");
+                Launch L_(ctx, order == OSC_ORDER_ANY ? "deposit_f32" : "deposit_f32_runs", 2);
+                if (launch_clear_quad(quad, N, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "clear quad");
                 if ((order == OSC_ORDER_ANY ? launch_deposit_quad(da, quad, ctx->d_small, ctx->stream)
                                             : launch_deposit_quad_runs(da, quad, ctx->d_small, ctx->stream)))
                     return set_err(ctx, OSC_E_CUDA, "deposit");
@@ -634,6 +655,9 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
     }
     return OSC_OK;
 }
+}  // namespace
+
+extern "C" {
 
 int osc_space_charge_step(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const double *x, const double *y,
                           const double *z, const double *q, const double *total_charge, int resize_mesh,

@@ -93,35 +93,44 @@ inline void apply_refit(osc_mesh3d *mesh, const double bmin[3], const double bma
 // the particle bounding box computed on the device.
 inline int refit_mesh(osc_ctx *ctx, int64_t np, const double *x, const double *y, const double *z, osc_mesh3d *mesh) {
     if (np <= 0) return set_err(ctx, OSC_E_INVALID, "resize_mesh needs at least one particle");
-    double *bb;
-    TRY(ws_get(ctx, "bbox", sizeof(double) * 8, (void **)&bb));
+    unsigned long long *part;
+    TRY(ws_get(ctx, "bbox_part", sizeof(unsigned long long) * bbox_scratch_words(), (void **)&part));
+    double *hb = reinterpret_cast<double *>(ctx->h_small + 16);
     {
-        Launch L_(ctx, "bbox", 3);
-        TRY(launch_bbox(np, x, y, z, ctx->d_small + 8, bb, ctx->d_small + 16, ctx->stream) ? set_err(ctx, OSC_E_CUDA, "bbox") : 0);
+        Launch L_(ctx, "bbox");
+        if (launch_bbox(np, x, y, z, part, reinterpret_cast<unsigned *>(ctx->d_small + 40), hb, ctx->stream))
+            return set_err(ctx, OSC_E_CUDA, "bbox");
     }
-    double hb[6];
-    TRY(d2h(ctx, hb, bb, sizeof(hb)));
-    TRY(d2h(ctx, ctx->h_small + 16, ctx->d_small + 16, sizeof(unsigned long long)));
     TRY(sync(ctx));
-    if (ctx->h_small[16]) return set_err(ctx, OSC_E_NAN, "%llu non-finite particle coordinates", ctx->h_small[16]);
+    if (hb[6] > 0) return set_err(ctx, OSC_E_NAN, "%.0f non-finite particle coordinates", hb[6]);
     const double mn[3] = {hb[0], hb[2], hb[4]}, mx[3] = {hb[1], hb[3], hb[5]};
     apply_refit(mesh, mn, mx);
     return OSC_OK;
 }
 
+// Queues the sum (or largest magnitude) of q into pinned word `word`; charge_wait returns it.
+inline int charge_queue(osc_ctx *ctx, int64_t np, const double *q, int word, bool max_abs) {
+    Launch L_(ctx, max_abs ? "charge_max" : "charge_sum");
+    if (launch_sum(np, q, ctx->d_partials, reinterpret_cast<unsigned *>(ctx->d_small + 41),
+                   reinterpret_cast<double *>(ctx->h_small + word), ctx->stream, max_abs))
+        return set_err(ctx, OSC_E_CUDA, "charge sum");
+    CK(cudaEventRecord(ctx->charge_ev, ctx->stream), "record charge");
+    return OSC_OK;
+}
+// The host needs the charge only to report it, so it waits for the sum's event alone, after the
+// rest of the step is queued: the GPU does not idle in between.
+inline int charge_wait(osc_ctx *ctx, int word, double *v) {
+    CK(cudaEventSynchronize(ctx->charge_ev), "wait for charge");
+    *v = *reinterpret_cast<volatile double *>(ctx->h_small + word);
+    return OSC_OK;
+}
+constexpr int kChargeWord = 24, kChargeMaxWord = 25;
+
 inline int set_charge(osc_ctx *ctx, int64_t np, const double *q, const double *total_charge, osc_mesh3d *mesh,
                double *charge1) {
     if (q) {
-        double *out;
-        TRY(ws_get(ctx, "qsum", sizeof(double), (void **)&out));
-        {
-            Launch L_(ctx, "charge_sum", 2);
-            if (launch_sum(np, q, ctx->d_partials, out, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "charge sum");
-        }
-        double s = 0;
-        TRY(d2h(ctx, &s, out, sizeof(double)));
-        TRY(sync(ctx));
-        mesh->charge = s;
+        TRY(charge_queue(ctx, np, q, kChargeWord, false));
+        TRY(charge_wait(ctx, kChargeWord, &mesh->charge));
         *charge1 = 0;
     } else if (total_charge) {
         mesh->charge = *total_charge;
@@ -233,15 +242,8 @@ inline int deposit_rho(osc_ctx *ctx, DepositArgs a, TR *rho, int64_t N, double m
     }
     double qmax;
     if (a.mode == 0 && a.q) {
-        double *out;
-        TRY(ws_get(ctx, "qmax", sizeof(double), (void **)&out));
-        {
-            Launch L_(ctx, "charge_max", 2);
-            if (launch_sum(a.np, a.q, ctx->d_partials, out, ctx->stream, true))
-                return set_err(ctx, OSC_E_CUDA, "charge max");
-        }
-        TRY(d2h(ctx, &qmax, out, sizeof(double)));
-        TRY(sync(ctx));
+        TRY(charge_queue(ctx, a.np, a.q, kChargeMaxWord, true));
+        TRY(charge_wait(ctx, kChargeMaxWord, &qmax));
     } else {
         qmax = a.mode == 0 ? std::fabs(a.charge1) : 1.0;
     }

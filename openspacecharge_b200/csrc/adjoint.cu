@@ -48,7 +48,6 @@ int osc_space_charge_step_vjp_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int64_t 
         TRY(ws_get(ctx, "vjp_lambda", sizeof(double) * N, (void **)&lam));
         TRY(counters_reset(ctx));
         CK(cudaMemsetAsync(quad3, 0, sizeof(float4) * 3 * N, ctx->stream), "memset quad3");
-        CK(cudaMemsetAsync(lam, 0, sizeof(double) * N, ctx->stream), "memset lambda");  // three-solve path
         if (reuse) {
             e8 = reinterpret_cast<float *>(f.e8);
         } else {
@@ -82,6 +81,7 @@ int osc_space_charge_step_vjp_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int64_t 
             js.acc_coef = -1.0;
             TRY(freespace_opt<float, float>(ctx, js, nullptr));
         } else {
+            CK(cudaMemsetAsync(lam, 0, sizeof(double) * N, ctx->stream), "memset lambda");
             for (int c = 0; c < 3; ++c) {
                 FreeSpaceJob jc = fs_job(mesh, n, nullptr, 0, 0);
                 jc.quad = reinterpret_cast<const float4 *>(quad3) + c * N;

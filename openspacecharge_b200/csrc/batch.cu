@@ -395,7 +395,6 @@ int batch_issue(osc_ctx *ctx, BatchPlan &P) {
         const int zp = zinner ? green_zpitch(nz + 1, sizeof(float)) : nz + 1;
         const int64_t per = (int64_t)(nx + 1) * (ny + 1) * zp;
         TRY(ws_get(ctx, "green_h", sizeof(float) * 3 * (size_t)B * nx * ny * nz, (void **)&h));
-        if (zinner) CK(cudaMemsetAsync(gbuf, 0, sizeof(float) * 3 * B * per, ctx->stream), "memset spectra");
         // Green spectra of the three E components of every member: members m = comp*B + i
         {
             CellArgs ca;

@@ -25,7 +25,12 @@ int cuda_check(osc_ctx *c, cudaError_t e, const char *what) {
 
 int ws_get(osc_ctx *c, const char *name, size_t bytes, void **out) {
     // work running on an auxiliary stream slot gets its own copy of every workspace
-    DevBuf &b = c->ws_slot ? c->ws[std::string(name) + "#" + std::to_string(c->ws_slot)] : c->ws[name];
+    auto slot = [&]() -> DevBuf & {
+        if (c->ws_slot) return c->ws[std::string(name) + "#" + std::to_string(c->ws_slot)];
+        auto it = c->ws.find(name);
+        return it != c->ws.end() ? it->second : c->ws[name];
+    };
+    DevBuf &b = slot();
     if (bytes == 0) bytes = 16;
     if (b.bytes < bytes) {
         if (c->capturing) return set_err(c, OSC_E_UNSUPPORTED, "workspace '%s' would grow during graph capture", name);
@@ -189,9 +194,16 @@ Launch::~Launch() {
     }
 }
 
-int tune_get(const osc_ctx *c, const std::string &key, int def) {
+int tune_get(const osc_ctx *c, const char *key, int def) {
+    if (c->tuning.empty()) return def;
     auto it = c->tuning.find(key);
     return it == c->tuning.end() ? def : it->second;
+}
+int tune_len(const osc_ctx *c, const char *family, size_t tbytes, int len) {
+    if (c->tuning.empty()) return 0;
+    char key[64];
+    snprintf(key, sizeof(key), "%s:%s:L%d", family, tbytes == 4 ? "f32" : "f64", len);
+    return tune_get(c, key);
 }
 
 int prof_flush(osc_ctx *c) {

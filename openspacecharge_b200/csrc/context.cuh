@@ -75,7 +75,7 @@ struct osc_ctx {
     int deposit_mode = 0;
     int particle_order = 0;  // OSC_ORDER_*
     // launch shapes picked by the autotuner (osc_ctx_set_tuning), by key; absent = default
-    std::map<std::string, int> tuning;
+    std::map<std::string, int, std::less<>> tuning;
     int strict_bounds = 0;
     int profile = 0;
     int check_finite = 0;
@@ -103,7 +103,7 @@ struct osc_ctx {
     // captured batched steps by call signature (batch.cu), most recently used first
     std::list<std::shared_ptr<void>> batch_plans;
     // workspaces by name
-    std::map<std::string, osc::DevBuf> ws;
+    std::map<std::string, osc::DevBuf, std::less<>> ws;
     std::map<int, osc::DevBuf> tw32, tw64;
     std::list<osc::GreenSet> gcache;
     // spectrum buffers of evicted sets, reused (same byte size) by the next builds; all
@@ -111,8 +111,9 @@ struct osc_ctx {
     std::vector<osc::DevBuf> gpool;
     uint64_t stamp = 0;
     // small device/pinned scratch for counters and reductions
-    unsigned long long *d_small = nullptr;  // 64 words
-    unsigned long long *h_small = nullptr;  // pinned 64 words
+    unsigned long long *d_small = nullptr;  // 64 words (40, 41: tickets of bbox and charge sum)
+    unsigned long long *h_small = nullptr;  // pinned, mapped, 64 words
+    cudaEvent_t charge_ev = nullptr;        // recorded after a charge sum
     double *d_partials = nullptr;           // 1024 doubles
     // host-mapped word where kernels report bounded waits that gave up (0 = none)
     unsigned *h_fault = nullptr;
@@ -147,8 +148,10 @@ struct Launch {
     ~Launch();
 };
 int prof_flush(osc_ctx *c);
-// Tuned value of `key` (autotuner), or def when none was set.
-int tune_get(const osc_ctx *c, const std::string &key, int def = 0);
+// Tuned value of `key` (autotuner), or def when none was set; tune_len: of the key
+// "<family>:<f32|f64>:L<length>".
+int tune_get(const osc_ctx *c, const char *key, int def = 0);
+int tune_len(const osc_ctx *c, const char *family, size_t tbytes, int len);
 
 // Green-spectrum cache.  A budget of 0 disables it: every solve rebuilds its spectra (the
 // reference's behaviour, code/open_spacecharge_mod.f90:570-573) into reused buffers.

@@ -149,6 +149,17 @@ __device__ __forceinline__ int quad_one(const DepositArgs &a, float4 *__restrict
     return 0;
 }
 
+// Clears a quad grid and the counters in one launch.
+__global__ void __launch_bounds__(256) k_clear_quad(float4 *__restrict__ quad, int64_t n, unsigned long long *counters) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    GRID_STRIDE(i, n) quad[i] = z;
+    if (blockIdx.x == 0 && threadIdx.x < 8) counters[threadIdx.x] = 0;
+}
+int launch_clear_quad(float *quad, int64_t nodes, unsigned long long *counters, cudaStream_t st) {
+    k_clear_quad<<<nblocks(nodes, 256, 148 * 8), 256, 0, st>>>(reinterpret_cast<float4 *>(quad), nodes, counters);
+    return ok();
+}
+
 __global__ void __launch_bounds__(256) k_deposit_quad(DepositArgs a, float4 *__restrict__ quad,
                                                       unsigned long long *__restrict__ counters) {
     const int64_t plane = (int64_t)a.nx * a.ny;
@@ -563,13 +574,24 @@ __device__ __forceinline__ double ord_val(unsigned long long u) {
     return __longlong_as_double((long long)b);
 }
 
-__global__ void k_bbox_init(unsigned long long *keys, unsigned long long *nonfinite) {
-    if (threadIdx.x < 6) keys[threadIdx.x] = (threadIdx.x & 1) ? 0ull : ~0ull;
-    if (threadIdx.x == 0) *nonfinite = 0;
+// True in exactly one block of a launch, the last one to get here; what the other blocks wrote
+// before is visible to it.  The ticket wraps to 0 with the last block, ready for the next launch.
+__device__ __forceinline__ bool last_block(unsigned *ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
 }
+
+// Bounding box and non-finite count: every block leaves its seven words in part, and the last
+// block reduces them into out (mapped host memory), so that one launch and the wait for the
+// stream give the host its result (three launches and two copies before).
 __global__ void __launch_bounds__(256) k_bbox(int64_t np, const double *__restrict__ x, const double *__restrict__ y,
-                                              const double *__restrict__ z, unsigned long long *keys,
-                                              unsigned long long *nonfinite) {
+                                              const double *__restrict__ z, unsigned long long *part,
+                                              unsigned *ticket, double *out) {
     unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
     unsigned long long bad = 0;
     const double *p[3] = {x, y, z};
@@ -598,64 +620,95 @@ __global__ void __launch_bounds__(256) k_bbox(int64_t np, const double *__restri
             }
         }
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        for (int off = 16; off; off >>= 1) {
-            const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo[d], off);
-            const unsigned long long b = __shfl_xor_sync(0xffffffffu, hi[d], off);
-            lo[d] = a < lo[d] ? a : lo[d];
-            hi[d] = b > hi[d] ? b : hi[d];
-        }
-    }
-    for (int off = 16; off; off >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, off);
-    // the block's warps combine in shared memory, then one thread adds the block's extremes:
-    // seven atomics per block instead of per warp on the same seven words
     __shared__ unsigned long long sk[8][7];
-    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
+    // the block's extremes in thread 0
+    auto block_reduce = [&]() {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            sk[w][2 * d] = lo[d];
-            sk[w][2 * d + 1] = hi[d];
+            for (int off = 16; off; off >>= 1) {
+                const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo[d], off);
+                const unsigned long long b = __shfl_xor_sync(0xffffffffu, hi[d], off);
+                lo[d] = a < lo[d] ? a : lo[d];
+                hi[d] = b > hi[d] ? b : hi[d];
+            }
         }
-        sk[w][6] = bad;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int v = 1; v < nw; ++v)
+        for (int off = 16; off; off >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, off);
+        const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        if ((threadIdx.x & 31) == 0) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                lo[d] = sk[v][2 * d] < lo[d] ? sk[v][2 * d] : lo[d];
-                hi[d] = sk[v][2 * d + 1] > hi[d] ? sk[v][2 * d + 1] : hi[d];
+                sk[w][2 * d] = lo[d];
+                sk[w][2 * d + 1] = hi[d];
             }
-        for (int v = 1; v < nw; ++v) bad += sk[v][6];
+            sk[w][6] = bad;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int v = 1; v < nw; ++v)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    lo[d] = sk[v][2 * d] < lo[d] ? sk[v][2 * d] : lo[d];
+                    hi[d] = sk[v][2 * d + 1] > hi[d] ? sk[v][2 * d + 1] : hi[d];
+                }
+            for (int v = 1; v < nw; ++v) bad += sk[v][6];
+        }
+    };
+    block_reduce();
+    if (threadIdx.x == 0) {
+        unsigned long long *q = part + 7 * (int64_t)blockIdx.x;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            atomicMin(&keys[2 * d], lo[d]);
-            atomicMax(&keys[2 * d + 1], hi[d]);
+            q[2 * d] = lo[d];
+            q[2 * d + 1] = hi[d];
         }
-        if (bad) atomicAdd(nonfinite, bad);
+        q[6] = bad;
+    }
+    if (!last_block(ticket)) return;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = ~0ull;
+        hi[d] = 0;
+    }
+    bad = 0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+        const unsigned long long *q = part + 7 * (int64_t)b;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const unsigned long long l = __ldcg(q + 2 * d), h = __ldcg(q + 2 * d + 1);
+            lo[d] = l < lo[d] ? l : lo[d];
+            hi[d] = h > hi[d] ? h : hi[d];
+        }
+        bad += __ldcg(q + 6);
+    }
+    block_reduce();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            out[2 * d] = ord_val(lo[d]);
+            out[2 * d + 1] = ord_val(hi[d]);
+        }
+        out[6] = (double)bad;
     }
 }
-__global__ void k_bbox_final(const unsigned long long *keys, double *bb) {
-    if (threadIdx.x < 6) bb[threadIdx.x] = ord_val(keys[threadIdx.x]);
-}
-int launch_bbox(int64_t np, const double *x, const double *y, const double *z, unsigned long long *keys, double *bb,
-                unsigned long long *nonfinite, cudaStream_t st) {
-    k_bbox_init<<<1, 32, 0, st>>>(keys, nonfinite);
-    if (np > 0) k_bbox<<<nblocks(np, 256, 148 * 16), 256, 0, st>>>(np, x, y, z, keys, nonfinite);
-    k_bbox_final<<<1, 32, 0, st>>>(keys, bb);
+int bbox_scratch_words() { return 7 * 148 * 8; }
+int launch_bbox(int64_t np, const double *x, const double *y, const double *z, unsigned long long *part,
+                unsigned *ticket, double *out, cudaStream_t st) {
+    // eight resident blocks per SM at most: each block's partial result is one more to reduce
+    k_bbox<<<nblocks(np, 256, 148 * 8), 256, 0, st>>>(np, x, y, z, part, ticket, out);
     return ok();
 }
 
-// Deterministic two-pass reductions of a particle array: op 0 sum, 1 maximum of |q|.
+// Deterministic reductions of a particle array (op 0 sum, 1 maximum of |q|): 1024 block partials,
+// which the last block combines in a fixed order into out (mapped host memory).
 __device__ __forceinline__ double red_op(double a, double b, int op) { return op ? fmax(a, b) : a + b; }
-__global__ void __launch_bounds__(256) k_sum_partial(int64_t n, const double *__restrict__ q, double *partials, int op) {
-    __shared__ double sh[256];
+__global__ void __launch_bounds__(256) k_sum(int64_t n, const double *__restrict__ q, double *partials,
+                                             unsigned *ticket, double *out, int op) {
+    __shared__ double sh[1024];
     double s = 0;
     const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
     const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
-    for (int64_t m = beg + threadIdx.x; m < end; m += blockDim.x) s = red_op(s, op ? fabs(q[m]) : q[m], op);
+#pragma unroll 4
+    for (int64_t m = beg + threadIdx.x; m < end; m += blockDim.x) s = red_op(s, op ? fabs(__ldg(q + m)) : __ldg(q + m), op);
     sh[threadIdx.x] = s;
     __syncthreads();
     for (int w = 128; w; w >>= 1) {
@@ -663,20 +716,18 @@ __global__ void __launch_bounds__(256) k_sum_partial(int64_t n, const double *__
         __syncthreads();
     }
     if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
-}
-__global__ void k_sum_final(const double *partials, int np, double *out, int op) {
-    __shared__ double sh[1024];
-    sh[threadIdx.x] = threadIdx.x < np ? partials[threadIdx.x] : 0.0;
+    if (!last_block(ticket)) return;
+    for (int t = threadIdx.x; t < 1024; t += 256) sh[t] = t < gridDim.x ? __ldcg(partials + t) : 0.0;
     __syncthreads();
     for (int w = 512; w; w >>= 1) {
-        if (threadIdx.x < w) sh[threadIdx.x] = red_op(sh[threadIdx.x], sh[threadIdx.x + w], op);
+        for (int t = threadIdx.x; t < w; t += 256) sh[t] = red_op(sh[t], sh[t + w], op);
         __syncthreads();
     }
     if (threadIdx.x == 0) *out = sh[0];
 }
-int launch_sum(int64_t n, const double *q, double *partials, double *out, cudaStream_t st, bool max_abs) {
-    k_sum_partial<<<1024, 256, 0, st>>>(n, q, partials, max_abs ? 1 : 0);
-    k_sum_final<<<1, 1024, 0, st>>>(partials, 1024, out, max_abs ? 1 : 0);
+int launch_sum(int64_t n, const double *q, double *partials, unsigned *ticket, double *out, cudaStream_t st,
+               bool max_abs) {
+    k_sum<<<1024, 256, 0, st>>>(n, q, partials, ticket, out, max_abs ? 1 : 0);
     return ok();
 }
 

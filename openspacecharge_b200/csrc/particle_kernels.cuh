@@ -70,6 +70,8 @@ int launch_fixed_to_real(const unsigned long long *acc, TO *out, double fx_scale
 // (i,j,k) holds the plane-k contributions to nodes (i,j), (i+1,j), (i,j+1), (i+1,j+1)),
 // then launch_quad_to_nodes sums every node's four slots in a fixed order.
 int launch_deposit_quad(const DepositArgs &a, float *quad, unsigned long long *counters, cudaStream_t st);
+// Zeroes `nodes` quad nodes and the eight counter words.
+int launch_clear_quad(float *quad, int64_t nodes, unsigned long long *counters, cudaStream_t st);
 int launch_quad_to_nodes(const float *quad, float *rho, int nx, int ny, int nz, cudaStream_t st);
 
 // CIC gather (interpolate_field, code/open_spacecharge_mod.f90:311-390): clamp cells to
@@ -102,15 +104,16 @@ int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsign
 int launch_interp_pairs_runs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
                              cudaStream_t st, double *B = nullptr, double bcoef = 0);
 
-// Bounding box {xmin,xmax,ymin,ymax,zmin,zmax} of the particles, written to bb (device)
-// through order-preserving 64-bit keys; also counts non-finite coordinates.
-int launch_bbox(int64_t np, const double *x, const double *y, const double *z,
-                unsigned long long *keys /*6*/, double *bb /*6*/, unsigned long long *nonfinite,
-                cudaStream_t st);
-// Deterministic sum of q (two passes, fixed order) into *out.
-// Sum of q (or, with max_abs, the largest |q|), reduced in a fixed order.
-int launch_sum(int64_t n, const double *q, double *partials /*>= 1024*/, double *out, cudaStream_t st,
-               bool max_abs = false);
+// Bounding box {xmin,xmax,ymin,ymax,zmin,zmax} and number of non-finite coordinates of np >= 1
+// particles, written to out[7] (host memory mapped into the device).  part: bbox_scratch_words()
+// words; ticket: zero before its first use, left zero.
+int bbox_scratch_words();
+int launch_bbox(int64_t np, const double *x, const double *y, const double *z, unsigned long long *part,
+                unsigned *ticket, double *out, cudaStream_t st);
+// Sum of q (or, with max_abs, the largest |q|), reduced in a fixed order into *out (mapped host
+// memory); ticket as above.
+int launch_sum(int64_t n, const double *q, double *partials /*>= 1024*/, unsigned *ticket, double *out,
+               cudaStream_t st, bool max_abs = false);
 
 // ---- batches of bunches ---------------------------------------------------------------
 // One CTA's share of a batched particle pass: particles [beg, end) of bunch `bunch`.

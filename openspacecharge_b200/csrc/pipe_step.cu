@@ -24,16 +24,13 @@ int osc_space_charge_step_rectpipe_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int
     if (np <= 0 || !x || !y || !z || !E) return bad(ctx, "pipe step arrays");
     if (!q && !total_charge) return set_err(ctx, OSC_E_NOCHARGE, "Error, must specify qa or total_charge");
     const int64_t N = (int64_t)n[0] * n[1] * n[2];
-    osc_mesh3d m = *mesh;
-    double charge1 = 0;
-    if (q) TRY(set_charge(ctx, np, q, total_charge, &m, &charge1));
-    else charge1 = *total_charge / (double)np;
+    const osc_mesh3d m = *mesh;
+    const double charge1 = q ? 0.0 : *total_charge / (double)np;
     double *rho, *phi, *Eg, *Bg;
     TRY(ws_get(ctx, "ps_rho64", sizeof(double) * N, (void **)&rho));
     TRY(ws_get(ctx, "ps_phi", sizeof(double) * N, (void **)&phi));
     TRY(ws_get(ctx, "ps_E", sizeof(double) * 3 * N, (void **)&Eg));
     TRY(ws_get(ctx, "ps_B", sizeof(double) * 3 * N, (void **)&Bg));
-    TRY(counters_reset(ctx));
     DepositArgs da = deposit_args(&m, n, np, x, y, z, q, charge1, ctx->check_finite);
     InterpArgs ia = interp_args(&m, n, np, x, y, z);
     const bool fp32 = precision == OSC_PREC_FP32 && ctx->deposit_mode == OSC_DEPOSIT_ATOMIC;
@@ -43,9 +40,9 @@ int osc_space_charge_step_rectpipe_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int
         float *quad, *e8;
         TRY(ws_get(ctx, "ps_quad", sizeof(float) * 4 * N, (void **)&quad));
         TRY(ws_get(ctx, "ps_E8", sizeof(float) * 8 * N, (void **)&e8));
-        CK(cudaMemsetAsync(quad, 0, sizeof(float) * 4 * N, ctx->stream), "memset quad");
         {
-            Launch L_(ctx, "deposit_f32");
+            Launch L_(ctx, "deposit_f32", 2);
+            if (launch_clear_quad(quad, N, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "clear quad");
             if (launch_deposit_quad(da, quad, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "deposit");
         }
         TRY(pipe_solve_checked(ctx, &m, precision, nullptr, phi, nullptr, nullptr,
@@ -60,9 +57,9 @@ int osc_space_charge_step_rectpipe_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int
         float *quad, *rho32;
         TRY(ws_get(ctx, "ps_quad", sizeof(float) * 4 * N, (void **)&quad));
         TRY(ws_get(ctx, "ps_rho32", sizeof(float) * N, (void **)&rho32));
-        CK(cudaMemsetAsync(quad, 0, sizeof(float) * 4 * N, ctx->stream), "memset quad");
         {
-            Launch L_(ctx, "deposit_f32");
+            Launch L_(ctx, "deposit_f32", 2);
+            if (launch_clear_quad(quad, N, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "clear quad");
             if (launch_deposit_quad(da, quad, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "deposit");
         }
         {
@@ -75,6 +72,7 @@ int osc_space_charge_step_rectpipe_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int
             if (launch_f32_to_f64(rho32, rho, N, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "rho to f64");
         }
     } else {
+        TRY(counters_reset(ctx));
         TRY(deposit_rho<double>(ctx, da, rho, N, 1.0));
     }
     TRY(osc_space_charge_rectpipe_dev(ctx, &m, rho, apipe, bpipe, 0, 1, precision, phi, Eg, Bg));

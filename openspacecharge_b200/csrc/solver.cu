@@ -9,7 +9,6 @@
 // real or imaginary.  The cathode image (-rho flipped in z) is folded into the same
 // spectral product, so the image costs one more spectrum read, not one more solve.
 #include <cstring>
-#include <sstream>
 #include <type_traits>
 
 #include "solver.cuh"
@@ -122,21 +121,20 @@ static int green_sym_xy(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, 
     TRY(twiddles<T>(c, 2 * ny, &twy));
     Launch L_(c, "green_sym_lines", 2);
     SymArgs a;
-    const std::string tp = sizeof(T) == 4 ? "f32" : "f64";
     // x: rows h[c][b][0..nx) -> hx[c][b][0..nx]
     a.p = px; a.n = nx; a.odd_lo = odd[0][0]; a.odd_hi = odd[0][1]; a.nq = ny;
     a.npq = (int64_t)ny * nz; a.nb = nb;
     a.in_ps = (int64_t)ny * nx; a.in_qs = nx; a.in_es = 1; a.in_bs = (int64_t)nx * ny * nz;
     a.out_ps = (int64_t)ny * nxh; a.out_qs = nxh; a.out_es = 1; a.out_bs = (int64_t)nxh * ny * nz;
     a.scale = 1.0;
-    a.nl_div = tune_get(c, "sym_nl_div:" + tp + ":L" + std::to_string(2 * nx));
+    a.nl_div = tune_len(c, "sym_nl_div", sizeof(T), 2 * nx);
     TRY(kerr(c, launch_sym_lines<T, T, T>(h, hx, a, twx, true, true, c->stream), "green x"));
     // y: lines (c, kx) of hx -> hy[c][ky][kx]
     a.p = py; a.n = ny; a.odd_lo = odd[1][0]; a.odd_hi = odd[1][1]; a.nq = nxh;
     a.npq = (int64_t)nz * nxh; a.nb = nb;
     a.in_ps = (int64_t)ny * nxh; a.in_qs = 1; a.in_es = nxh; a.in_bs = (int64_t)nxh * ny * nz;
     a.out_ps = (int64_t)nyh * nxh; a.out_qs = 1; a.out_es = nxh; a.out_bs = (int64_t)nxh * nyh * nz;
-    a.nl_div = tune_get(c, "sym_nl_div:" + tp + ":L" + std::to_string(2 * ny));
+    a.nl_div = tune_len(c, "sym_nl_div", sizeof(T), 2 * ny);
     TRY(kerr(c, launch_sym_lines<T, T, T>(hx, hy, a, twy, false, false, c->stream), "green y"));
     *out = hy;
     return OSC_OK;
@@ -165,7 +163,7 @@ int green_sym_lines3(osc_ctx *c, const T *h, int nb, int nx, int ny, int nz, con
     }
     a.out_bs = out_bstride;
     a.scale = fpei_solver2() / (8.0 * nx * ny * nz);
-    a.nl_div = tune_get(c, std::string("sym_nl_div:") + (sizeof(T) == 4 ? "f32" : "f64") + ":L" + std::to_string(2 * nz));
+    a.nl_div = tune_len(c, "sym_nl_div", sizeof(T), 2 * nz);
     TRY(kerr(c, launch_sym_lines<T, T, T>(hy, out, a, twz, false, zinner != 0, c->stream), "green z"));
     return OSC_OK;
 }
@@ -210,8 +208,8 @@ static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[
             odd[comps[i] - 1][0] = i;
             odd[comps[i] - 1][1] = i + 1;
         }
-    int rc = zinner ? cuda_check(c, cudaMemsetAsync(store.p, 0, store.bytes, c->stream), "memset spectra") : OSC_OK;
-    if (!rc) rc = green_sym_lines3<T>(c, h, ncomp, nx, ny, nz, odd, zinner, zp, reinterpret_cast<T *>(store.p), per);
+    // the padding of a column (up to 16 bytes) is copied along with it and never used
+    const int rc = green_sym_lines3<T>(c, h, ncomp, nx, ny, nz, odd, zinner, zp, reinterpret_cast<T *>(store.p), per);
     if (rc) {
         green_release(c, store);
         return rc;
@@ -287,7 +285,7 @@ static int green_zoff_set(osc_ctx *c, int nx, int ny, int nz, const double delta
     const int64_t per = (int64_t)nxh * nyh * s.zpitch;
     DevBuf store;
     TRY(green_alloc(c, sizeof(cplx<T>) * (size_t)per * ncomp, store));
-    int rc = s.zpitch > s.dimz ? cuda_check(c, cudaMemsetAsync(store.p, 0, store.bytes, c->stream), "memset spectra") : OSC_OK;
+    int rc = OSC_OK;
     TwPair<cplx<double>> twz;
     if (!rc && !make_fft_plan(Nz, za.p)) rc = set_err(c, OSC_E_FFT_SIZE, "doubled grid lengths must be 2^a 3^b 5^c");
     if (!rc) rc = twiddles<double>(c, Nz, &twz);
@@ -383,13 +381,22 @@ static int build_green_component(osc_ctx *c, int nx, int ny, int nz, const doubl
 }
 
 static std::string fs_key(const FreeSpaceJob &j, int tbytes, const int *comps, int ncomp) {
-    std::ostringstream s;
-    s.precision(17);
-    s << "fs|" << tbytes << "|" << j.nx << "," << j.ny << "," << j.nz << "|" << j.delta[0] << "," << j.delta[1]
-      << "," << j.delta[2] << "|" << j.gamma << "|" << j.offset[0] << "," << j.offset[1] << "," << j.offset[2]
-      << "|" << (j.at_cathode ? j.img_zoff : 0.0) << "|" << j.at_cathode << "|";
-    for (int i = 0; i < ncomp; ++i) s << comps[i];
-    return s.str();
+    // the bytes of everything the spectra depend on (-0 and 0 the same)
+    struct {
+        int64_t i[5];
+        double d[8];
+    } k = {};
+    k.i[0] = tbytes;
+    k.i[1] = ((int64_t)j.nx << 40) | ((int64_t)j.ny << 20) | j.nz;
+    k.i[2] = j.at_cathode;
+    for (int i = 0; i < ncomp; ++i) k.i[3] = 8 * k.i[3] + comps[i] + 1;
+    for (int d = 0; d < 3; ++d) {
+        k.d[d] = j.delta[d] + 0.0;
+        k.d[3 + d] = j.offset[d] + 0.0;
+    }
+    k.d[6] = j.gamma;
+    k.d[7] = (j.at_cathode ? j.img_zoff : 0.0) + 0.0;
+    return std::string(reinterpret_cast<const char *>(&k), sizeof(k));
 }
 
 // Cached Green set for a job: spectra [direct comps..., image comps...].
@@ -555,8 +562,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     ra.nrows = (int64_t)Bin * ny * nz;
     ra.in_rstride = nx;
     ra.out_rstride = nxh;
-    const std::string tprec = sizeof(T) == 4 ? "f32" : "f64";
-    ra.nl_div = tune_get(c, "r2c_nl_div:" + tprec + ":L" + std::to_string(Nx));
+    ra.nl_div = tune_len(c, "r2c_nl_div", sizeof(T), Nx);
     {
         Launch L_(c, "fft_x_r2c");
         if constexpr (std::is_same<T, float>::value) {
@@ -588,7 +594,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     ly.out_zstride = 0;
     ly.scale = 1.0;
     ly.flip_mask = 0;
-    ly.nl_div = tune_get(c, std::string("lines_nl_div:") + (sizeof(T) == 4 ? "f32" : "f64") + ":L" + std::to_string(Ny));
+    ly.nl_div = tune_len(c, "lines_nl_div", sizeof(T), Ny);
     ly.flat_lines = 1;  // tiles over the (z, kx) line sequence: no part-empty tile per plane
     {
         Launch L_(c, "fft_y_fwd");
@@ -612,7 +618,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     za.img_phase_mul = nz - 1;
     za.ng = gs->nspec;
     za.fault = c->d_fault;
-    za.engine = tune_get(c, "zconv_engine:" + std::string(sizeof(T) == 4 ? "f32" : "f64") + ":L" + std::to_string(Nz));
+    za.engine = tune_len(c, "zconv_engine", sizeof(T), Nz);
     if (c->test_wait_timeout) {  // test only: waits that must run out quickly
         za.poll_limit = 64;
         za.skip_copies = 1;
@@ -658,7 +664,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     cr.zin_nz = nz;
     cr.zin_ny = ny;
     cr.ncomp = j.B4 ? 3 : nout;
-    cr.nl_div = tune_get(c, "c2r_nl_div:" + tprec + ":L" + std::to_string(Nx));
+    cr.nl_div = tune_len(c, "c2r_nl_div", sizeof(T), Nx);
     {
         Launch L_(c, "fft_x_c2r");
         TRY(kerr(c, launch_c2r_rows<T>(X4, cr, twx, c->stream), "x c2r"));
@@ -694,7 +700,7 @@ int slab_forward(osc_ctx *c, int nx, int ny, int nzl, const float4 *quad, cplx<f
     ra.in_rstride = nx;
     ra.out_rstride = nxh;
     ra.qny = ny;
-    ra.nl_div = tune_get(c, "r2c_nl_div:f32:L" + std::to_string(Nx));
+    ra.nl_div = tune_len(c, "r2c_nl_div", 4, Nx);
     {
         Launch L_(c, "fft_x_r2c");
         TRY(kerr(c, launch_r2c_rows<float, float4>(quad, X1, ra, twx, c->stream), "x r2c"));
@@ -716,7 +722,7 @@ int slab_forward(osc_ctx *c, int nx, int ny, int nzl, const float4 *quad, cplx<f
     ly.out_zstride = 0;
     ly.scale = 1.0;
     ly.flip_mask = 0;
-    ly.nl_div = tune_get(c, "lines_nl_div:f32:L" + std::to_string(Ny));
+    ly.nl_div = tune_len(c, "lines_nl_div", 4, Ny);
     ly.flat_lines = 1;
     Launch L_(c, "fft_y_fwd");
     return kerr(c, launch_lines<float>(X1, X2, ly, nzl, 1, false, twy, c->stream), "y forward");
@@ -790,7 +796,7 @@ int slab_inverse(osc_ctx *c, int nx, int ny, int nzl, const cplx<float> *X3, flo
     li.out_pstride = li.out_zstride = (int64_t)nxh * ny * nzl;
     li.scale = 1.0;
     li.flip_mask = 0;
-    li.nl_div = tune_get(c, "lines_nl_div:f32:L" + std::to_string(Ny));
+    li.nl_div = tune_len(c, "lines_nl_div", 4, Ny);
     {
         Launch L_(c, "fft_y_inv");
         TRY(kerr(c, launch_lines<float>(X3, X4, li, 1, 3, false, twy, c->stream), "y inverse"));
@@ -809,7 +815,7 @@ int slab_inverse(osc_ctx *c, int nx, int ny, int nzl, const cplx<float> *X3, flo
     cr.e8 = e8;
     for (int q = 0; q < 3; ++q) cr.e8_comp[q] = q;
     cr.e8_node = 0;
-    cr.nl_div = tune_get(c, "c2r_nl_div:f32:L" + std::to_string(Nx));
+    cr.nl_div = tune_len(c, "c2r_nl_div", 4, Nx);
     Launch L_(c, "fft_x_c2r");
     return kerr(c, launch_c2r_rows<float>(X4, cr, twx, c->stream), "x c2r");
 }

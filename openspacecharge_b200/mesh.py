@@ -11,6 +11,7 @@ Device-resident variants (``*_dev``) take torch CUDA tensors and do no host copi
 from __future__ import annotations
 
 import ctypes
+import struct
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -26,6 +27,10 @@ __all__ = [
     "get_mesh_quantities", "depose_rho_scalar", "space_charge_step", "space_charge_step_dev",
     "sort_particles_dev", "cell_keys",
 ]
+
+
+# osc_mesh3d (native.OscMesh3D): nlo, nhi, npad, padding, then min, max, delta, gamma, charge
+_MESH_C = struct.Struct("=9i4x11d")
 
 
 @dataclass
@@ -50,22 +55,14 @@ class Mesh3D:
         return tuple(int(self.nhi[d]) - int(self.nlo[d]) + 1 for d in range(3))
 
     def to_c(self) -> OscMesh3D:
-        m = OscMesh3D()
-        m.nlo[:] = [int(v) for v in self.nlo]
-        m.nhi[:] = [int(v) for v in self.nhi]
-        m.npad[:] = [int(v) for v in self.npad]
-        m.min[:] = [float(v) for v in self.min]
-        m.max[:] = [float(v) for v in self.max]
-        m.delta[:] = [float(v) for v in self.delta]
-        m.gamma = float(self.gamma)
-        m.charge = float(self.charge)
-        return m
+        return OscMesh3D.from_buffer_copy(_MESH_C.pack(
+            *map(int, self.nlo), *map(int, self.nhi), *map(int, self.npad), *map(float, self.min),
+            *map(float, self.max), *map(float, self.delta), float(self.gamma), float(self.charge)))
 
     def from_c(self, m: OscMesh3D) -> None:
-        self.min = np.array(m.min[:])
-        self.max = np.array(m.max[:])
-        self.delta = np.array(m.delta[:])
-        self.charge = float(m.charge)
+        v = np.frombuffer(m, dtype=np.float64, count=11, offset=40).copy()
+        self.min, self.max, self.delta = v[0:3], v[3:6], v[6:9]
+        self.charge = float(v[10])
 
     def allocate(self) -> None:
         """(Re)allocate the grids when their bounds changed (code/open_spacecharge_mod.f90:193-219)."""
@@ -291,13 +288,13 @@ def space_charge_step(ctx, mesh3d: Mesh3D, x, y, z, qa=None, total_charge=None, 
     return E, B
 
 
-def _tp(t) -> ctypes.c_void_p | None:
+def _tp(t) -> int | None:
     """Device pointer of a torch CUDA tensor (contiguous float64 required)."""
     if t is None:
         return None
     if not t.is_cuda or not t.is_contiguous():
         raise ValueError("device entry points need contiguous CUDA tensors")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def space_charge_step_dev(ctx, mesh3d: Mesh3D, x, y, z, E, qa=None, total_charge=None, resize_mesh=False,

@@ -164,6 +164,8 @@ def header_symbols(path: str = HEADER) -> list[str]:
 def lib() -> ctypes.CDLL:
     """Load the native library (raises if it is missing; there is no fallback)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
