@@ -219,6 +219,8 @@ template <int kRun, bool HQ>
 __global__ void __launch_bounds__(256, kRun == 4 ? 3 : 2) k_deposit_quad_runs(DepositArgs a, float4 *__restrict__ quad, bool vec,
                                                            unsigned long long *__restrict__ counters) {
     const int64_t plane = (int64_t)a.nx * a.ny;
+    pdl_wait(quad);
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 * kRun < a.np; w += nwarps) {
@@ -290,11 +292,11 @@ int launch_deposit_quad_runs(const DepositArgs &a, float *quad, unsigned long lo
     const unsigned nb = nblocks(chunks * 32, 256, 148 * (int64_t)(a.ctas > 0 ? a.ctas : 16));
     float4 *q4 = reinterpret_cast<float4 *>(quad);
     if (run == 8) {
-        if (a.q) k_deposit_quad_runs<8, true><<<nb, 256, 0, st>>>(a, q4, vec, counters);
-        else k_deposit_quad_runs<8, false><<<nb, 256, 0, st>>>(a, q4, vec, counters);
+        if (a.q) launch_pdl(k_deposit_quad_runs<8, true>, dim3(nb), dim3(256), 0, st, a, q4, vec, counters);
+        else launch_pdl(k_deposit_quad_runs<8, false>, dim3(nb), dim3(256), 0, st, a, q4, vec, counters);
     } else {
-        if (a.q) k_deposit_quad_runs<4, true><<<nb, 256, 0, st>>>(a, q4, vec, counters);
-        else k_deposit_quad_runs<4, false><<<nb, 256, 0, st>>>(a, q4, vec, counters);
+        if (a.q) launch_pdl(k_deposit_quad_runs<4, true>, dim3(nb), dim3(256), 0, st, a, q4, vec, counters);
+        else launch_pdl(k_deposit_quad_runs<4, false>, dim3(nb), dim3(256), 0, st, a, q4, vec, counters);
     }
     return ok();
 }

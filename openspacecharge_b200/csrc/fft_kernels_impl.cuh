@@ -50,9 +50,12 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_lines(const cplx<T> *in, cpl
     constexpr int lstr = NL + 1;
     const int nthreads = blockDim.x, tid = threadIdx.x;
     const int col0 = blockIdx.x * NL;
-    const V *src = in + (int64_t)blockIdx.z * a.in_zstride + (int64_t)blockIdx.y * a.in_pstride;
+    const V *src;
     V *dst = out + (int64_t)blockIdx.z * a.out_zstride + (int64_t)blockIdx.y * a.out_pstride;
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
+    src = in + (int64_t)blockIdx.z * a.in_zstride + (int64_t)blockIdx.y * a.in_pstride;
     if (!ROW) {
         // columns: the first stage reads global memory, the last stage writes it
         __syncthreads();
@@ -185,6 +188,8 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
         __syncthreads();
     }
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     auto elem = [&](int rr, int e) -> T {
         const int64_t row = row0 + rr;
         if (row >= a.nrows || e >= a.nin) return (T)0;
@@ -301,6 +306,8 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
     for (int t = tid; t < 2 * NL; t += nthreads) row_bases(a, row0 + t, rin[t], rout[t]);
     const int64_t ies = a.zin ? a.zin_nz : 1;
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     __syncthreads();
     for (int c = 0; c < a.ncomp; ++c) {
         const V *src = in + (int64_t)c * a.in_cstride;
@@ -427,6 +434,8 @@ __global__ void __launch_bounds__(FftRuntime::kMaxThreads) k_zconv(const cplx<T>
     out += blockIdx.y * a.out_bstride + (int64_t)colc * a.out_colstride;
     const int64_t goff = blockIdx.y * a.g_bstride;
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     __syncthreads();
     auto ld_in = [&](int e, int) -> V { return live && e < a.nz ? in[(int64_t)e * a.in_estride] : mk<T>(0, 0); };
     auto st_rhat = [&](int e, int l, const V &v) { rhat[e * lstr + l] = v; };
@@ -495,6 +504,8 @@ __global__ void __launch_bounds__(E::kLen * 3 * NLC / E::kEPT, sizeof(T) == 4 ? 
     for (int t = tid; t < 2 * NLC; t += nthreads) row_bases(a, row0 + t, rin[t], rout[t]);
     const int64_t ies = a.zin ? a.zin_nz : 1;
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     __syncthreads();
     // line = two real rows A + iB; each stored value k <= L/2 is read once and also gives
     // the line's value at L-k (from the conjugates)
@@ -587,6 +598,8 @@ __global__ void __launch_bounds__(FftRuntime::kMaxThreads) k_c2r_e8_rt(const cpl
     for (int t = tid; t < 2 * NLC; t += blockDim.x) row_bases(a, row0 + t, rin[t], rout[t]);
     const int64_t ies = a.zin ? a.zin_nz : 1;
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     __syncthreads();
     auto put = [&](int ln, int k) {  // ln = c * NLC + line
         const int c = ln / NLC, line = ln - c * NLC;
@@ -660,6 +673,8 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
         podd[t] = odd;
     }
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     __syncthreads();
     if constexpr (E::kLen > 0) {
         // static engine (L = 2n known, L*NL/E::kEPT threads): each thread first loads its
@@ -756,6 +771,8 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_green_zlines(const double *_
         bim[t] = (a.imag >> b) & 1u;
     }
     load_twiddles(tw, twg, L);
+    pdl_wait(in);
+    pdl_trigger();
     __syncthreads();
 #pragma unroll 4
     for (int idx = tid; idx < 2 * NL * L; idx += nthreads) {
@@ -789,24 +806,26 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_green_zlines(const double *_
 // Launchers.  Shared memory above 48 KB needs the opt-in attribute, set per kernel.
 // The attribute is set once per kernel, device and size (a lookup instead of a driver call
 // on every launch of the many small launches of a batch).
-template <typename K> inline int set_smem(K kern, size_t bytes) {
+// prefer_smem: the SM's storage is split in favour of shared memory even where one CTA needs little
+// (the runtime engine's kernels, whose CTAs per SM are bounded by their line buffers).  A kernel started
+// by launch_pdl otherwise comes up with the split of the kernel that is still running.
+template <typename K> inline int set_smem(K kern, size_t bytes, bool prefer_smem = false) {
     if (bytes > 227 * 1024) return OSC_E_INVALID;
-    if (bytes <= 46 * 1024) return OSC_OK;  // with the kernel's static arrays within the 48 KB that need no opt-in
+    // with the kernel's static arrays within the 48 KB that need no opt-in
+    if (bytes <= 46 * 1024 && !prefer_smem) return OSC_OK;
     static std::mutex mu;
     static std::map<std::pair<const void *, int>, size_t> done;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return OSC_E_CUDA;
     const auto key = std::make_pair(reinterpret_cast<const void *>(kern), dev);
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = done.find(key);
-        if (it != done.end() && it->second >= bytes) return OSC_OK;
-    }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return OSC_E_CUDA;
     std::lock_guard<std::mutex> lk(mu);
-    size_t &v = done[key];
-    if (bytes > v) v = bytes;
+    auto it = done.find(key);
+    if (it != done.end() && it->second >= bytes) return OSC_OK;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        (prefer_smem && cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                             cudaSharedmemCarveoutMaxShared) != cudaSuccess))
+        return OSC_E_CUDA;
+    done[key] = bytes;
     return OSC_OK;
 }
 inline int launch_ok() { return cudaGetLastError() == cudaSuccess ? OSC_OK : OSC_E_CUDA; }
@@ -861,7 +880,7 @@ inline int launch_lines_k(const cplx<T> *in, cplx<T> *out, const LineArgs &a, in
     const int nt = eng_threads<E>(a.p, NL);
     const size_t sm = eng_smem<E, T>(L, NL);
     auto kern = k_lines<T, NL, ROW, E, MODE>;
-    int rc = set_smem(kern, sm);
+    int rc = set_smem(kern, sm, E::kLen == 0);
     if (rc) return rc;
     // the flat tiling needs a column layout, at most one plane wrap per tile and int line indices
     const bool flat = !ROW && a.flat_lines > 0 && a.ncols >= NL && (int64_t)a.ncols * nplanes < (1ll << 30);
@@ -869,7 +888,7 @@ inline int launch_lines_k(const cplx<T> *in, cplx<T> *out, const LineArgs &a, in
     af.flat_lines = flat ? a.ncols * nplanes : 0;
     dim3 grid(flat ? (unsigned)ceil_div(af.flat_lines, NL) : (unsigned)ceil_div(a.ncols, NL),
               flat ? 1u : (unsigned)nplanes, (unsigned)ncomp);
-    kern<<<grid, nt, sm, st>>>(in, out, af, tw);
+    launch_pdl(kern, dim3(grid), dim3(nt), sm, st, in, out, af, tw);
     return launch_ok();
 }
 
@@ -917,12 +936,12 @@ int launch_r2c_rows(const TIn *in, cplx<T> *out, const R2CArgs &a, const TwPair<
                 auto kern = k_r2c_rows<T, TIn, NL, E, true>;
                 int rc = set_smem(kern, sm);
                 if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, out, a, twe);
+                launch_pdl(kern, dim3(nblk), dim3(nt), sm, st, in, out, a, twe);
             } else {
                 auto kern = k_r2c_rows<T, TIn, NL, E, false>;
-                int rc = set_smem(kern, sm);
+                int rc = set_smem(kern, sm, E::kLen == 0);
                 if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, out, a, twe);
+                launch_pdl(kern, dim3(nblk), dim3(nt), sm, st, in, out, a, twe);
             }
             return launch_ok();
         }, a.nl_div);
@@ -948,7 +967,7 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
                         auto kern = k_c2r_e8<T, NLC, E>;
                         int r = set_smem(kern, sm);
                         if (r) return r;
-                        kern<<<(unsigned)ceil_div(a.nrows, 2 * NLC), nt, sm, st>>>(in, a, tw.st);
+                        launch_pdl(kern, dim3((unsigned)ceil_div(a.nrows, 2 * NLC)), dim3(nt), sm, st, in, a, tw.st);
                         return launch_ok();
                     };
                     constexpr int NLC = c2r_e8_nlc<T, E>();
@@ -962,9 +981,9 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
                         constexpr int NLC = decltype(nlcc)::value;
                         const size_t sm = eng_smem<E, T>(L, 3 * NLC);
                         auto kern = k_c2r_e8_rt<T, NLC>;
-                        int r = set_smem(kern, sm);
+                        int r = set_smem(kern, sm, true);
                         if (r) return r;
-                        kern<<<(unsigned)ceil_div(a.nrows, 2 * NLC), mix_threads(a.p, 3 * NLC), sm, st>>>(in, a, tw.st);
+                        launch_pdl(kern, dim3((unsigned)ceil_div(a.nrows, 2 * NLC)), dim3(mix_threads(a.p, 3 * NLC)), sm, st, in, a, tw.st);
                         return launch_ok();
                     };
                     if (eng_smem<E, T>(L, 12) <= 75 * 1024) return go(std::integral_constant<int, 4>{});
@@ -988,12 +1007,12 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
                 auto kern = k_c2r_rows<T, NL, E, true>;
                 int rc = set_smem(kern, sm);
                 if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, a, twe);
+                launch_pdl(kern, dim3(nblk), dim3(nt), sm, st, in, a, twe);
             } else {
                 auto kern = k_c2r_rows<T, NL, E, false>;
-                int rc = set_smem(kern, sm);
+                int rc = set_smem(kern, sm, E::kLen == 0);
                 if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, a, twe);
+                launch_pdl(kern, dim3(nblk), dim3(nt), sm, st, in, a, twe);
             }
             return launch_ok();
         }, 0, a.e8 ? sizeof(T) * 3 * 2 * (size_t)a.nout : 0);
@@ -1010,7 +1029,7 @@ inline int launch_zconv_warp_k(const cplx<T> *in, cplx<T> *out, const ZConvArgs 
     // summed inputs: the members are the inputs of one output, read by every CTA
     const unsigned gy = MODE == ZW_SUM ? 1u : (unsigned)(a.nbatch > 0 ? a.nbatch : 1);
     const dim3 grid((unsigned)ceil_div(a.ncols, W), gy);
-    kern<<<grid, W * 32, sm, st>>>(in, out, a, tw.wt, tw.rt);
+    launch_pdl(kern, dim3(grid), dim3(W * 32), sm, st, in, out, a, tw.wt, tw.rt);
     return launch_ok();
 }
 template <typename T, int MODE, int L, int... Rs>
@@ -1069,7 +1088,7 @@ inline int launch_zconv_img(WarpFft<L, Rs...>, const cplx<T> *in, cplx<T> *out, 
     if (rc) return rc;
     const int nkp = (a.nxh + 1) / 2;
     const dim3 grid((unsigned)(nkp * (a.ny + 1)), (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
-    kern<<<grid, ZI_WARPS * 32, sm, st>>>(in, out, a, tw.wt);
+    launch_pdl(kern, dim3(grid), dim3(ZI_WARPS * 32), sm, st, in, out, a, tw.wt);
     return launch_ok();
 }
 
@@ -1080,7 +1099,7 @@ inline int launch_zconv_w512(const float2 *in, float2 *out, const ZConvArgs &a, 
     int rc = set_smem(kern, sm);
     if (rc) return rc;
     const dim3 grid((unsigned)ceil_div(a.ncols, W), (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
-    kern<<<grid, W * 32, sm, st>>>(in, out, a, rt);
+    launch_pdl(kern, dim3(grid), dim3(W * 32), sm, st, in, out, a, rt);
     return launch_ok();
 }
 
@@ -1142,10 +1161,10 @@ int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPa
         constexpr int NL = decltype(nlc)::value;
         const size_t sm = sizeof(cplx<T>) * ((size_t)L + (size_t)(a.p.nst > 2 ? 3 : 2) * L * (NL + 1));
         auto kern = k_zconv<T, NL>;
-        int rc = set_smem(kern, sm);
+        int rc = set_smem(kern, sm, true);
         if (rc) return rc;
         const dim3 nblk((unsigned)ceil_div(a.ncols, NL), (unsigned)(a.nbatch > 0 ? a.nbatch : 1));
-        kern<<<nblk, mix_threads(a.p, NL), sm, st>>>(in, out, a, tw.st, tw.rt);
+        launch_pdl(kern, dim3(nblk), dim3(mix_threads(a.p, NL)), sm, st, in, out, a, tw.st, tw.rt);
         return launch_ok();
     };
     const int nls[2] = {8, 1};
@@ -1186,9 +1205,9 @@ int launch_sym_lines(const TI *in, TO *out, const SymArgs &a, const TwPair<cplx<
             const size_t sm = eng_smem<E, TC>(L, NL);
             const unsigned nblk = (unsigned)ceil_div(((a.npq + 1) & ~(int64_t)1) * a.nb, 2 * NL);
             auto go = [&](auto kern) -> int {
-                int rc = set_smem(kern, sm);
+                int rc = set_smem(kern, sm, E::kLen == 0);
                 if (rc) return rc;
-                kern<<<nblk, nt, sm, st>>>(in, out, a, twe);
+                launch_pdl(kern, dim3(nblk), dim3(nt), sm, st, in, out, a, twe);
                 return launch_ok();
             };
             if (row_load) return k_fast_store ? go(k_sym_lines<TC, TI, TO, NL, E, true, true>)
@@ -1209,10 +1228,10 @@ int launch_green_zlines(const double *in, cplx<TO> *out, const ZLineArgs &a, con
             constexpr int NL = decltype(nlc)::value;
             auto kern = k_green_zlines<TO, NL, E>;
             const size_t sm = eng_smem<E, double>(L, NL);
-            int rc = set_smem(kern, sm);
+            int rc = set_smem(kern, sm, E::kLen == 0);
             if (rc) return rc;
             const unsigned nblk = (unsigned)ceil_div(((a.nq + 1) & ~(int64_t)1) * a.nb, 2 * NL);
-            kern<<<nblk, eng_threads<E>(a.p, NL), sm, st>>>(in, out, a, tw.st, tw.rt);
+            launch_pdl(kern, dim3(nblk), dim3(eng_threads<E>(a.p, NL)), sm, st, in, out, a, tw.st, tw.rt);
             return launch_ok();
         });
     });

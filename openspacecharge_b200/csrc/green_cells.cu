@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(256, 3) k_green_cells(TH *__restrict__ h, Cell
                                                      const CellGeom *__restrict__ gb) {
     __shared__ double sF[(CT_X + 1) * (CT_Y + 1) * (CT_Z + 1)];
     __shared__ alignas(16) double sc[BATCH ? 4 * kSerP : 2];
+    pdl_wait(h);
+    pdl_trigger();
     const CellGeom &g = BATCH ? gb[blockIdx.y] : g0;
     const int ntx = (a.nx + CT_X - 1) / CT_X, nty = (a.ny + CT_Y - 1) / CT_Y, ntz = (a.nz + CT_Z - 1) / CT_Z;
     // components of a tile side by side: the near tiles come early for all of them
@@ -223,14 +225,14 @@ static dim3 cells_grid(const CellArgs &a) {
 }
 template <typename TH> int launch_green_cells(TH *h, const CellArgs &a, const CellGeom &g, cudaStream_t st) {
     if (a.nmem != 1 || a.ncomp < 1 || a.ncomp > 4) return OSC_E_INVALID;
-    k_green_cells<TH, false><<<cells_grid(a), 256, 0, st>>>(h, a, g, nullptr);
+    launch_pdl(k_green_cells<TH, false>, cells_grid(a), dim3(256), 0, st, h, a, g, nullptr);
     return ok();
 }
 template int launch_green_cells<float>(float *, const CellArgs &, const CellGeom &, cudaStream_t);
 template int launch_green_cells<double>(double *, const CellArgs &, const CellGeom &, cudaStream_t);
 int launch_green_cells_batch(float *h, const CellArgs &a, const CellGeom *g, cudaStream_t st) {
     if (a.nmem < 1 || a.ncomp < 1 || a.ncomp > 4) return OSC_E_INVALID;
-    k_green_cells<float, true><<<cells_grid(a), 256, 0, st>>>(h, a, CellGeom{}, g);
+    launch_pdl(k_green_cells<float, true>, cells_grid(a), dim3(256), 0, st, h, a, CellGeom{}, g);
     return ok();
 }
 

@@ -263,6 +263,8 @@ int launch_fd_efield(const double *phi, double *E, int nx, int ny, int nz, doubl
 __global__ void k_fd_efield_pairs(const double *__restrict__ phi, float4 *__restrict__ e8, int nx, int ny, int nz,
                                   double dx, double dy, double dz, double gam0) {
     const int64_t N = (int64_t)nx * ny * nz;
+    pdl_wait(phi);
+    pdl_trigger();
     GRID_STRIDE(m, N) {
         const int i = (int)(m % nx);
         const int64_t r = m / nx;
@@ -289,8 +291,8 @@ __global__ void k_fd_efield_pairs(const double *__restrict__ phi, float4 *__rest
 }
 int launch_fd_efield_pairs(const double *phi, float *e8, int nx, int ny, int nz, double dx, double dy, double dz,
                            double gam0, cudaStream_t st) {
-    k_fd_efield_pairs<<<nblocks((int64_t)nx * ny * nz, 256), 256, 0, st>>>(phi, reinterpret_cast<float4 *>(e8), nx, ny,
-                                                                           nz, dx, dy, dz, gam0);
+    launch_pdl(k_fd_efield_pairs, dim3(nblocks((int64_t)nx * ny * nz, 256)), dim3(256), 0, st, phi,
+               reinterpret_cast<float4 *>(e8), nx, ny, nz, dx, dy, dz, gam0);
     return ok();
 }
 

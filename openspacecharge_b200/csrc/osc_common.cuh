@@ -66,6 +66,42 @@ template <typename V> __host__ __device__ __forceinline__ V cmul_si(V a, int s) 
     return r;
 }
 
+// Programmatic dependent launch.  A kernel started by launch_pdl may begin while the kernel queued
+// before it on the stream is still finishing: its blocks come up, load their twiddles and work
+// out their indexes, and pdl_wait holds them until that kernel is complete and its
+// writes are visible.  Every kernel started this way calls pdl_wait before it touches anything that
+// an earlier kernel writes or reads (the pointers that go through it cannot be read
+// ahead of it), and only then pdl_trigger, so that when the next kernel's blocks come up, all
+// kernels before this one are complete.
+template <typename Ptr> __device__ __forceinline__ void pdl_wait(Ptr &p) {
+    asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+}
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Kernels with dynamic shared memory start this way up to 2400 CTAs, the others (particle and
+// clearing kernels, Green cells) up to 600.  A kernel that starts early comes up with the
+// shared-memory split of the one before it and keeps it for its whole run, so a gather loses its
+// L1 and a transform its resident CTAs: with every launch early, the gather of 1e7 particles on
+// 128 x 128 x 256 takes 700 us against 220 and the z pass 180 against 140.  What it gains is a few
+// us per launch however large the grid is.  Steps in us with limits 0, 300, 600, 1200, 2400, 5000
+// (600 at most for the kernels without dynamic shared memory; "all" without a limit): 32 x 32 x 48
+// with refit 91 79 75 75 74 74 (all: 69), 64^3 117 114 114 114 110 110 (all: 106), 64^3 cathode with refit 350 342 339 333 329 329 (all: 323), 128^3 FP64 589 589 588 585 579
+// 580 (all: 688), 128 x 128 x 256 691 691 692 690 685 685 (all: 1227).
+template <typename... KP, typename... A>
+inline void launch_pdl(void (*kern)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = (uint64_t)grid.x * grid.y * grid.z <= (smem > 0 ? 2400u : 600u) ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, KP(args)...);  // the caller checks cudaGetLastError
+}
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 }  // namespace osc

@@ -152,11 +152,14 @@ __device__ __forceinline__ int quad_one(const DepositArgs &a, float4 *__restrict
 // Clears a quad grid and the counters in one launch.
 __global__ void __launch_bounds__(256) k_clear_quad(float4 *__restrict__ quad, int64_t n, unsigned long long *counters) {
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait(quad);
+    pdl_trigger();
     GRID_STRIDE(i, n) quad[i] = z;
     if (blockIdx.x == 0 && threadIdx.x < 8) counters[threadIdx.x] = 0;
 }
 int launch_clear_quad(float *quad, int64_t nodes, unsigned long long *counters, cudaStream_t st) {
-    k_clear_quad<<<nblocks(nodes, 256, 148 * 8), 256, 0, st>>>(reinterpret_cast<float4 *>(quad), nodes, counters);
+    launch_pdl(k_clear_quad, dim3(nblocks(nodes, 256, 148 * 8)), dim3(256), 0, st, reinterpret_cast<float4 *>(quad), nodes,
+               counters);
     return ok();
 }
 
@@ -173,6 +176,9 @@ __global__ void __launch_bounds__(256) k_deposit_quad(DepositArgs a, float4 *__r
         zn = __ldg(a.z + m);
         if (a.q) qn = __ldg(a.q + m);
     }
+    // the particles are the caller's, complete before the kernel that clears the grid began
+    pdl_wait(quad);
+    pdl_trigger();
     for (; m < a.np; m += stride) {
         const double xm = xn, ym = yn, zm = zn, c = qn;
         const int64_t mn = m + stride;
@@ -192,7 +198,7 @@ int launch_deposit_quad(const DepositArgs &a, float *quad, unsigned long long *c
     if (a.np <= 0) return OSC_OK;
     // default: one particle per thread; the autotuner may cap the grid at a.ctas CTAs per SM
     const int64_t cap = a.ctas > 0 ? 148 * (int64_t)a.ctas : (1 << 20);
-    k_deposit_quad<<<nblocks(a.np, 256, cap), 256, 0, st>>>(a, reinterpret_cast<float4 *>(quad), counters);
+    launch_pdl(k_deposit_quad, dim3(nblocks(a.np, 256, cap)), dim3(256), 0, st, a, reinterpret_cast<float4 *>(quad), counters);
     return ok();
 }
 
@@ -290,6 +296,8 @@ __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T>
     TO *ws = stage + (threadIdx.x - lane) * 3;
     const int64_t plane = (int64_t)a.nx * a.ny;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    pdl_wait(g);
+    pdl_trigger();
     for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m - lane < a.np; m += stride) {
         bool fl = false;
         if (m < a.np) {
@@ -326,8 +334,8 @@ template <typename T>
 int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp, cudaStream_t st,
                        double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
-    k_interp_vec4<T, double><<<nblocks(a.np, 256, 148 * 64), 256, 0, st>>>(a, reinterpret_cast<const vec4<T> *>(E4),
-                                                                            E, B, bcoef, nclamp);
+    launch_pdl(k_interp_vec4<T, double>, dim3(nblocks(a.np, 256, 148 * 64)), dim3(256), 0, st, a,
+               reinterpret_cast<const vec4<T> *>(E4), E, B, bcoef, nclamp);
     return ok();
 }
 template int launch_interp_vec4<double>(const InterpArgs &, const void *, double *, unsigned long long *, cudaStream_t,
@@ -424,6 +432,8 @@ __global__ void __launch_bounds__(256) k_interp_pairs(InterpArgs a, const float4
         yn = __ldg(a.y + m);
         zn = __ldg(a.z + m);
     }
+    pdl_wait(g8);
+    pdl_trigger();
     // the loop runs while the warp's first particle exists, so all lanes take the same trips
     for (; m - lane < a.np; m += stride) {
         const double xm = xn, ym = yn, zm = zn;
@@ -457,6 +467,8 @@ __global__ void __launch_bounds__(256, RUN == 4 ? 3 : 2) k_interp_pairs_runs(Int
                                                            double *__restrict__ E, double *__restrict__ B, double bcoef,
                                                            unsigned long long *__restrict__ nclamp) {
     static_assert(RUN % 4 == 0, "runs of whole 256-bit vectors");
+    pdl_wait(g8);
+    pdl_trigger();
     const int64_t plane = (int64_t)a.nx * a.ny;
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -542,9 +554,9 @@ int launch_interp_pairs_runs(const InterpArgs &a, const float4 *E8, double *E, u
     const int64_t chunks = (a.np + 32 * run - 1) / (32 * run);
     const unsigned nb = nblocks(chunks * 32, 256, 148 * (int64_t)(a.ctas > 0 ? a.ctas : 16));
     if (run == 8)
-        k_interp_pairs_runs<8><<<nb, 256, 0, st>>>(a, E8, vec, E, B, bcoef, nclamp);
+        launch_pdl(k_interp_pairs_runs<8>, dim3(nb), dim3(256), 0, st, a, E8, vec, E, B, bcoef, nclamp);
     else
-        k_interp_pairs_runs<4><<<nb, 256, 0, st>>>(a, E8, vec, E, B, bcoef, nclamp);
+        launch_pdl(k_interp_pairs_runs<4>, dim3(nb), dim3(256), 0, st, a, E8, vec, E, B, bcoef, nclamp);
     return ok();
 }
 
@@ -553,7 +565,7 @@ int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsign
     if (a.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(E8) % 32) return OSC_E_INVALID;
     const int64_t cap = 148 * (int64_t)(a.ctas > 0 ? a.ctas : 64);
-    k_interp_pairs<<<nblocks(a.np, 256, cap), 256, 0, st>>>(a, E8, E, B, bcoef, nclamp);
+    launch_pdl(k_interp_pairs, dim3(nblocks(a.np, 256, cap)), dim3(256), 0, st, a, E8, E, B, bcoef, nclamp);
     return ok();
 }
 
@@ -1040,6 +1052,8 @@ __global__ void __launch_bounds__(256) k_vjp_pairs(InterpArgs ia, DepositArgs da
     const int lane = threadIdx.x & 31;
     double *ws = stage + (threadIdx.x - lane) * 3;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    pdl_wait(g8);
+    pdl_trigger();
     for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m - lane < ia.np; m += stride) {
         // coordinates first, so that their loads are in flight with the dL/dE rows
         double xm = 0, ym = 0, zm = 0;
@@ -1115,8 +1129,8 @@ int launch_vjp_pairs(const InterpArgs &ia, const DepositArgs &da, const float *e
                      double *gy, double *gz, double *gq, cudaStream_t st) {
     if (ia.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(e8) % 32) return OSC_E_INVALID;
-    k_vjp_pairs<<<nblocks(ia.np, 256, 148 * 64), 256, 0, st>>>(ia, da, reinterpret_cast<const float4 *>(e8), gE, gx,
-                                                               gy, gz, gq);
+    launch_pdl(k_vjp_pairs, dim3(nblocks(ia.np, 256, 148 * 64)), dim3(256), 0, st, ia, da,
+               reinterpret_cast<const float4 *>(e8), gE, gx, gy, gz, gq);
     return ok();
 }
 

@@ -71,8 +71,11 @@ __global__ void __launch_bounds__(ZI_WARPS * 32, zi_minb<T, IMG>())
     in += blockIdx.y * a.in_bstride;
     out += blockIdx.y * a.out_bstride;
     V *wb = wbufs + warp * WB;
+    load_twiddles(tw, twg, L);
+    if (threadIdx.x == 0) mbar_init(&gbar, 1);
+    pdl_wait(in);
+    pdl_trigger();
     if (threadIdx.x == 0) {
-        mbar_init(&gbar, 1);
         const int nk = min(2, a.nxh - kx0);
         mbar_arrive_expect_tx(&gbar, (unsigned)(nk * nout * (zp * (int)sizeof(T) + (IMG ? zpi * (int)sizeof(V) : 0))));
         for (int kk = 0; kk < nk; ++kk) {
@@ -89,12 +92,11 @@ __global__ void __launch_bounds__(ZI_WARPS * 32, zi_minb<T, IMG>())
             }
         }
     }
-    load_twiddles(tw, twg, L);
     for (int idx = threadIdx.x; idx < W * a.nz; idx += W * 32) {
         const int e = idx / W, c = idx - e * W;
         const int col = col_of(c);
         V v = mk<T>(0, 0);
-        if (col >= 0) v = in[(int64_t)e * a.in_estride + col];
+        if (col >= 0) v = __ldg(in + (int64_t)e * a.in_estride + col);
         wbufs[c * WB + wpad<V>(e)] = v;
     }
     __syncthreads();

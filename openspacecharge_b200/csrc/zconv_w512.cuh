@@ -136,8 +136,10 @@ __global__ void __launch_bounds__(W * 32, 6) k_zconv_w512(const float2 *__restri
     out += blockIdx.y * a.out_bstride;
     const int64_t goff = blockIdx.y * a.g_bstride;
     float2 *wb = wbufs + warp * W5_BUF;
+    if (threadIdx.x == 0) mbar_init(&gbar, 1);
+    pdl_wait(in);
+    pdl_trigger();
     if (threadIdx.x == 0) {
-        mbar_init(&gbar, 1);
         const int ncv = min(W, a.ncols - col0);
         mbar_arrive_expect_tx(&gbar, (unsigned)(ncv * nst * zp * (int)sizeof(float)));
         for (int cc = 0; cc < ncv; ++cc) {
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(W * 32, 6) k_zconv_w512(const float2 *__restri
         const int e = idx / W, cc = idx - e * W;
         const int col = col0 + cc;
         float2 v = make_float2(0.f, 0.f);
-        if (col < a.ncols) v = in[(int64_t)e * a.in_estride + col];
+        if (col < a.ncols) v = __ldg(in + (int64_t)e * a.in_estride + col);
         wbufs[cc * W5_BUF + e] = v;
     }
     __syncthreads();

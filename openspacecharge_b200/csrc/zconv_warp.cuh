@@ -187,9 +187,12 @@ __global__ void __launch_bounds__(W * 32, zw_minb<T>()) k_zconv_warp(const cplx<
     out += blockIdx.y * a.out_bstride;
     const int64_t goff = blockIdx.y * a.g_bstride;
     V *wb = wbufs + warp * WB;
+    load_twiddles(tw, twg, L);
+    if (GS && threadIdx.x == 0) mbar_init(&gbar, 1);
+    pdl_wait(in);
+    pdl_trigger();
     if (GS) {
         if (threadIdx.x == 0) {
-            mbar_init(&gbar, 1);
             const int ncv = min(W, a.ncols - col0);
             mbar_arrive_expect_tx(&gbar, (unsigned)(ncv * nst * zp * (int)sizeof(T)));
             for (int c = 0; c < ncv; ++c) {
@@ -203,14 +206,13 @@ __global__ void __launch_bounds__(W * 32, zw_minb<T>()) k_zconv_warp(const cplx<
             }
         }
     }
-    load_twiddles(tw, twg, L);
     // the non-zero half (z < nz) of this CTA's W columns of input `src`, into the warp buffers
     auto load_columns = [&](const cplx<T> *__restrict__ src) {
         for (int idx = threadIdx.x; idx < W * a.nz; idx += W * 32) {
             const int e = idx / W, c = idx - e * W;
             const int col = col0 + c;
             V v = mk<T>(0, 0);
-            if (col < a.ncols) v = src[(int64_t)e * a.in_estride + col];
+            if (col < a.ncols) v = __ldg(src + (int64_t)e * a.in_estride + col);
             wbufs[c * WB + wpad<V>(e)] = v;
         }
     };
