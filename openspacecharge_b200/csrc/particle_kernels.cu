@@ -40,21 +40,36 @@ __device__ __forceinline__ void count_one(unsigned long long *c, bool pred) {
     if (pred && (threadIdx.x & 31) == __ffs(mask) - 1) atomicAdd(c, (unsigned long long)__popc(mask));
 }
 
+// Scalar deposit (FP64 and fixed point): eight reductions per particle, two lanes to a particle, the
+// even lane its four nodes at i and the odd lane those at i + 1, so that the pair's reductions
+// of a row go to one 32-byte sector (three times in four) as one request.  The L2 takes about
+// 165e9 reduction requests a second from any of the deposits, whatever their width: it is
+// the requests that bound this kernel.  4e6 particles on 128^3: 190 us with one lane to a
+// particle, 115 with two.  Each weight is the product of the same factors in the same order as there.
 template <typename TA>
 __global__ void __launch_bounds__(256) k_deposit(DepositArgs a, TA *__restrict__ rho,
                                                  unsigned long long *__restrict__ counters) {
     const int64_t plane = (int64_t)a.nx * a.ny;
-    GRID_STRIDE(m, a.np) {
-        bool skip = false, outside = false, nonfinite = false;
-        if (a.lost && a.lost[m] != 0.0) skip = true;
-        const double xm = a.x[m], ym = a.y[m], zm = a.z[m];
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    // whole warps stay in the loop while their first particle exists
+    for (int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; m - lane < a.np; m += stride) {
+        bool skip = m >= a.np, outside = false, nonfinite = false;
+        double xm = 0, ym = 0, zm = 0;
+        if (!skip) {
+            if (a.lost && a.lost[m] != 0.0) skip = true;
+            xm = a.x[m];
+            ym = a.y[m];
+            zm = a.z[m];
+        }
         if (!skip && a.check_finite && !(isfinite(xm) && isfinite(ym) && isfinite(zm))) {
             nonfinite = true;
             skip = true;
         }
-        double fx, fy, fz, ab, de, gh;
-        int i = 0, j = 0, k = 0;
+        double ab = 0, de = 0, gh = 0, c = 0;
+        long long n0 = -1;  // the lowest corner's node, or none
         if (!skip) {
+            int i = 0, j = 0, k = 0;
             if (a.mode == 0) {
                 // the 2x2x2 stencil must lie inside the array
                 CicCell cc = {0, 0, 0, 0.0, 0.0, 0.0};
@@ -62,13 +77,13 @@ __global__ void __launch_bounds__(256) k_deposit(DepositArgs a, TA *__restrict__
                 ab = cc.ab;
                 de = cc.de;
                 gh = cc.gh;
-                fx = cc.i + a.nlo[0];
-                fy = cc.j + a.nlo[1];
-                fz = cc.k + a.nlo[2];
+                i = cc.i;
+                j = cc.j;
+                k = cc.k;
             } else {
-                fx = floor(__dmul_rn(xm - a.xmin, a.dxi) + a.nlogbl[0]);
-                fy = floor(__dmul_rn(ym - a.ymin, a.dyi) + a.nlogbl[1]);
-                fz = floor(__dmul_rn(zm - a.zmin, a.dzi) + a.nlogbl[2]);
+                const double fx = floor(__dmul_rn(xm - a.xmin, a.dxi) + a.nlogbl[0]);
+                const double fy = floor(__dmul_rn(ym - a.ymin, a.dyi) + a.nlogbl[1]);
+                const double fz = floor(__dmul_rn(zm - a.zmin, a.dzi) + a.nlogbl[2]);
                 ab = ((a.xmin - xm) + (fx - a.nlogbl[0] + 1) * a.dx) * a.dxi;
                 de = ((a.ymin - ym) + (fy - a.nlogbl[1] + 1) * a.dy) * a.dyi;
                 gh = ((a.zmin - zm) + (fz - a.nlogbl[2] + 1) * a.dz) * a.dzi;
@@ -76,27 +91,34 @@ __global__ void __launch_bounds__(256) k_deposit(DepositArgs a, TA *__restrict__
                 outside = !(fx >= a.nlo[0] && fx <= a.nx && fy >= a.nlo[1] && fy <= a.ny && fz >= a.nlo[2] &&
                             fz <= a.nz) ||
                           !(fx - a.nlo[0] + 1 < a.nx && fy - a.nlo[1] + 1 < a.ny && fz - a.nlo[2] + 1 < a.nz);
+                if (!outside) {
+                    i = (int)fx - a.nlo[0];
+                    j = (int)fy - a.nlo[1];
+                    k = (int)fz - a.nlo[2];
+                }
             }
             if (!outside) {
-                i = (int)fx - a.nlo[0];
-                j = (int)fy - a.nlo[1];
-                k = (int)fz - a.nlo[2];
+                n0 = i + (long long)a.nx * j + plane * k;
+                c = a.mode == 0 ? (a.q ? a.q[m] : a.charge1) : 1.0;
             }
         }
         count_one(&counters[0], !skip && outside);
         count_one(&counters[1], nonfinite);
-        if (skip || outside) continue;
-        const double c = a.mode == 0 ? (a.q ? a.q[m] : a.charge1) : 1.0;
-        const double omab = 1. - ab, omde = 1. - de, omgh = 1. - gh;
-        TA *r0 = rho + i + (int64_t)a.nx * j + plane * k;
-        atomic_add_t(r0, ab * de * gh * c, a.fx_scale);
-        atomic_add_t(r0 + a.nx, ab * omde * gh * c, a.fx_scale);
-        atomic_add_t(r0 + a.nx + plane, ab * omde * omgh * c, a.fx_scale);
-        atomic_add_t(r0 + plane, ab * de * omgh * c, a.fx_scale);
-        atomic_add_t(r0 + 1 + plane, omab * de * omgh * c, a.fx_scale);
-        atomic_add_t(r0 + 1 + a.nx + plane, omab * omde * omgh * c, a.fx_scale);
-        atomic_add_t(r0 + 1 + a.nx, omab * omde * gh * c, a.fx_scale);
-        atomic_add_t(r0 + 1, omab * de * gh * c, a.fx_scale);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int src = 16 * r + (lane >> 1);
+            const long long n = __shfl_sync(0xffffffffu, n0, src);
+            const double sab = __shfl_sync(0xffffffffu, ab, src), sde = __shfl_sync(0xffffffffu, de, src);
+            const double sgh = __shfl_sync(0xffffffffu, gh, src), sc = __shfl_sync(0xffffffffu, c, src);
+            if (n < 0) continue;
+            const double w = (lane & 1) ? 1. - sab : sab, omde = 1. - sde, omgh = 1. - sgh;
+            TA *r0 = rho + n + (lane & 1);
+            atomic_add_t(r0, w * sde * sgh * sc, a.fx_scale);
+            atomic_add_t(r0 + a.nx, w * omde * sgh * sc, a.fx_scale);
+            atomic_add_t(r0 + a.nx + plane, w * omde * omgh * sc, a.fx_scale);
+            atomic_add_t(r0 + plane, w * sde * omgh * sc, a.fx_scale);
+        }
     }
 }
 
