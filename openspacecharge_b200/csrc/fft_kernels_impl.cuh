@@ -156,10 +156,10 @@ __device__ __forceinline__ TIn r2c_in(const TIn *__restrict__ p, const R2CArgs &
 // fixed order (the order of k_quad_to_nodes, so rho is the same to the bit).
 __device__ __forceinline__ float r2c_in(const float4 *__restrict__ p, const R2CArgs &a, bool jn, int e) {
     const float4 *q = p + e;
-    float s = __ldg(&q->x);
-    if (e > 0) s += __ldg(&q[-1].y);
-    if (jn) s += __ldg(&q[-a.in_rstride].z);
-    if (e > 0 && jn) s += __ldg(&q[-a.in_rstride - 1].w);
+    float s = __ldca(&q->x);
+    if (e > 0) s += __ldca(&q[-1].y);
+    if (jn) s += __ldca(&q[-a.in_rstride].z);
+    if (e > 0 && jn) s += __ldca(&q[-a.in_rstride - 1].w);
     return s;
 }
 

@@ -72,7 +72,9 @@ template <typename V> __host__ __device__ __forceinline__ V cmul_si(V a, int s) 
 // writes are visible.  Every kernel started this way calls pdl_wait before it touches anything that
 // an earlier kernel writes or reads (the pointers that go through it cannot be read
 // ahead of it), and only then pdl_trigger, so that when the next kernel's blocks come up, all
-// kernels before this one are complete.
+// kernels before this one are complete.  What the kernel before may still be writing when this one
+// comes up is read with plain loads (__ldca), not through the read-only path, whose data has to be
+// constant while the kernel runs.
 template <typename Ptr> __device__ __forceinline__ void pdl_wait(Ptr &p) {
     asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
 }
@@ -87,6 +89,7 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // (600 at most for the kernels without dynamic shared memory; "all" without a limit): 32 x 32 x 48
 // with refit 91 79 75 75 74 74 (all: 69), 64^3 117 114 114 114 110 110 (all: 106), 64^3 cathode with refit 350 342 339 333 329 329 (all: 323), 128^3 FP64 589 589 588 585 579
 // 580 (all: 688), 128 x 128 x 256 691 691 692 690 685 685 (all: 1227).
+inline bool pdl_early(uint64_t ctas, size_t smem) { return ctas <= (smem > 0 ? 2400u : 600u); }
 template <typename... KP, typename... A>
 inline void launch_pdl(void (*kern)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
     cudaLaunchAttribute at{};
@@ -98,7 +101,7 @@ inline void launch_pdl(void (*kern)(KP...), dim3 grid, dim3 block, size_t smem, 
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &at;
-    cfg.numAttrs = (uint64_t)grid.x * grid.y * grid.z <= (smem > 0 ? 2400u : 600u) ? 1 : 0;
+    cfg.numAttrs = pdl_early((uint64_t)grid.x * grid.y * grid.z, smem) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kern, KP(args)...);  // the caller checks cudaGetLastError
 }
 

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(ZI_WARPS * 32, zi_minb<T, IMG>())
         const int e = idx / W, c = idx - e * W;
         const int col = col_of(c);
         V v = mk<T>(0, 0);
-        if (col >= 0) v = __ldg(in + (int64_t)e * a.in_estride + col);
+        if (col >= 0) v = __ldca(in + (int64_t)e * a.in_estride + col);
         wbufs[c * WB + wpad<V>(e)] = v;
     }
     __syncthreads();

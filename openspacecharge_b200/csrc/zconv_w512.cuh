@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(W * 32, 6) k_zconv_w512(const float2 *__restri
         const int e = idx / W, cc = idx - e * W;
         const int col = col0 + cc;
         float2 v = make_float2(0.f, 0.f);
-        if (col < a.ncols) v = __ldg(in + (int64_t)e * a.in_estride + col);
+        if (col < a.ncols) v = __ldca(in + (int64_t)e * a.in_estride + col);
         wbufs[cc * W5_BUF + e] = v;
     }
     __syncthreads();

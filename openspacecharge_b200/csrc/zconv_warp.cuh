@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(W * 32, zw_minb<T>()) k_zconv_warp(const cplx<
             const int e = idx / W, c = idx - e * W;
             const int col = col0 + c;
             V v = mk<T>(0, 0);
-            if (col < a.ncols) v = __ldg(src + (int64_t)e * a.in_estride + col);
+            if (col < a.ncols) v = __ldca(src + (int64_t)e * a.in_estride + col);
             wbufs[c * WB + wpad<V>(e)] = v;
         }
     };
