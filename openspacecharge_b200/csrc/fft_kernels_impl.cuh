@@ -1107,7 +1107,8 @@ template <typename T>
 int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPair<cplx<T>> &tw,
                  cudaStream_t st) {
     const int L = a.p.L;
-    // a column range of a z slab (col_base > 0) runs on the radix warp engine only
+    // a column range of a z slab runs on the radix warp engine only
+    const bool whole = a.col_base == 0 && (int64_t)a.ncols == (int64_t)a.nxh * a.Ny;
     if (a.col_base != 0 && (!zconv_warp_ok(L, a.nz, (int)sizeof(T)) || a.nsum > 0)) return OSC_E_UNSUPPORTED;
     if (zconv_warp_ok(L, a.nz, (int)sizeof(T))) {
         for (int i = 0; i < a.ng; ++i)
@@ -1119,7 +1120,7 @@ int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPa
         }
         if (tw.wt == tw.rt) return OSC_E_INVALID;
         if (herm) {  // image spectra stored for the image z pass: no other kernel reads them
-            if (a.col_base != 0 || !zconv_img_ok(L, a.nz, (int)sizeof(T)) || !zconv_img_can<T>(a))
+            if (!whole || !zconv_img_ok(L, a.nz, (int)sizeof(T)) || !zconv_img_can<T>(a))
                 return OSC_E_INVALID;
             return dispatch_warp_len(L, [&](auto eng) -> int {
                 using E = decltype(eng);
@@ -1133,12 +1134,16 @@ int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPa
         const bool staged = !img && zconv_can_stage<T>(a);
         if (a.nsum > 0 && (img || !staged || a.nout != 1)) return OSC_E_UNSUPPORTED;
         if constexpr (sizeof(T) == 4) {
-            if (L == 512 && staged && a.nsum == 0 && a.out_estride == 1 && a.engine == 1 && a.col_base == 0 &&
+            if (L == 512 && staged && a.nsum == 0 && a.out_estride == 1 && a.engine == 1 && whole &&
                 zconv_w512_smem<4>(a.nout, a.g[0].zpitch) <= 100 * 1024)
                 return launch_zconv_w512(in, out, a, tw.rt, st);
         }
-        // engine 2: the staged product with Green columns shared by the rows ky and Ny - ky
-        const bool pair = staged && a.engine == 2 && a.col_base == 0 && zconv_img_ok(L, a.nz, (int)sizeof(T)) &&
+        // The staged product with Green columns shared by the rows ky and Ny - ky wherever it applies,
+        // unless the caller asks for the other engine (1): it reads half the spectra, and is never the
+        // slower one.  Paired against one warp per column (us), FP32: 16^3 8.6 10.6, 64^3 18.9 24.4,
+        // 64 x 64 x 96 27.1 31.1, 128^3 76.2 81.7, 192 x 192 x 64 113 148, 128 x 128 x 256 138.5 143.9
+        // (one exchange 155); FP64: 32^3 10.6 16.9, 128^3 128 137, 96^3 72 97, 128 x 128 x 256 287 326.
+        const bool pair = staged && a.engine != 1 && whole && zconv_img_ok(L, a.nz, (int)sizeof(T)) &&
                           zconv_pair_can<T>(a);
         return dispatch_warp_len(L, [&](auto eng) -> int {
             using E = decltype(eng);
