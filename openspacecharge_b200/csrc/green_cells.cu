@@ -105,16 +105,19 @@ __device__ __forceinline__ double ser_eval(const double *c, double u, double v, 
     return s;
 }
 
-// A CTA of 256 threads owns a tile of 16 x 8 x 4 cells of one component, two cells a thread.  A tile
-// whose nearest cell is closer than the series' distance evaluates the primitives of its
-// 17 x 9 x 5 corners in shared memory (1.5 per cell) and differences them; the far tiles compute
-// all components at once from one 1/r, and their CTAs of the other components leave at
-// once.  Bound by the FP64 rate: about 150 operations per far cell for three components, against
-// 3 x 200 with two logs, an atan, a square root and two divisions each for the primitives of
-// every corner, which were also written out and read back: 104 us for 128 x 128 x 256, against 170
-// for the corners and 71 for their differences.  The tile is small so that the few near tiles,
-// whose chains of logs and atans are the longest, spread over the SMs (tiles of 32 x 8 x 4 took
-// 144 us there, and 20 against 11 us for 32 x 32 x 48).
+// A CTA of 256 threads owns a tile of 16 x 8 x 4 cells, two cells a thread.  A tile whose nearest cell
+// is closer than the series' distance evaluates the primitives of its 17 x 9 x 5 corners in
+// shared memory (1.5 per cell) and differences them; the far tiles compute all components at
+// once from one 1/r.  On grids of few tiles the components of a near tile go to as many CTAs
+// (split; a far tile's other CTAs leave at once), since the chain of one is what the launch
+// takes; on larger ones a CTA walks them and no CTA is launched to leave: 128 x 128 x 256 takes
+// 106 us with the split and 73 without, 128^3 62 and 44, 48^3 12.8 and 10.8, and 32^3 takes 11 with
+// it.  Bound by the FP64 rate: about 150 operations per far cell for three components, against 3 x
+// 200 with two logs, an atan, a square root and two divisions each for the primitives of every
+// corner, which were also written out and read back: 170 us for the corners of 128 x 128 x 256
+// and 71 for their differences.  The tile is small so that the few near tiles, whose chains of
+// logs and atans are the longest, spread over the SMs (tiles of 32 x 8 x 4 took 144 us there with
+// the split, against 106).
 constexpr int CT_X = 16, CT_Y = 8, CT_Z = 4, CT_K = CT_X * CT_Y * CT_Z / 256;
 
 // Component ICOMP of the CT_K far cells of a thread.
@@ -130,7 +133,7 @@ __device__ __forceinline__ void far_cells(const double *cf, double fac, const do
 
 template <typename TH, bool BATCH>
 __global__ void __launch_bounds__(256, 3) k_green_cells(TH *__restrict__ h, CellArgs a, CellGeom g0,
-                                                     const CellGeom *__restrict__ gb) {
+                                                     const CellGeom *__restrict__ gb, bool split) {
     __shared__ double sF[(CT_X + 1) * (CT_Y + 1) * (CT_Z + 1)];
     __shared__ alignas(16) double sc[BATCH ? 4 * kSerP : 2];
     pdl_wait(h);
@@ -138,7 +141,7 @@ __global__ void __launch_bounds__(256, 3) k_green_cells(TH *__restrict__ h, Cell
     const CellGeom &g = BATCH ? gb[blockIdx.y] : g0;
     const int ntx = (a.nx + CT_X - 1) / CT_X, nty = (a.ny + CT_Y - 1) / CT_Y, ntz = (a.nz + CT_Z - 1) / CT_Z;
     // components of a tile side by side: the near tiles come early for all of them
-    const int ci = blockIdx.x % a.ncomp, t = blockIdx.x / a.ncomp;
+    const int nci = split ? a.ncomp : 1, ci = blockIdx.x % nci, t = blockIdx.x / nci;
     const int tx = t % ntx, ty = (t / ntx) % nty, tzz = t / (ntx * nty);
     const int half = tzz / ntz;  // zwrap: 1 for the negative displacements
     const int i0 = tx * CT_X, j0 = ty * CT_Y, k0 = (tzz - half * ntz) * CT_Z;
@@ -157,32 +160,38 @@ __global__ void __launch_bounds__(256, 3) k_green_cells(TH *__restrict__ h, Cell
     TH *out = h + (int64_t)blockIdx.y * a.hstride + (int64_t)(half * a.nz + k0 + lz) * plane + (int64_t)j * a.nx + i;
     const int64_t cstride = (int64_t)a.nmem * a.hstride;
     if (!far) {
-        const int icomp = a.comps[ci];
-        const double factor = (icomp == 1 || icomp == 2 ? g.gamma : 1.0) / (hx * hy * hz);
         const int mx = min(CT_X, a.nx - i0), my = min(CT_Y, a.ny - j0);
+#pragma unroll 1
+        for (int c = ci; c < a.ncomp; c += nci) {
+            const int icomp = a.comps[c];
+            const double factor = (icomp == 1 || icomp == 2 ? g.gamma : 1.0) / (hx * hy * hz);
+#pragma unroll 1
+            for (int q = threadIdx.x; q < (CT_X + 1) * (CT_Y + 1) * (CT_Z + 1); q += 256) {
+                const int cx = q % (CT_X + 1), r = q / (CT_X + 1), cy = r % (CT_Y + 1), cz = r / (CT_Y + 1);
+                if (cx <= mx && cy <= my && cz <= nz_t)
+                    sF[q] = igf_primitive(icomp, (i0 + cx - 0.5) * hx, (j0 + cy - 0.5) * hy,
+                                          (c0 + cz - 0.5) * hz + woff) * factor;
+            }
+            __syncthreads();
+            if (i < a.nx && j < a.ny) {
+                constexpr int sy = CT_X + 1, sz = sy * (CT_Y + 1);
 #pragma unroll
-        for (int q = threadIdx.x; q < (CT_X + 1) * (CT_Y + 1) * (CT_Z + 1); q += 256) {
-            const int cx = q % (CT_X + 1), r = q / (CT_X + 1), cy = r % (CT_Y + 1), cz = r / (CT_Y + 1);
-            if (cx <= mx && cy <= my && cz <= nz_t)
-                sF[q] = igf_primitive(icomp, (i0 + cx - 0.5) * hx, (j0 + cy - 0.5) * hy, (c0 + cz - 0.5) * hz + woff) *
-                        factor;
-        }
-        __syncthreads();
-        if (i >= a.nx || j >= a.ny) return;
-        constexpr int sy = CT_X + 1, sz = sy * (CT_Y + 1);
-#pragma unroll
-        for (int k = 0; k < CT_K; ++k) {
-            if (k >= nk) break;
-            const double *f0 = sF + lx + sy * ly + sz * (lz + k);
-            double v = +f0[1 + sy + sz];
-            v = v - f0[sy + sz];
-            v = v - f0[1 + sz];
-            v = v - f0[1 + sy];
-            v = v - f0[0];
-            v = v + f0[sz];
-            v = v + f0[sy];
-            v = v + f0[1];
-            out[ci * cstride + k * plane] = k == zero ? (TH)0 : (TH)v;
+                for (int k = 0; k < CT_K; ++k) {
+                    if (k >= nk) break;
+                    const double *f0 = sF + lx + sy * ly + sz * (lz + k);
+                    double v = +f0[1 + sy + sz];
+                    v = v - f0[sy + sz];
+                    v = v - f0[1 + sz];
+                    v = v - f0[1 + sy];
+                    v = v - f0[0];
+                    v = v + f0[sz];
+                    v = v + f0[sy];
+                    v = v + f0[1];
+                    out[c * cstride + k * plane] = k == zero ? (TH)0 : (TH)v;
+                }
+            }
+            if (nci == a.ncomp) return;
+            __syncthreads();
         }
         return;
     }
@@ -219,20 +228,27 @@ __global__ void __launch_bounds__(256, 3) k_green_cells(TH *__restrict__ h, Cell
     }
 }
 
-static dim3 cells_grid(const CellArgs &a) {
+// CTAs of a launch; split where one CTA per component of every tile is still within two waves.
+static dim3 cells_grid(const CellArgs &a, bool &split) {
     const int64_t ntx = ceil_div(a.nx, CT_X), nty = ceil_div(a.ny, CT_Y), ntz = ceil_div(a.nz, CT_Z);
-    return dim3((unsigned)(ntx * nty * ntz * (a.zwrap ? 2 : 1) * a.ncomp), (unsigned)a.nmem);
+    const int64_t nt = ntx * nty * ntz * (a.zwrap ? 2 : 1);
+    split = nt * a.ncomp * a.nmem <= 148 * 3 * 2;
+    return dim3((unsigned)(nt * (split ? a.ncomp : 1)), (unsigned)a.nmem);
 }
 template <typename TH> int launch_green_cells(TH *h, const CellArgs &a, const CellGeom &g, cudaStream_t st) {
     if (a.nmem != 1 || a.ncomp < 1 || a.ncomp > 4) return OSC_E_INVALID;
-    launch_pdl(k_green_cells<TH, false>, cells_grid(a), dim3(256), 0, st, h, a, g, nullptr);
+    bool split;
+    const dim3 grid = cells_grid(a, split);
+    launch_pdl(k_green_cells<TH, false>, grid, dim3(256), 0, st, h, a, g, nullptr, split);
     return ok();
 }
 template int launch_green_cells<float>(float *, const CellArgs &, const CellGeom &, cudaStream_t);
 template int launch_green_cells<double>(double *, const CellArgs &, const CellGeom &, cudaStream_t);
 int launch_green_cells_batch(float *h, const CellArgs &a, const CellGeom *g, cudaStream_t st) {
     if (a.nmem < 1 || a.ncomp < 1 || a.ncomp > 4) return OSC_E_INVALID;
-    launch_pdl(k_green_cells<float, true>, cells_grid(a), dim3(256), 0, st, h, a, CellGeom{}, g);
+    bool split;
+    const dim3 grid = cells_grid(a, split);
+    launch_pdl(k_green_cells<float, true>, grid, dim3(256), 0, st, h, a, CellGeom{}, g, split);
     return ok();
 }
 
