@@ -677,73 +677,69 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
     pdl_trigger();
     __syncthreads();
     if constexpr (E::kLen > 0) {
-        // static engine (L = 2n known, L*NL/E::kEPT threads): each thread first loads its
-        // share of the n+1 distinct values of every line into registers (all loads in
-        // flight), then writes each value at e and its parity image at L-e
-        constexpr int nh = E::kLen / 2, NK = nh + 1, TOT = 2 * NL * NK;
+        // static engine (L = 2n known, L*NL/E::kEPT threads): each thread first loads its share of
+        // the n+1 distinct values of every line pair into registers (all loads in flight), then
+        // writes each pair of values at e and its parity image at L-e
+        constexpr int nh = E::kLen / 2, NK = nh + 1, TOT = NL * NK;
         constexpr int NT = E::kLen * NL / E::kEPT, IT = (TOT + NT - 1) / NT;
-        TC v[IT];
+        V v[IT];
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
             const int idx = tid + it * NT;
-            v[it] = (TC)0;
+            v[it] = mk<TC>(0, 0);
             if (idx < TOT) {
-                int rr, e;
-                if (LDE) { rr = idx / NK; e = idx - rr * NK; }
-                else { e = idx / (2 * NL); rr = idx - e * (2 * NL); }
-                const int64_t o = bin[rr];
-                if (o >= 0 && e != nh) v[it] = (TC)in[o + (int64_t)e * a.in_es];
+                const int ln = LDE ? idx / NK : idx % NL, e = LDE ? idx - ln * NK : idx / NL;
+                const int64_t o0 = bin[2 * ln], o1 = bin[2 * ln + 1];
+                if (o0 >= 0 && e != nh) v[it].x = (TC)in[o0 + (int64_t)e * a.in_es];
+                if (o1 >= 0 && e != nh) v[it].y = (TC)in[o1 + (int64_t)e * a.in_es];
             }
         }
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
             const int idx = tid + it * NT;
             if (idx < TOT) {
-                int rr, e;
-                if (LDE) { rr = idx / NK; e = idx - rr * NK; }
-                else { e = idx / (2 * NL); rr = idx - e * (2 * NL); }
-                reinterpret_cast<TC *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = v[it];
+                const int ln = LDE ? idx / NK : idx % NL, e = LDE ? idx - ln * NK : idx / NL;
+                buf[e * lstr + ln] = v[it];
                 if (e > 0 && e < nh)
-                    reinterpret_cast<TC *>(&buf[(E::kLen - e) * lstr + (rr >> 1)])[rr & 1] =
-                        podd[rr] ? -v[it] : v[it];
+                    buf[(E::kLen - e) * lstr + ln] = podd[2 * ln] ? mk<TC>(-v[it].x, -v[it].y) : v[it];
             }
         }
     } else {
         // each of the n+1 distinct values is read once and written at e and at L - e
-        auto put = [&](int rr, int e) {
-            const int64_t o = bin[rr];
-            TC v = (TC)0;
-            if (o >= 0 && e != n) v = (TC)in[o + (int64_t)e * a.in_es];
-            reinterpret_cast<TC *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = v;
-            if (e > 0 && e < n) reinterpret_cast<TC *>(&buf[(L - e) * lstr + (rr >> 1)])[rr & 1] = podd[rr] ? -v : v;
+        auto put = [&](int ln, int e) {
+            const int64_t o0 = bin[2 * ln], o1 = bin[2 * ln + 1];
+            V v = mk<TC>(0, 0);
+            if (o0 >= 0 && e != n) v.x = (TC)in[o0 + (int64_t)e * a.in_es];
+            if (o1 >= 0 && e != n) v.y = (TC)in[o1 + (int64_t)e * a.in_es];
+            buf[e * lstr + ln] = v;
+            if (e > 0 && e < n) buf[(L - e) * lstr + ln] = podd[2 * ln] ? mk<TC>(-v.x, -v.y) : v;
         };
-        if (LDE) for_rows(2 * NL, n + 1, put);
+        if (LDE) for_rows(NL, n + 1, put);
         else
 #pragma unroll 4
-            for (int idx = tid; idx < 2 * NL * (n + 1); idx += nthreads) put(idx % (2 * NL), idx / (2 * NL));
+            for (int idx = tid; idx < NL * (n + 1); idx += nthreads) put(idx % NL, idx / NL);
     }
     __syncthreads();
     const V *res = E::template run<V, NL, false, false>(buf, a.p, tw, +1);
     const int nk = n + 1;
-    auto fin = [&](int rr, int k) {
-        const int64_t o = bout[rr];
-        if (o < 0) return;
-        const V Z = res[k * lstr + (rr >> 1)];
-        const V Zm = res[(k > 0 ? L - k : 0) * lstr + (rr >> 1)];
-        const bool odd = podd[rr];
-        TC sv;
+    // both lines of a pair have the same parity (members start on even lines)
+    auto fin = [&](int ln, int k) {
+        const int64_t o0 = bout[2 * ln], o1 = bout[2 * ln + 1];
+        const V Z = res[k * lstr + ln], Zm = res[(k > 0 ? L - k : 0) * lstr + ln];
+        const bool odd = podd[2 * ln];
         const TC hf = (TC)0.5;
-        if ((rr & 1) == 0) sv = !odd ? hf * (Z.x + Zm.x) : hf * (Z.y - Zm.y);
-        else sv = !odd ? hf * (Z.y + Zm.y) : hf * (Zm.x - Z.x);
-        out[o + (int64_t)k * a.out_es] = (TO)(sv * (TC)a.scale);
+        const TC s0 = !odd ? hf * (Z.x + Zm.x) : hf * (Z.y - Zm.y);
+        const TC s1 = !odd ? hf * (Z.y + Zm.y) : hf * (Zm.x - Z.x);
+        if (o0 >= 0) out[o0 + (int64_t)k * a.out_es] = (TO)(s0 * (TC)a.scale);
+        if (o1 >= 0) out[o1 + (int64_t)k * a.out_es] = (TO)(s1 * (TC)a.scale);
     };
     if (!STK)
-        for (int idx = tid; idx < 2 * NL * nk; idx += nthreads) fin(idx % (2 * NL), idx / (2 * NL));
+        for (int idx = tid; idx < NL * nk; idx += nthreads) fin(idx % NL, idx / NL);
     else if constexpr (E::kLen > 0)
-        for (int idx = tid; idx < 2 * NL * (E::kLen / 2 + 1); idx += nthreads)
+        for (int idx = tid; idx < NL * (E::kLen / 2 + 1); idx += nthreads)
             fin(idx / (E::kLen / 2 + 1), idx % (E::kLen / 2 + 1));
     else
-        for_rows(2 * NL, nk, fin);
+        for_rows(NL, nk, fin);
 }
 
 // z transforms of the Green columns that are not even or odd in z (ZLineArgs): two real columns per
