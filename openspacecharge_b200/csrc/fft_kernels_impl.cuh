@@ -165,7 +165,8 @@ __device__ __forceinline__ float r2c_in(const float4 *__restrict__ p, const R2CA
 
 // resident CTAs the register allocation of k_r2c_rows is bounded for: 4 (32 registers, no
 // spills) for the FP32 step's quad-grid input on the 8-values-per-thread engine at L = 256,
-// whose loads wait on L2 (35.4 against 40.8 us at 40 registers and 3 CTAs); 1 otherwise
+// whose loads wait on L2 (35.4 against 40.8 us at 40 registers and 3 CTAs, then with one row of a
+// line per thread; 29 us with both); 1 otherwise
 template <typename T, typename TIn, class E> constexpr int r2c_minb() {
     return (std::is_same<TIn, float4>::value && E::kLen == 256 && E::kEPT == 8) ? 4 : 1;
 }
@@ -196,49 +197,40 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
         return (T)r2c_in(in + row * a.in_rstride, a, std::is_same<TIn, float4>::value ? jns[rr] : false, e);
     };
     if constexpr (E::kLen > 0) {
-        // all of a thread's loads are issued before any is stored to shared memory
+        // a thread carries both rows of a line; all of its loads are issued before any is stored to
+        // shared memory
         constexpr int LDL = HIN ? E::kLen / 2 : E::kLen, NT = E::kLen * NL / E::kEPT;
-        constexpr int IT = (2 * NL * LDL + NT - 1) / NT;
-        T v[IT];
+        constexpr int IT = (NL * LDL + NT - 1) / NT;
+        V v[IT];
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
-            const int idx = tid + it * NT, rr = idx / LDL, e = idx - rr * LDL;
-            v[it] = 0;
-            if (idx < 2 * NL * LDL) v[it] = elem(rr, e);
+            const int idx = tid + it * NT, ln = idx / LDL, e = idx - ln * LDL;
+            v[it] = mk<T>(0, 0);
+            if (idx < NL * LDL) v[it] = mk<T>(elem(2 * ln, e), elem(2 * ln + 1, e));
         }
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
-            const int idx = tid + it * NT, rr = idx / LDL, e = idx - rr * LDL;
-            if (idx < 2 * NL * LDL) reinterpret_cast<T *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = v[it];
+            const int idx = tid + it * NT, ln = idx / LDL, e = idx - ln * LDL;
+            if (idx < NL * LDL) buf[e * lstr + ln] = v[it];
         }
     } else {
-        for_rows(2 * NL, L, [&](int rr, int e) {
-            reinterpret_cast<T *>(&buf[e * lstr + (rr >> 1)])[rr & 1] = elem(rr, e);
-        });
+        for_rows(NL, L, [&](int ln, int e) { buf[e * lstr + ln] = mk<T>(elem(2 * ln, e), elem(2 * ln + 1, e)); });
     }
     __syncthreads();
     const V *res = E::template run<V, NL, HIN, false>(buf, a.p, tw, +1);
-    auto put = [&](int rr, int k) {
-        const int64_t row = row0 + rr;
-        if (row >= a.nrows) return;
-        const int line = rr >> 1;
-        const V Z = res[k * lstr + line];
-        const V Zm = res[(k > 0 ? L - k : 0) * lstr + line];
-        V r;
-        if ((rr & 1) == 0) {  // (Z + conj Zm)/2
-            r.x = (T)0.5 * (Z.x + Zm.x);
-            r.y = (T)0.5 * (Z.y - Zm.y);
-        } else {  // (Z - conj Zm)/(2i)
-            r.x = (T)0.5 * (Z.y + Zm.y);
-            r.y = (T)0.5 * (Zm.x - Z.x);
-        }
-        out[row * a.out_rstride + k] = r;
+    auto put = [&](int ln, int k) {
+        const int64_t row = row0 + 2 * ln;
+        const V Z = res[k * lstr + ln], Zm = res[(k > 0 ? L - k : 0) * lstr + ln];
+        V *o = out + row * a.out_rstride + k;
+        // (Z + conj Zm)/2 and (Z - conj Zm)/(2i)
+        if (row < a.nrows) *o = mk<T>((T)0.5 * (Z.x + Zm.x), (T)0.5 * (Z.y - Zm.y));
+        if (row + 1 < a.nrows) o[a.out_rstride] = mk<T>((T)0.5 * (Z.y + Zm.y), (T)0.5 * (Zm.x - Z.x));
     };
     if constexpr (E::kLen > 0) {
         constexpr int nh = E::kLen / 2 + 1;
-        for (int idx = tid; idx < 2 * NL * nh; idx += nthreads) put(idx / nh, idx % nh);
+        for (int idx = tid; idx < NL * nh; idx += nthreads) put(idx / nh, idx % nh);
     } else {
-        for_rows(2 * NL, L / 2 + 1, put);
+        for_rows(NL, L / 2 + 1, put);
     }
 }
 
@@ -483,6 +475,25 @@ __device__ __forceinline__ void st_pair(float4 *p, const float4 &lo, const float
 __device__ __forceinline__ void st_node(double4 *p, double x, double y, double z) {
     asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(0.0) : "memory");
 }
+// Node x of the two real rows (row, row + 1) that came out as one complex line per component:
+// z0 at x and, for x-pairs, z1 at x + 1 (0 past the end).
+template <typename T>
+__device__ __forceinline__ void e8_rows(const C2RArgs &a, const cplx<T> (&z0)[3], const cplx<T> (&z1)[3], int64_t row,
+                                        const int64_t *rout, int nout, int x) {
+    if constexpr (sizeof(T) == 4) {
+        float4 *g = reinterpret_cast<float4 *>(a.e8);
+        if (row < a.nrows)
+            st_pair(g + 2 * (rout[0] * nout + x), make_float4(z0[0].x, z0[1].x, z0[2].x, 0.f),
+                    make_float4(z1[0].x, z1[1].x, z1[2].x, 0.f));
+        if (row + 1 < a.nrows)
+            st_pair(g + 2 * (rout[1] * nout + x), make_float4(z0[0].y, z0[1].y, z0[2].y, 0.f),
+                    make_float4(z1[0].y, z1[1].y, z1[2].y, 0.f));
+    } else {
+        double4 *g = reinterpret_cast<double4 *>(a.e8);
+        if (row < a.nrows) st_node(g + rout[0] * nout + x, z0[0].x, z0[1].x, z0[2].x);
+        if (row + 1 < a.nrows) st_node(g + rout[1] * nout + x, z0[0].y, z0[1].y, z0[2].y);
+    }
+}
 template <typename T, class E> constexpr int c2r_e8_nlc() {
     return (E::kLen <= 128 ? 16 : (E::kLen <= 256 ? 8 : 4)) / (sizeof(T) == 8 ? 2 : 1);
 }
@@ -553,32 +564,15 @@ __global__ void __launch_bounds__(E::kLen * 3 * NLC / E::kEPT, sizeof(T) == 4 ? 
     }
     __syncthreads();
     E::template run<V, NLT, false, true>(buf, a.p, tw, -1);
-    for (int idx = tid; idx < 2 * NLC * nout; idx += nthreads) {
-        const int rr = idx / nout, x = idx - rr * nout;
-        const int64_t row = row0 + rr;
-        if (row >= a.nrows) continue;
-        const int ln = rr >> 1;
-        const bool odd = rr & 1;
-        T e0[3], e1[3];
+    for (int idx = tid; idx < NLC * nout; idx += nthreads) {
+        const int ln = idx / nout, x = idx - ln * nout;
+        V z0[3], z1[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const V z0 = buf[x * lstr + c * NLC + ln];
-            e0[c] = odd ? z0.y : z0.x;
-            if constexpr (sizeof(T) == 4) {
-                if (x + 1 < nout) {
-                    const V z1 = buf[(x + 1) * lstr + c * NLC + ln];
-                    e1[c] = odd ? z1.y : z1.x;
-                } else {
-                    e1[c] = 0;
-                }
-            }
+            z0[c] = buf[x * lstr + c * NLC + ln];
+            if constexpr (sizeof(T) == 4) z1[c] = x + 1 < nout ? buf[(x + 1) * lstr + c * NLC + ln] : mk<T>(0, 0);
         }
-        if constexpr (sizeof(T) == 4) {
-            st_pair(reinterpret_cast<float4 *>(a.e8) + 2 * (rout[rr] * nout + x),
-                    make_float4(e0[0], e0[1], e0[2], 0.f), make_float4(e1[0], e1[1], e1[2], 0.f));
-        } else {
-            st_node(reinterpret_cast<double4 *>(a.e8) + rout[rr] * nout + x, e0[0], e0[1], e0[2]);
-        }
+        e8_rows<T>(a, z0, z1, row0 + 2 * ln, &rout[2 * ln], nout, x);
     }
 }
 
@@ -619,23 +613,14 @@ __global__ void __launch_bounds__(FftRuntime::kMaxThreads) k_c2r_e8_rt(const cpl
         for_rows(NLT, half + 1, put);
     __syncthreads();
     const V *res = FftRuntime::template run<V, NLT, false, true>(buf, a.p, tw, -1);
-    for_rows(2 * NLC, nout, [&](int rr, int x) {
-        const int64_t row = row0 + rr;
-        if (row >= a.nrows) return;
-        const int ln = rr >> 1;
-        const bool odd = rr & 1;
-        T e0[3], e1[3];
+    for_rows(NLC, nout, [&](int ln, int x) {
+        V z0[3], z1[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const V z0 = res[x * lstr + c * NLC + ln], z1 = res[(x + 1) * lstr + c * NLC + ln];
-            e0[c] = odd ? z0.y : z0.x;
-            e1[c] = x + 1 < nout ? (odd ? z1.y : z1.x) : (T)0;
+            z0[c] = res[x * lstr + c * NLC + ln];
+            if constexpr (sizeof(T) == 4) z1[c] = x + 1 < nout ? res[(x + 1) * lstr + c * NLC + ln] : mk<T>(0, 0);
         }
-        if constexpr (sizeof(T) == 4)
-            st_pair(reinterpret_cast<float4 *>(a.e8) + 2 * (rout[rr] * nout + x),
-                    make_float4(e0[0], e0[1], e0[2], 0.f), make_float4(e1[0], e1[1], e1[2], 0.f));
-        else
-            st_node(reinterpret_cast<double4 *>(a.e8) + rout[rr] * nout + x, e0[0], e0[1], e0[2]);
+        e8_rows<T>(a, z0, z1, row0 + 2 * ln, &rout[2 * ln], nout, x);
     });
 }
 
