@@ -235,11 +235,10 @@ def kernel_bytes(nx, ny, nz, npart, at_cathode=False):
 
 
 def green_bytes(nx, ny, nz):
-    """Algorithmic bytes of one FP32 Green build (three E components): FP64 corner blocks
-    written and read once, FP32 octant differences, three FP32 line-transform passes, the
-    stored FP32 spectra written."""
+    """Algorithmic bytes of one FP32 Green build (three E components): FP32 cell integrals
+    written and read once, three FP32 line-transform passes, the stored FP32 spectra written."""
     c3 = (nx + 1) * (ny + 1) * (nz + 1)
-    return 3 * (8 * c3 + 8 * c3 + 4 * nx * ny * nz + 4 * nx * ny * nz + 4 * (nx + 1) * ny * nz +
+    return 3 * (4 * nx * ny * nz + 4 * nx * ny * nz + 4 * (nx + 1) * ny * nz +
                 4 * (nx + 1) * ny * nz + 4 * (nx + 1) * (ny + 1) * nz + 4 * (nx + 1) * (ny + 1) * nz + 4 * c3)
 
 
@@ -576,7 +575,7 @@ def run_ours(args, ws, rank, local, dist):
         refit = {"value": ws * 1000.0 / msr, "unit": "solves/s", "ms_per_step": msr, "steps": kr,
                  "green_build_ms": green_ms, "green_build_share": green_ms / msr,
                  "how": "resize_mesh=1 and the Green cache off (OSC_OPT_GREEN_CACHE_MB=0): bounding box, mesh "
-                        "refit, Green spectra rebuilt (FP64 IGF corners, octant differences, three even/odd "
+                        "refit, Green spectra rebuilt (cell integrals, three even/odd "
                         "line-transform passes), deposit, field, interpolation on every call",
                  "kernels": prof_r}
 
