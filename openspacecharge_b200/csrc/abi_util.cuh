@@ -93,8 +93,8 @@ inline void apply_refit(osc_mesh3d *mesh, const double bmin[3], const double bma
 // the particle bounding box computed on the device.
 inline int refit_mesh(osc_ctx *ctx, int64_t np, const double *x, const double *y, const double *z, osc_mesh3d *mesh) {
     if (np <= 0) return set_err(ctx, OSC_E_INVALID, "resize_mesh needs at least one particle");
-    unsigned long long *part;
-    TRY(ws_get(ctx, "bbox_part", sizeof(unsigned long long) * bbox_scratch_words(), (void **)&part));
+    double *part;
+    TRY(ws_get(ctx, "bbox_part", sizeof(double) * bbox_scratch_words(), (void **)&part));
     double *hb = reinterpret_cast<double *>(ctx->h_small + 16);
     {
         Launch L_(ctx, "bbox");

@@ -108,7 +108,7 @@ int launch_interp_pairs_runs(const InterpArgs &a, const float4 *E8, double *E, u
 // particles, written to out[7] (host memory mapped into the device).  part: bbox_scratch_words()
 // words; ticket: zero before its first use, left zero.
 int bbox_scratch_words();
-int launch_bbox(int64_t np, const double *x, const double *y, const double *z, unsigned long long *part,
+int launch_bbox(int64_t np, const double *x, const double *y, const double *z, double *part,
                 unsigned *ticket, double *out, cudaStream_t st);
 // Sum of q (or, with max_abs, the largest |q|), reduced in a fixed order into *out (mapped host
 // memory); ticket as above.
