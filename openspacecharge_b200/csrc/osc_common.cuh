@@ -87,8 +87,9 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // 128 x 128 x 256 takes 700 us against 220 and the z pass 180 against 140.  What it gains is a few
 // us per launch however large the grid is.  Steps in us with limits 0, 300, 600, 1200, 2400, 5000
 // (600 at most for the kernels without dynamic shared memory; "all" without a limit): 32 x 32 x 48
-// with refit 91 79 75 75 74 74 (all: 69), 64^3 117 114 114 114 110 110 (all: 106), 64^3 cathode with refit 350 342 339 333 329 329 (all: 323), 128^3 FP64 589 589 588 585 579
-// 580 (all: 688), 128 x 128 x 256 691 691 692 690 685 685 (all: 1227).
+// with refit 91 79 75 75 74 74 (all: 69), 64 x 64 x 128 117 114 114 114 110 110 (all: 106), 64^3
+// cathode with refit 350 342 339 333 329 329 (all: 323), 128^3 FP64 589 589 588 585 579 580 (all: 688),
+// 128 x 128 x 256 691 691 692 690 685 685 (all: 1227).
 inline bool pdl_early(uint64_t ctas, size_t smem) { return ctas <= (smem > 0 ? 2400u : 600u); }
 template <typename... KP, typename... A>
 inline void launch_pdl(void (*kern)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {

@@ -310,7 +310,7 @@ __device__ __forceinline__ void load_node(const vec4<T> *g, int64_t n, double &a
 // Two lanes to a particle, the even lane the four nodes at i and the odd lane those at i + 1: the
 // two 32-byte nodes of a row are adjacent, so that both loads travel as one request.  Bound by the
 // sectors the L1 and L2 hand out; 4e6 particles on 128^3: 169 us with one lane to a particle, 146 with
-// two.
+// two, 140.5 on 16 CTAs per SM instead of 64.
 template <typename T, typename TO>
 __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T> *__restrict__ g, TO *__restrict__ E,
                                                      TO *__restrict__ B, double bcoef,
@@ -375,7 +375,7 @@ template <typename T>
 int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp, cudaStream_t st,
                        double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
-    launch_pdl(k_interp_vec4<T, double>, dim3(nblocks(a.np, 256, 148 * 64)), dim3(256), 0, st, a,
+    launch_pdl(k_interp_vec4<T, double>, dim3(nblocks(a.np, 256, 148 * 16)), dim3(256), 0, st, a,
                reinterpret_cast<const vec4<T> *>(E4), E, B, bcoef, nclamp);
     return ok();
 }
@@ -613,7 +613,10 @@ int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsign
                         cudaStream_t st, double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(E8) % 32) return OSC_E_INVALID;
-    const int64_t cap = 148 * (int64_t)(a.ctas > 0 ? a.ctas : 64);
+    // 16 CTAs per SM (four are resident): with more, starting CTAs costs what their prefetch of the next
+    // particle gains (64 per SM: 1e7 particles 226 us against 219, 4e6 98.8 against 94.2, 2e6 on 128^3 58.4
+    // against 53.6), and 8 leave 1e7 particles on 64^3 a longer tail (220.2 against 217.5)
+    const int64_t cap = 148 * (int64_t)(a.ctas > 0 ? a.ctas : 16);
     const unsigned nb = nblocks(a.np, 256, cap);
     launch_pdl(pdl_early(nb, 0) ? k_interp_pairs<true> : k_interp_pairs<false>, dim3(nb), dim3(256), 0, st, a, E8, E, B,
                bcoef, nclamp);
@@ -1099,7 +1102,7 @@ __global__ void __launch_bounds__(256) k_vjp_particles(InterpArgs ia, DepositArg
 // at the nodes and interpolated side by side (75 FP64 operations instead of 230 with the value and the
 // three slopes of each component kept apart), which leaves room for four CTAs per SM (64 registers, no
 // spills) to cover the gather's latency: 4e6 particles on 128^3 170 us before, 115 with three CTAs
-// (80 registers), 105 with four.
+// (80 registers), 105 with four, 102.7 on 16 CTAs per SM of the grid instead of 64.
 template <bool EARLY>
 __global__ void __launch_bounds__(256, 4) k_vjp_pairs(InterpArgs ia, DepositArgs da, const float4 *__restrict__ g8,
                                                    const double *__restrict__ gE, double *gx, double *gy, double *gz,
@@ -1184,7 +1187,7 @@ int launch_vjp_pairs(const InterpArgs &ia, const DepositArgs &da, const float *e
                      double *gy, double *gz, double *gq, cudaStream_t st) {
     if (ia.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(e8) % 32) return OSC_E_INVALID;
-    const unsigned nb = nblocks(ia.np, 256, 148 * 64);
+    const unsigned nb = nblocks(ia.np, 256, 148 * 16);
     launch_pdl(pdl_early(nb, 0) ? k_vjp_pairs<true> : k_vjp_pairs<false>, dim3(nb), dim3(256), 0, st, ia, da,
                reinterpret_cast<const float4 *>(e8), gE, gx, gy, gz, gq);
     return ok();
