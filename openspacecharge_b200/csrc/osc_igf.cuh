@@ -9,32 +9,26 @@
 
 namespace osc {
 
-// log(r + t) with r^2 = s2 + t^2.  For t < 0 the sum cancels (with a cell edge of 1e-4 at a distance of
-// 0.16 it keeps seven digits), and s2 / (r - t) is the same without the loss.
-__device__ __forceinline__ double igf_logsum(double r, double t, double s2) {
-    const double p = r + fabs(t);
-    return log(t < 0.0 ? s2 / p : p);
-}
-
 // \int 1/r dx dy dz  (code/open_spacecharge_mod.f90:741-747, lafun2)
 __device__ __forceinline__ double igf_lafun2(double x, double y, double z) {
     const double r = sqrt(x * x + y * y + z * z);
     double t = -((z * z) * atan(x * y / (z * r))) / 2;
     t = t - ((y * y) * atan(x * z / (y * r))) / 2;
     t = t - ((x * x) * atan(y * z / (x * r))) / 2;
-    t = t + y * z * igf_logsum(r, x, y * y + z * z);
-    t = t + x * z * igf_logsum(r, y, x * x + z * z);
-    t = t + x * y * igf_logsum(r, z, x * x + y * y);
+    t = t + y * z * log(x + r);
+    t = t + x * z * log(y + r);
+    t = t + x * y * log(z + r);
     return t;
 }
 
 // \int x/r^3 dx dy dz  (code/open_spacecharge_mod.f90:721-726, xlafun2).  log((r - |z|) / (r + |z|)) is
-// taken as log((x^2 + y^2) / (r + |z|)^2): r - |z| loses the same digits as above.
+// taken as log((x^2 + y^2) / (r + |z|)^2), at the same cost: r - |z| cancels far along z (with a cell
+// edge of 1e-4 at a distance of 0.16 it keeps seven digits).
 __device__ __forceinline__ double igf_xlafun2(double x, double y, double z) {
     const double r = sqrt(x * x + y * y + z * z);
     const double q = r + fabs(z);
     const double lz = copysign(0.5, -z) * log((q * q) / (x * x + y * y));
-    return x * atan((y * z) / (r * x)) - z * igf_logsum(r, y, x * x + z * z) + y * lz;
+    return x * atan((y * z) / (r * x)) - z * log(r + y) + y * lz;
 }
 
 // Primitive of component icomp at (u,v,w): 0 phi, 1 Ex, 2 Ey, 3 Ez -- the argument
