@@ -422,7 +422,9 @@ static int green_set(osc_ctx *c, const FreeSpaceJob &j, const int *comps, int nc
             continue;
         }
         if (off[0] == 0.0 && off[1] == 0.0) {
-            const int rc = green_zoff_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off[2], s == 1, comps, ncomp, gs);
+            // the image z pass reads direct spectra that are even or odd in z too: not those of a user's z offset
+            const bool image = s == 1 && j.offset[2] == 0.0;
+            const int rc = green_zoff_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off[2], image, comps, ncomp, gs);
             if (rc) {
                 for (int q = 0; q < gs.nspec; ++q) green_release(c, gs.buf[q]);
                 return rc;
