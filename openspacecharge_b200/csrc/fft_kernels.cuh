@@ -201,6 +201,14 @@ int launch_c2r_rows(const cplx<T> *in, const C2RArgs &a, const TwPair<cplx<T>> &
 // True when the z pass of length L with nz = L/2 non-zero planes runs the warp-per-column
 // kernel, whose Green spectra must be stored with zinner set.
 bool zconv_warp_ok(int L, int nz, int elem_bytes);
+// Layout of a convolution's Green spectra: kz-innermost for the warp-per-column z pass, or
+// kz-outermost for the CTA one.  staged: all spectra real and even or odd in z (a kernel without an
+// offset, and its images), whose columns the warp kernels stage in shared memory.  The others are read
+// complex and in full from global memory, and at the doubled lengths 32 and 64 a warp per column
+// has too few bytes in flight for that: 128 x 128 x 32 displaced, with images, takes 181 us in FP32 and
+// 340 in FP64 with a warp per column, 92 and 177 with CTAs of eight columns (128 x 128 x 16 132 and 330
+// against 72 and 162; a pipe on 128 x 64 x 32 FP64 73).  Lengths from 96 on keep the warps.
+bool zconv_zinner(int L, int nz, int elem_bytes, bool staged);
 // True when the cathode-image z pass (zconv_img.cuh) covers length L: the warp-per-column
 // lengths whose first-stage butterfly count L/R is a multiple of 32 or below 32.
 bool zconv_img_ok(int L, int nz, int elem_bytes);

@@ -1090,8 +1090,9 @@ int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPa
     const int L = a.p.L;
     // a column range of a z slab runs on the radix warp engine only
     const bool whole = a.col_base == 0 && (int64_t)a.ncols == (int64_t)a.nxh * a.Ny;
-    if (a.col_base != 0 && (!zconv_warp_ok(L, a.nz, (int)sizeof(T)) || a.nsum > 0)) return OSC_E_UNSUPPORTED;
-    if (zconv_warp_ok(L, a.nz, (int)sizeof(T))) {
+    const bool warp = zconv_warp_ok(L, a.nz, (int)sizeof(T)) && (a.ng < 1 || a.g[0].zinner);
+    if (a.col_base != 0 && (!warp || a.nsum > 0)) return OSC_E_UNSUPPORTED;
+    if (warp) {
         for (int i = 0; i < a.ng; ++i)
             if (!a.g[i].zinner) return OSC_E_INVALID;  // spectra stored for the other z pass
         bool img = false, herm = false;

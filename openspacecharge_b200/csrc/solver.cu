@@ -179,7 +179,7 @@ template int green_sym_lines3<double>(osc_ctx *, const double *, int, int, int, 
 // components, in gs.buf[0], and gs.spec[i] points at component comps[i].
 template <typename T>
 static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[3], double gamma, const int *comps,
-                         int ncomp, GreenSet &gs) {
+                         int ncomp, int zinner, GreenSet &gs) {
     T *h;
     TRY(ws_get(c, "green_h", sizeof(T) * (size_t)ncomp * nx * ny * nz, (void **)&h));
     {
@@ -197,7 +197,6 @@ static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[
                                                            kSerRatio), c->stream),
                  "green cells"));
     }
-    const int zinner = zconv_warp_ok(2 * nz, nz, (int)sizeof(T)) ? 1 : 0;
     const int zp = zinner ? green_zpitch(nz + 1, sizeof(T)) : nz + 1;
     const int64_t per = (int64_t)(nx + 1) * (ny + 1) * zp;
     DevBuf store;
@@ -245,7 +244,7 @@ static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[
 // 64^3 cathode step with a refit mesh: 548 us that way, 381 this way).
 template <typename T>
 static int green_zoff_set(osc_ctx *c, int nx, int ny, int nz, const double delta[3], double gamma, double zoff,
-                          bool image, const int *comps, int ncomp, GreenSet &gs) {
+                          bool image, const int *comps, int ncomp, int zinner, GreenSet &gs) {
     const int Nz = 2 * nz, nxh = nx + 1, nyh = ny + 1;
     double *h, *hy;
     TRY(ws_get(c, "green_h", sizeof(double) * (size_t)ncomp * nx * ny * Nz, (void **)&h));
@@ -276,7 +275,7 @@ static int green_zoff_set(osc_ctx *c, int nx, int ny, int nz, const double delta
     TRY(green_sym_xy<double>(c, h, ncomp, nx, ny, Nz, odd, &hy));
     GSpecDev s{};
     s.sym_y = 1;
-    s.zinner = zconv_warp_ok(Nz, nz, (int)sizeof(T)) ? 1 : 0;
+    s.zinner = zinner;
     s.herm_img = image && zconv_img_ok(Nz, nz, (int)sizeof(T)) ? 1 : 0;
     s.dimy = nyh;
     s.dimz = s.herm_img ? nz + 1 : Nz;
@@ -325,7 +324,7 @@ static int green_zoff_set(osc_ctx *c, int nx, int ny, int nz, const double delta
 // complex doubled grid, an FP64 3D FFT and the extraction into the stored layout.
 template <typename T>
 static int build_green_component(osc_ctx *c, int nx, int ny, int nz, const double delta[3], double gamma,
-                                 const double off[3], int icomp, DevBuf &store, GSpecDev &spec) {
+                                 const double off[3], int icomp, int zinner, DevBuf &store, GSpecDev &spec) {
     const int n[3] = {nx, ny, nz};
     const int N[3] = {2 * nx, 2 * ny, 2 * nz};
     const int64_t M = (int64_t)N[0] * N[1] * N[2];
@@ -364,7 +363,7 @@ static int build_green_component(osc_ctx *c, int nx, int ny, int nz, const doubl
     spec.par_z = par[2];
     spec.dimy = sym[1] ? ny + 1 : N[1];
     spec.dimz = sym[2] ? nz + 1 : N[2];
-    spec.zinner = zconv_warp_ok(N[2], nz, (int)sizeof(T)) ? 1 : 0;
+    spec.zinner = zinner;
     spec.zpitch = spec.zinner ? green_zpitch(spec.dimz, spec.real_valued ? sizeof(T) : sizeof(cplx<T>)) : spec.dimz;
     const size_t elems = (size_t)(nx + 1) * spec.dimy * spec.zpitch;
     const size_t bytes = elems * (spec.real_valued ? sizeof(T) : sizeof(cplx<T>));
@@ -410,11 +409,13 @@ static int green_set(osc_ctx *c, const FreeSpaceJob &j, const int *comps, int nc
     GreenSet gs;
     gs.key = key;
     const int nsets = j.at_cathode ? 2 : 1;
+    const bool displaced = j.offset[0] != 0.0 || j.offset[1] != 0.0 || j.offset[2] != 0.0;
+    const int zinner = zconv_zinner(2 * j.nz, j.nz, (int)sizeof(T), !displaced) ? 1 : 0;
     for (int s = 0; s < nsets; ++s) {
         double off[3] = {j.offset[0], j.offset[1], j.offset[2]};
         if (s == 1) off[2] = off[2] + j.img_zoff;
         if (off[0] == 0.0 && off[1] == 0.0 && off[2] == 0.0) {
-            const int rc = green_sym_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, comps, ncomp, gs);
+            const int rc = green_sym_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, comps, ncomp, zinner, gs);
             if (rc) {
                 for (int q = 0; q < gs.nspec; ++q) green_release(c, gs.buf[q]);
                 return rc;
@@ -424,7 +425,8 @@ static int green_set(osc_ctx *c, const FreeSpaceJob &j, const int *comps, int nc
         if (off[0] == 0.0 && off[1] == 0.0) {
             // the image z pass reads direct spectra that are even or odd in z too: not those of a user's z offset
             const bool image = s == 1 && j.offset[2] == 0.0;
-            const int rc = green_zoff_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off[2], image, comps, ncomp, gs);
+            const int rc = green_zoff_set<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off[2], image, comps, ncomp, zinner,
+                                             gs);
             if (rc) {
                 for (int q = 0; q < gs.nspec; ++q) green_release(c, gs.buf[q]);
                 return rc;
@@ -433,8 +435,8 @@ static int green_set(osc_ctx *c, const FreeSpaceJob &j, const int *comps, int nc
         }
         for (int i = 0; i < ncomp; ++i) {
             const int k = gs.nspec;
-            int rc = build_green_component<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off, comps[i],
-                                                       gs.buf[k], gs.spec[k]);
+            int rc = build_green_component<T>(c, j.nx, j.ny, j.nz, j.delta, j.gamma, off, comps[i], zinner,
+                                              gs.buf[k], gs.spec[k]);
             if (rc) {
                 for (int q = 0; q <= k; ++q) green_release(c, gs.buf[q]);
                 return rc;
@@ -612,7 +614,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     za.in_estride = (int64_t)nxh * Ny;
     // the warp-per-column z pass writes its spectra kz-innermost ([o][b][ky][kx][z]); the
     // inverse y and x passes then read them with adjacent z in adjacent lines
-    const bool zin = zconv_warp_ok(Nz, nz, (int)sizeof(T));
+    const bool zin = gs->spec[0].zinner != 0;
     za.out_estride = zin ? 1 : (int64_t)nxh * Ny;
     za.out_colstride = zin ? nz : 1;
     za.out_cstride = (int64_t)Bout * nxh * Ny * nz;
