@@ -78,6 +78,14 @@ template <typename V> __host__ __device__ __forceinline__ V cmul_si(V a, int s) 
 template <typename Ptr> __device__ __forceinline__ void pdl_wait(Ptr &p) {
     asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
 }
+// The same where the compiler has to go on knowing that p points to global memory: loads through the
+// pointer that comes out of pdl_wait are generic ones, which keep their order with stores to
+// shared memory, so that a loop that copies rows there has one load in flight at a time.
+template <typename Ptr> __device__ __forceinline__ void pdl_wait_global(Ptr &p) {
+    size_t g = __cvta_generic_to_global(p);
+    pdl_wait(g);
+    p = reinterpret_cast<Ptr>(__cvta_global_to_generic(g));
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Kernels with dynamic shared memory start this way up to 2400 CTAs, the others (particle and
