@@ -26,9 +26,17 @@ namespace osc {
 // Line buffers of a kernel that transforms in shared memory (FftRuntime alternates between two).
 template <class E> constexpr int eng_bufs() { return E::kLen > 0 ? 1 : 2; }
 
-// f(row, e) for e < len of rows [0, nrows): whole warps walk a row, so that no index is divided
-// by a length known only at run time.
-template <class F> __device__ __forceinline__ void for_rows(int nrows, int len, F &&f) {
+// f(row, e) for e < len of rows [0, nrows).  Where len is the compile-time LEN, threads walk the flat
+// sequence; otherwise whole warps walk a row, so that no index is divided by a length known only
+// at run time, at the price of part-empty warps at the ends of rows: the x inverse to planes of
+// 16 x 16 x 16 takes 28.9 us with rows of 16 walked by warps, 18.9 flat.
+template <int LEN, class F> __device__ __forceinline__ void for_rows(int nrows, int len, F &&f) {
+    if constexpr (LEN > 0) {
+        if (len == LEN) {
+            for (int idx = threadIdx.x; idx < nrows * LEN; idx += blockDim.x) f(idx / LEN, idx % LEN);
+            return;
+        }
+    }
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 #pragma unroll 2
     for (int r = threadIdx.x >> 5; r < nrows; r += nw)
@@ -136,11 +144,11 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_lines(const cplx<T> *in, cpl
     if constexpr (E::kLen > 0)
         for (int idx = tid; idx < NL * E::kLen; idx += nthreads) put(idx / E::kLen, idx % E::kLen);
     else
-        for_rows(NL, L, put);
+        for_rows<0>(NL, L, put);
     __syncthreads();
     const V *res = E::template run<V, NL, false, false>(buf, a.p, tw, a.sign);
     const T sc = (T)a.scale;
-    for_rows(NL, a.out_len, [&](int c, int e) {
+    for_rows<0>(NL, a.out_len, [&](int c, int e) {
         const int col = col0 + c;
         const int p = e + a.out_lo, src_e = ((a.flip_mask >> blockIdx.z) & 1u) && p > 0 ? L - p : p;
         if (col < a.ncols)
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
             if (idx < NL * LDL) buf[e * lstr + ln] = v[it];
         }
     } else {
-        for_rows(NL, L, [&](int ln, int e) { buf[e * lstr + ln] = mk<T>(elem(2 * ln, e), elem(2 * ln + 1, e)); });
+        for_rows<0>(NL, L, [&](int ln, int e) { buf[e * lstr + ln] = mk<T>(elem(2 * ln, e), elem(2 * ln + 1, e)); });
     }
     __syncthreads();
     const V *res = E::template run<V, NL, HIN, false>(buf, a.p, tw, +1);
@@ -233,7 +241,7 @@ __global__ void __launch_bounds__(E::kMaxThreads, r2c_minb<T, TIn, E>()) k_r2c_r
         constexpr int nh = E::kLen / 2 + 1;
         for (int idx = tid; idx < NL * nh; idx += nthreads) put(idx / nh, idx % nh);
     } else {
-        for_rows(NL, L / 2 + 1, put);
+        for_rows<0>(NL, L / 2 + 1, put);
     }
 }
 
@@ -319,10 +327,10 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
         if (a.zin)  // adjacent lines (adjacent z) fastest for the kz-innermost spectra
             for (int idx = tid; idx < NL * L; idx += nthreads) put(idx % NL, idx / NL);
         else
-            for_rows(NL, L, put);
+            for_rows<E::kLen>(NL, L, put);
         __syncthreads();
         const V *fb = E::template run<V, NL, false, HOUT>(buf, a.p, tw, -1);
-        for_rows(2 * NL, a.nout, [&](int rr, int x) {
+        for_rows<E::kLen / 2>(2 * NL, a.nout, [&](int rr, int x) {
             const int64_t row = row0 + rr;
             if (row >= a.nrows) return;
             const int xs = ((a.flip_mask >> c) & 1u) && x > 0 ? L - x : x;
@@ -342,7 +350,7 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_c2r_rows(const cplx<T> *__re
         // x-pair grid rows: node n gets (E(n), E(n+1)), the row's last node (E(n), 0)
         typedef vec4<T> V4;
         V4 *g = reinterpret_cast<V4 *>(a.e8);
-        for_rows(2 * NL, a.nout, [&](int rr, int x) {
+        for_rows<E::kLen / 2>(2 * NL, a.nout, [&](int rr, int x) {
             const int64_t row = row0 + rr;
             if (row >= a.nrows) return;
             const int64_t gidx = rout[rr] * a.nout + x;
@@ -613,10 +621,10 @@ __global__ void __launch_bounds__(FftRuntime::kMaxThreads) k_c2r_e8_rt(const cpl
 #pragma unroll 4
         for (int idx = tid; idx < NLT * (half + 1); idx += blockDim.x) put(idx % NLT, idx / NLT);
     else
-        for_rows(NLT, half + 1, put);
+        for_rows<0>(NLT, half + 1, put);
     __syncthreads();
     const V *res = FftRuntime::template run<V, NLT, false, true>(buf, a.p, tw, -1);
-    for_rows(NLC, nout, [&](int ln, int x) {
+    for_rows<0>(NLC, nout, [&](int ln, int x) {
         V z0[3], z1[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -702,7 +710,7 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
             buf[e * lstr + ln] = v;
             if (e > 0 && e < n) buf[(L - e) * lstr + ln] = podd[2 * ln] ? mk<TC>(-v.x, -v.y) : v;
         };
-        if (LDE) for_rows(NL, n + 1, put);
+        if (LDE) for_rows<0>(NL, n + 1, put);
         else
 #pragma unroll 4
             for (int idx = tid; idx < NL * (n + 1); idx += nthreads) put(idx % NL, idx / NL);
@@ -727,7 +735,7 @@ __global__ void __launch_bounds__(E::kMaxThreads) k_sym_lines(const TI *__restri
         for (int idx = tid; idx < NL * (E::kLen / 2 + 1); idx += nthreads)
             fin(idx / (E::kLen / 2 + 1), idx % (E::kLen / 2 + 1));
     else
-        for_rows(NL, nk, fin);
+        for_rows<0>(NL, nk, fin);
 }
 
 // z transforms of the Green columns that are not even or odd in z (ZLineArgs): two real columns per
