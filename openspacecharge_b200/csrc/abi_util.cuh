@@ -121,6 +121,7 @@ inline int charge_queue(osc_ctx *ctx, int64_t np, const double *q, int word, boo
 // rest of the step is queued: the GPU does not idle in between.
 inline int charge_wait(osc_ctx *ctx, int word, double *v) {
     CK(cudaEventSynchronize(ctx->charge_ev), "wait for charge");
+    TRY(fault_check(ctx));  // of an earlier call's kernels, complete before the sum
     *v = *reinterpret_cast<volatile double *>(ctx->h_small + word);
     return OSC_OK;
 }

@@ -57,7 +57,9 @@ int ws_get(osc_ctx *c, const char *name, size_t bytes, void **out) {
 
 int ctx_sync(osc_ctx *c) {
     const int rc = cuda_check(c, cudaStreamSynchronize(c->stream), "stream synchronize");
-    if (rc) return rc;
+    return rc ? rc : fault_check(c);
+}
+int fault_check(osc_ctx *c) {
     if (c->h_fault && *reinterpret_cast<volatile unsigned *>(c->h_fault)) {
         const unsigned f = *c->h_fault;
         *reinterpret_cast<volatile unsigned *>(c->h_fault) = 0;

@@ -132,6 +132,8 @@ int set_err(osc_ctx *c, int code, const char *fmt, ...);
 int cuda_check(osc_ctx *c, cudaError_t e, const char *what);
 // Synchronises the context stream, then reports (and clears) a fault word set by a kernel.
 int ctx_sync(osc_ctx *c);
+// The same without waiting: of the kernels known to be complete.
+int fault_check(osc_ctx *c);
 // Named device workspace of at least `bytes` (grown by reallocation; contents not kept).
 int ws_get(osc_ctx *c, const char *name, size_t bytes, void **out);
 // Twiddle tables of length L (runtime table and, when L has a static engine, its
