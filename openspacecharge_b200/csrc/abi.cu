@@ -505,13 +505,12 @@ int osc_space_charge_step_dev(osc_ctx *ctx, osc_mesh3d *mesh, int64_t np, const 
     if (!(mesh->gamma >= 1.0)) return set_err(ctx, OSC_E_INVALID, "gamma must be >= 1");
     ++ctx->step_calls;  // any earlier step's kept E grid is out of date from here on
     double charge1 = 0;
-    if (q) {
-        TRY(charge_queue(ctx, np, q, kChargeWord, false));
-    } else {
+    if (q) TRY(charge_queue(ctx, np, q, kChargeWord, false));
+    if (resize_mesh) TRY(refit_mesh(ctx, np, x, y, z, mesh));  // refused: the mesh stays as it was
+    if (!q) {
         mesh->charge = *total_charge;
         charge1 = *total_charge / (double)np;
     }
-    if (resize_mesh) TRY(refit_mesh(ctx, np, x, y, z, mesh));
     const int rc = step_queue(ctx, mesh, n, np, x, y, z, q, charge1, at_cathode, precision, E, B);
     const int rq = q ? charge_wait(ctx, kChargeWord, &mesh->charge) : OSC_OK;
     return rc ? rc : rq;
