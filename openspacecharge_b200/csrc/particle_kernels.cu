@@ -475,7 +475,8 @@ __global__ void __launch_bounds__(256) k_interp_pairs(InterpArgs a, const float4
     const int64_t plane = (int64_t)a.nx * a.ny;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    // the next particle's coordinates are loaded while this particle's field is gathered
+    // the next particle's coordinates are loaded while this particle's field is gathered, the first
+    // one's before the wait: started early only where the coordinates are settled
     double xn = 0, yn = 0, zn = 0;
     if (m < a.np) {
         xn = __ldg(a.x + m);
@@ -610,7 +611,7 @@ int launch_interp_pairs_runs(const InterpArgs &a, const float4 *E8, double *E, u
 }
 
 int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
-                        cudaStream_t st, double *B, double bcoef) {
+                        cudaStream_t st, double *B, double bcoef, bool settled) {
     if (a.np <= 0) return OSC_OK;
     if (reinterpret_cast<uintptr_t>(E8) % 32) return OSC_E_INVALID;
     // 16 CTAs per SM (four are resident): with more, starting CTAs costs what their prefetch of the next
@@ -618,8 +619,11 @@ int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsign
     // against 53.6), and 8 leave 1e7 particles on 64^3 a longer tail (220.2 against 217.5)
     const int64_t cap = 148 * (int64_t)(a.ctas > 0 ? a.ctas : 16);
     const unsigned nb = nblocks(a.np, 256, cap);
-    launch_pdl(pdl_early(nb, 0) ? k_interp_pairs<true> : k_interp_pairs<false>, dim3(nb), dim3(256), 0, st, a, E8, E, B,
-               bcoef, nclamp);
+    if (settled)
+        launch_pdl(pdl_early(nb, 0) ? k_interp_pairs<true> : k_interp_pairs<false>, dim3(nb), dim3(256), 0, st, a, E8, E, B,
+                   bcoef, nclamp);
+    else  // a kernel that starts early reads coordinates before it waits
+        k_interp_pairs<false><<<nb, 256, 0, st>>>(a, E8, E, B, bcoef, nclamp);
     return ok();
 }
 

@@ -96,8 +96,11 @@ int launch_interp_planes(const InterpArgs &a, const double *F, double *out,
                          unsigned long long *nclamp, cudaStream_t st);
 // Gather from an x-pair grid: node n holds (E(n), E(n+1)) as two float4 in one 32-byte
 // sector, so the 8 nodes of a particle come from 4 sectors.
+// settled: the kernels that wrote the coordinates were complete before the kernel queued last began
+// (as in a step, where kernels of the step lie between); false where the caller's own kernel may
+// be the last one, which can let others start before it has written them.
 int launch_interp_pairs(const InterpArgs &a, const float4 *E8, double *E, unsigned long long *nclamp,
-                        cudaStream_t st, double *B = nullptr, double bcoef = 0);
+                        cudaStream_t st, double *B = nullptr, double bcoef = 0, bool settled = true);
 // The same gather for particles in cell order: runs of consecutive particles in one cell
 // share their stencil's loads; coordinates and E move as 256-bit vectors.  Bit-identical
 // to launch_interp_pairs for any order.

@@ -100,7 +100,8 @@ int osc_slab_interp_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int p0, int np_pla
     InterpArgs ia = interp_args(&m, nl, np, x, y, z);
     ia.ctas = tune_get(ctx, "gather_ctas_per_sm");
     Launch L_(ctx, "interp_f32");
-    if (launch_interp_pairs(ia, reinterpret_cast<const float4 *>(e8), E, ctx->d_small + 2, ctx->stream))
+    if (launch_interp_pairs(ia, reinterpret_cast<const float4 *>(e8), E, ctx->d_small + 2, ctx->stream, nullptr, 0,
+                            false))
         return set_err(ctx, OSC_E_CUDA, "slab interp");
     return OSC_OK;
 }
