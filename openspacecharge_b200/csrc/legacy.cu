@@ -508,11 +508,12 @@ int pipe_solve(osc_ctx *c, int precision, const double delta[3], double gam0, co
             TRY(conv_extract(c, g, crho, ct, PIPE_INV[t], PIPE_SIGN[t] * factr, phi, t > 0));
         }
     }
-    if (e8) {  // E only as the x-pair grid of the FP32 gather
+    if (e8) {  // E as the x-pair grid of the FP32 gather; B, in FP64, from planes of its own
         Launch L_(c, "fd_efield");
-        return kchk(c, launch_fd_efield_pairs(phi, e8, g.n[0], g.n[1], g.n[2], delta[0], delta[1], delta[2], gam0,
-                                              c->stream),
-                    "fd pairs");
+        TRY(kchk(c, launch_fd_efield_pairs(phi, e8, g.n[0], g.n[1], g.n[2], delta[0], delta[1], delta[2], gam0,
+                                           c->stream),
+                 "fd pairs"));
+        if (!B) return OSC_OK;
     }
     if (!E) return set_err(c, OSC_E_INVALID, "pipe solve: E planes needed");
     {

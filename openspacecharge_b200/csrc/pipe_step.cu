@@ -26,18 +26,20 @@ int osc_space_charge_step_rectpipe_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int
     const int64_t N = (int64_t)n[0] * n[1] * n[2];
     const osc_mesh3d m = *mesh;
     const double charge1 = q ? 0.0 : *total_charge / (double)np;
-    double *rho, *phi, *Eg, *Bg;
-    TRY(ws_get(ctx, "ps_rho64", sizeof(double) * N, (void **)&rho));
+    double *rho, *phi, *Eg = nullptr, *Bg = nullptr;
     TRY(ws_get(ctx, "ps_phi", sizeof(double) * N, (void **)&phi));
-    TRY(ws_get(ctx, "ps_E", sizeof(double) * 3 * N, (void **)&Eg));
-    TRY(ws_get(ctx, "ps_B", sizeof(double) * 3 * N, (void **)&Bg));
     DepositArgs da = deposit_args(&m, n, np, x, y, z, q, charge1, ctx->check_finite);
     InterpArgs ia = interp_args(&m, n, np, x, y, z);
     const bool fp32 = precision == OSC_PREC_FP32 && ctx->deposit_mode == OSC_DEPOSIT_ATOMIC;
     if (fp32 && m.npad[0] == 1 && m.npad[1] == 1 && m.npad[2] == 1) {
         // the x transform reads the quad grid; E goes straight from phi to the x-pair grid,
-        // and B at a particle is that of E there
+        // and B, when it is wanted, through FP64 planes: phi's differences keep more bits than the
+        // FP32 pairs hold
         float *quad, *e8;
+        if (B) {
+            TRY(ws_get(ctx, "ps_E", sizeof(double) * 3 * N, (void **)&Eg));
+            TRY(ws_get(ctx, "ps_B", sizeof(double) * 3 * N, (void **)&Bg));
+        }
         TRY(ws_get(ctx, "ps_quad", sizeof(float) * 4 * N, (void **)&quad));
         TRY(ws_get(ctx, "ps_E8", sizeof(float) * 8 * N, (void **)&e8));
         {
@@ -45,14 +47,21 @@ int osc_space_charge_step_rectpipe_dev(osc_ctx *ctx, const osc_mesh3d *mesh, int
             if (launch_clear_quad(quad, N, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "clear quad");
             if (launch_deposit_quad(da, quad, ctx->d_small, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "deposit");
         }
-        TRY(pipe_solve_checked(ctx, &m, precision, nullptr, phi, nullptr, nullptr,
-                               reinterpret_cast<const float4 *>(quad), e8));
-        const double bcoef = std::sqrt(1 - 1 / (m.gamma * m.gamma)) / CLIGHT_CORE;
-        Launch L_(ctx, "interp_f32");
-        if (launch_interp_pairs(ia, reinterpret_cast<const float4 *>(e8), E, ctx->d_small + 2, ctx->stream, B, bcoef))
-            return set_err(ctx, OSC_E_CUDA, "interp");
+        TRY(pipe_solve_checked(ctx, &m, precision, nullptr, phi, Eg, Bg, reinterpret_cast<const float4 *>(quad), e8));
+        {
+            Launch L_(ctx, "interp_f32");
+            if (launch_interp_pairs(ia, reinterpret_cast<const float4 *>(e8), E, ctx->d_small + 2, ctx->stream))
+                return set_err(ctx, OSC_E_CUDA, "interp");
+        }
+        if (B) {
+            Launch L_(ctx, "interp_f64");
+            if (launch_interp_planes(ia, Bg, B, ctx->d_small + 3, ctx->stream)) return set_err(ctx, OSC_E_CUDA, "interp");
+        }
         return OSC_OK;
     }
+    TRY(ws_get(ctx, "ps_rho64", sizeof(double) * N, (void **)&rho));
+    TRY(ws_get(ctx, "ps_E", sizeof(double) * 3 * N, (void **)&Eg));
+    TRY(ws_get(ctx, "ps_B", sizeof(double) * 3 * N, (void **)&Bg));
     if (fp32) {
         float *quad, *rho32;
         TRY(ws_get(ctx, "ps_quad", sizeof(float) * 4 * N, (void **)&quad));
