@@ -644,12 +644,12 @@ int step_queue(osc_ctx *ctx, const osc_mesh3d *mesh, const int n[3], int64_t np,
     TRY(freespace_opt<double, double>(ctx, j, rho));
     {
         Launch L_(ctx, "interp_f64");
-        if (launch_interp_vec4<double>(ia, E4, E, ctx->d_small + 2, ctx->stream, at_cathode ? nullptr : B, j.bcoef))
+        if (launch_interp_vec4(ia, E4, E, ctx->d_small + 2, ctx->stream, at_cathode ? nullptr : B, j.bcoef))
             return set_err(ctx, OSC_E_CUDA, "interp");
     }
     if (j.B4) {
         Launch L_(ctx, "interp_f64");
-        if (launch_interp_vec4<double>(ia, j.B4, nullptr, ctx->d_small + 3, ctx->stream, B, j.bcoef))
+        if (launch_interp_vec4(ia, j.B4, nullptr, ctx->d_small + 3, ctx->stream, B, j.bcoef))
             return set_err(ctx, OSC_E_CUDA, "interp");
     }
     return OSC_OK;

@@ -278,9 +278,8 @@ __device__ __forceinline__ bool locate(const InterpArgs &a, double x, double y, 
 // field is v (space_charge_3d, code/open_spacecharge_mod.f90:456-461): B on the grid is
 // proportional to E there, so gathering it would only repeat the gather of E (FP64 step, 128^3 and
 // 4e6 particles: 998 us with B planes and their gather, 655 without).
-template <typename TO>
-__device__ __forceinline__ void store_rows(const TO *ws, int64_t m0, int64_t np, int lane, TO *__restrict__ E,
-                                           TO *__restrict__ B, double bcoef) {
+__device__ __forceinline__ void store_rows(const double *ws, int64_t m0, int64_t np, int lane, double *__restrict__ E,
+                                           double *__restrict__ B, double bcoef) {
     const int64_t o0 = 3 * m0, n3 = 3 * np;
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
@@ -289,37 +288,28 @@ __device__ __forceinline__ void store_rows(const TO *ws, int64_t m0, int64_t np,
         if (E) E[o0 + e] = ws[e];
         if (B) {
             const int c = e % 3;
-            B[o0 + e] = c == 0 ? (TO)(-bcoef * ws[e + 1]) : (c == 1 ? (TO)(bcoef * ws[e - 1]) : (TO)0);
+            B[o0 + e] = c == 0 ? -bcoef * ws[e + 1] : (c == 1 ? bcoef * ws[e - 1] : 0.0);
         }
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void load_node(const vec4<T> *g, int64_t n, double &a, double &b, double &c) {
-    if constexpr (sizeof(T) == 8) {  // one 256-bit load per node
-        double w;
-        asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(w) : "l"(g + n));
-    } else {
-        const vec4<T> v = __ldg(g + n);
-        a = (double)v.x;
-        b = (double)v.y;
-        c = (double)v.z;
-    }
+__device__ __forceinline__ void load_node(const double4 *g, int64_t n, double &a, double &b, double &c) {
+    double w;  // one 256-bit load per node
+    asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(w) : "l"(g + n));
 }
 
 // Two lanes to a particle, the even lane the four nodes at i and the odd lane those at i + 1: the
 // two 32-byte nodes of a row are adjacent, so that both loads travel as one request.  Bound by the
 // sectors the L1 and L2 hand out; 4e6 particles on 128^3: 169 us with one lane to a particle, 146 with
 // two, 140.5 on 16 CTAs per SM instead of 64.
-template <typename T, typename TO>
-__global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T> *__restrict__ g, TO *__restrict__ E,
-                                                     TO *__restrict__ B, double bcoef,
+__global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const double4 *__restrict__ g,
+                                                     double *__restrict__ E, double *__restrict__ B, double bcoef,
                                                      unsigned long long *__restrict__ nclamp) {
     // E goes through a per-warp shared-memory stage and is stored as contiguous rows (as in
     // k_interp_pairs); the loop runs while the warp's first particle exists
-    __shared__ TO stage[256 * 3];
+    __shared__ double stage[256 * 3];
     const int lane = threadIdx.x & 31;
-    TO *ws = stage + (threadIdx.x - lane) * 3;
+    double *ws = stage + (threadIdx.x - lane) * 3;
     const int64_t plane = (int64_t)a.nx * a.ny;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     pdl_wait(g);
@@ -348,7 +338,7 @@ __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T>
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     double vx, vy, vz;
-                    load_node<T>(g, nodes[q], vx, vy, vz);
+                    load_node(g, nodes[q], vx, vy, vz);
                     v[r][0] += vx * wts[q];
                     v[r][1] += vy * wts[q];
                     v[r][2] += vz * wts[q];
@@ -361,7 +351,7 @@ __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T>
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 const double e = v[r][d] + __shfl_xor_sync(0xffffffffu, v[r][d], 1);
-                if ((d == 1) == (lane & 1)) ws[3 * src + d] = (TO)e;
+                if ((d == 1) == (lane & 1)) ws[3 * src + d] = e;
             }
         }
         count_one(nclamp, fl);
@@ -371,16 +361,13 @@ __global__ void __launch_bounds__(256) k_interp_vec4(InterpArgs a, const vec4<T>
     }
 }
 
-template <typename T>
 int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp, cudaStream_t st,
                        double *B, double bcoef) {
     if (a.np <= 0) return OSC_OK;
-    launch_pdl(k_interp_vec4<T, double>, dim3(nblocks(a.np, 256, 148 * 16)), dim3(256), 0, st, a,
-               reinterpret_cast<const vec4<T> *>(E4), E, B, bcoef, nclamp);
+    launch_pdl(k_interp_vec4, dim3(nblocks(a.np, 256, 148 * 16)), dim3(256), 0, st, a,
+               reinterpret_cast<const double4 *>(E4), E, B, bcoef, nclamp);
     return ok();
 }
-template int launch_interp_vec4<double>(const InterpArgs &, const void *, double *, unsigned long long *, cudaStream_t,
-                                        double *, double);
 
 // Three double planes [3][N], reference order of the 8-term sum per component.
 __global__ void __launch_bounds__(256) k_interp_planes(InterpArgs a, const double *__restrict__ F,

@@ -76,7 +76,7 @@ int launch_quad_to_nodes(const float *quad, float *rho, int nx, int ny, int nz, 
 
 // CIC gather (interpolate_field, code/open_spacecharge_mod.f90:311-390): clamp cells to
 // [1, nhi-1] (and the array), weights computed after clamping, 8-node sum in the
-// reference's order.  Source: a vec4<T> interleaved grid or three double planes.
+// reference's order.  Source: a double4 grid, an x-pair grid or three double planes.
 struct InterpArgs {
     int64_t np;
     const double *x, *y, *z;
@@ -89,7 +89,6 @@ struct InterpArgs {
     int ctas = 0;
 };
 // The gathers from a grid write E (when not null) and/or B = bcoef (-E_y, E_x, 0) (when not null).
-template <typename T>
 int launch_interp_vec4(const InterpArgs &a, const void *E4, double *E, unsigned long long *nclamp,
                        cudaStream_t st, double *B = nullptr, double bcoef = 0);
 int launch_interp_planes(const InterpArgs &a, const double *F, double *out,
