@@ -130,7 +130,8 @@ OSC_API int osc_ctx_get_option(osc_ctx *ctx, int option, int64_t *value);
 OSC_API int osc_ctx_synchronize(osc_ctx *ctx);
 /* Launch shapes chosen by an autotuner (openspacecharge_b200.autotune times the candidates
  * on the GPU and keeps the winners in a JSON cache keyed by GPU, kernel and length); no
- * reference counterpart.  Keys and values (0 restores the built-in default):
+ * reference counterpart.  Keys and values (0 restores the built-in default, except of
+ * "zconv_engine", whose default is 2; a key that was not set reads as its default):
  *   "deposit_run", "gather_run": particles per lane of the cell-ordered deposit and gather
  *     (4 or 8);
  *   "deposit_ctas_per_sm", "gather_ctas_per_sm", "deposit_runs_ctas_per_sm",
@@ -140,9 +141,9 @@ OSC_API int osc_ctx_synchronize(osc_ctx *ctx);
  *     that doubled length; "r2c_nl_div:..." and "c2r_nl_div:..." the rows per CTA of the
  *     forward and inverse x transforms;
  *   "zconv_engine:<f32|f64>:L<length>": the free-space z pass of that doubled z length on
- *     the radix warp engine (0), the one-exchange 16 x 32 engine (1, FP32 length 512 only),
- *     or the warp engine with CTAs that pair the rows ky and Ny - ky and fetch their common
- *     Green columns once (2);
+ *     the radix warp engine (0), the one-exchange 16 x 32 engine (1, FP32 length 512 only,
+ *     elsewhere as 0), or the warp engine with CTAs that pair the rows ky and Ny - ky and
+ *     fetch their common Green columns once (2, the default);
  *   "batch_copy_chunks": chunks of bunches the FP32 osc_batch_space_charge_step (host
  *     arrays) copies in, solves and copies out in a pipeline (1 to 16; 1: one copy in, one
  *     batched step, one copy out);

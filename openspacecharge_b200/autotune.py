@@ -7,8 +7,9 @@ Every choice gives identical results; only the time changes.  The tuned shapes a
 * the lines per CTA of the y transforms of each doubled length ("lines_nl_div:<prec>:L<n>":
   the widest tile that fits, or half of it), and the rows per CTA of the x transforms
   ("r2c_nl_div", "c2r_nl_div");
-* the transform engine of the z pass at doubled length 512 (the radix-8-8-8 warp engine, or
-  one exchange per transform with a 16 x 32 split);
+* the engine of the z pass of each doubled length ("zconv_engine:<prec>:L<n>": one warp per
+  column, rows ky and Ny - ky paired, or at the FP32 length 512 one exchange per transform
+  with a 16 x 32 split);
 * the line-pair tile of the Green build's even/odd transforms of each doubled length
   ("sym_nl_div", tuned where the spectra are rebuilt: the refit case and the batch).
 
@@ -26,7 +27,7 @@ import tempfile
 
 from .native import OPT_PARTICLE_ORDER, OPT_PROFILE, ORDER_ANY, PREC_FP32
 
-# candidate values per key family (0 = the built-in default)
+# candidate values per key family (0 = the built-in default; of zconv_engine it is 2)
 CTAS = [0, 8, 32, 128]
 RUNS = [4, 8]
 

@@ -164,7 +164,7 @@ int osc_ctx_set_tuning(osc_ctx *ctx, const char *key, int value) {
     if (!ctx || !key) return OSC_E_INVALID;
     const std::string k(key);
     if (!tuning_value_ok(k, value)) return set_err(ctx, OSC_E_INVALID, "tuning %s = %d is not a valid choice", key, value);
-    if (value == 0) ctx->tuning.erase(k);  // the built-in default
+    if (value == tune_default(key)) ctx->tuning.erase(k);
     else ctx->tuning[k] = value;
     ++ctx->tune_gen;
     return OSC_OK;
@@ -172,7 +172,7 @@ int osc_ctx_set_tuning(osc_ctx *ctx, const char *key, int value) {
 
 int osc_ctx_get_tuning(osc_ctx *ctx, const char *key, int *value) {
     if (!ctx || !key || !value) return OSC_E_INVALID;
-    *value = tune_get(ctx, key);
+    *value = tune_get(ctx, key, tune_default(key));
     return OSC_OK;
 }
 

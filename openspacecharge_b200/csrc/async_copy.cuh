@@ -12,7 +12,9 @@
 namespace osc {
 
 // Fault codes written by kernels to the context's host-mapped fault word.
-constexpr unsigned FAULT_BULK_WAIT = 1u;  // a bulk copy did not complete within the poll limit
+// A bulk copy did not complete within the poll limit, in the z pass with one warp per column, with
+// rows paired (images included), with one exchange per transform.
+constexpr unsigned FAULT_BULK_WAIT = 1u, FAULT_BULK_WAIT_PAIRED = 2u, FAULT_BULK_WAIT_EXCHANGE = 3u;
 
 constexpr unsigned MBAR_POLL_LIMIT = 1u << 22;
 

@@ -201,11 +201,12 @@ int tune_get(const osc_ctx *c, const char *key, int def) {
     auto it = c->tuning.find(key);
     return it == c->tuning.end() ? def : it->second;
 }
-int tune_len(const osc_ctx *c, const char *family, size_t tbytes, int len) {
-    if (c->tuning.empty()) return 0;
+int tune_default(const char *key) { return strncmp(key, "zconv_engine:", 13) == 0 ? ZCONV_PAIRED : 0; }
+int tune_len(const osc_ctx *c, const char *family, size_t tbytes, int len, int def) {
+    if (c->tuning.empty()) return def;
     char key[64];
     snprintf(key, sizeof(key), "%s:%s:L%d", family, tbytes == 4 ? "f32" : "f64", len);
-    return tune_get(c, key);
+    return tune_get(c, key, def);
 }
 
 int prof_flush(osc_ctx *c) {

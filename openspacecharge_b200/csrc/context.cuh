@@ -153,7 +153,9 @@ int prof_flush(osc_ctx *c);
 // Tuned value of `key` (autotuner), or def when none was set; tune_len: of the key
 // "<family>:<f32|f64>:L<length>".
 int tune_get(const osc_ctx *c, const char *key, int def = 0);
-int tune_len(const osc_ctx *c, const char *family, size_t tbytes, int len);
+int tune_len(const osc_ctx *c, const char *family, size_t tbytes, int len, int def = 0);
+// The value of `key` that stands for the built-in choice.
+int tune_default(const char *key);
 
 // Green-spectrum cache.  A budget of 0 disables it: every solve rebuilds its spectra (the
 // reference's behaviour, code/open_spacecharge_mod.f90:570-573) into reused buffers.

@@ -110,6 +110,11 @@ __device__ __forceinline__ cplx<T> g_lookup(const GSpecDev &g, int kx, int ky, i
     return v;
 }
 
+// Kernels of the z pass with staged spectra, the values of the tuning key zconv_engine: one warp per
+// column; one exchange per transform (FP32 length 512, else as 0); rows ky and Ny - ky paired, the
+// default (where it does not apply, as 0).
+constexpr int ZCONV_RADIX = 0, ZCONV_EXCHANGE = 1, ZCONV_PAIRED = 2;
+
 // Fused z pass of the free-space convolution: forward transform of each (kx,ky) column
 // (nz non-zero planes, length Nz), multiply by stored Green spectra (optionally adding the
 // mirrored-image term), inverse transform, keep z in [0, nz) of every output.
@@ -133,9 +138,7 @@ struct ZConvArgs {
     unsigned poll_limit;  // polls of a bounded mbarrier wait (0: MBAR_POLL_LIMIT)
     int skip_copies;      // test only: arm the Green-column barrier but issue no bulk copy,
                           // so the bounded wait runs out and the fault path is exercised
-    int engine;           // staged spectra (tuning key zconv_engine): 0 and 2 rows ky and Ny - ky
-                          // paired where that applies, 1 one warp per column (at the FP32
-                          // length 512 the one-exchange 16 x 32 engine)
+    int engine;           // staged spectra (tuning key zconv_engine): ZCONV_RADIX, ..
     // batches of equal grids (blockIdx.y = member): input, output and spectrum offsets of
     // member b are b*in_bstride, b*out_bstride and b*g_bstride (elements of the spectrum)
     int nbatch;
@@ -143,7 +146,7 @@ struct ZConvArgs {
     // > 0: the nsum members are the inputs of the single output (warp engine, staged real
     // spectra): out = inverse of sum_s spectrum[gdir[s]] x forward(input s)
     int nsum;
-    // global index of local column 0 (a z slab's share of the columns, warp engine 0): the
+    // global index of local column 0 (a z slab's share of the columns, ZCONV_RADIX): the
     // Green spectra are read at column col_base + col, input and output at col
     int col_base;
 };

@@ -1127,16 +1127,16 @@ int launch_zconv(const cplx<T> *in, cplx<T> *out, const ZConvArgs &a, const TwPa
         const bool staged = !img && zconv_can_stage<T>(a);
         if (a.nsum > 0 && (img || !staged || a.nout != 1)) return OSC_E_UNSUPPORTED;
         if constexpr (sizeof(T) == 4) {
-            if (L == 512 && staged && a.nsum == 0 && a.out_estride == 1 && a.engine == 1 && whole &&
+            if (L == 512 && staged && a.nsum == 0 && a.out_estride == 1 && a.engine == ZCONV_EXCHANGE && whole &&
                 zconv_w512_smem<4>(a.nout, a.g[0].zpitch) <= 100 * 1024)
                 return launch_zconv_w512(in, out, a, tw.rt, st);
         }
         // The staged product with Green columns shared by the rows ky and Ny - ky wherever it applies,
-        // unless the caller asks for the other engine (1): it reads half the spectra, and is never the
+        // unless the caller asks for another engine: it reads half the spectra, and is never the
         // slower one.  Paired against one warp per column (us), FP32: 16^3 8.6 10.6, 64^3 18.9 24.4,
         // 64 x 64 x 96 27.1 31.1, 128^3 76.2 81.7, 192 x 192 x 64 113 148, 128 x 128 x 256 138.5 143.9
         // (one exchange 155); FP64: 32^3 10.6 16.9, 128^3 128 137, 96^3 72 97, 128 x 128 x 256 287 326.
-        const bool pair = staged && a.engine != 1 && whole && zconv_img_ok(L, a.nz, (int)sizeof(T)) &&
+        const bool pair = staged && a.engine == ZCONV_PAIRED && whole && zconv_img_ok(L, a.nz, (int)sizeof(T)) &&
                           zconv_pair_can<T>(a);
         return dispatch_warp_len(L, [&](auto eng) -> int {
             using E = decltype(eng);

@@ -622,7 +622,7 @@ int freespace_opt(osc_ctx *c, const FreeSpaceJob &j, const TIn *rho) {
     za.img_phase_mul = nz - 1;
     za.ng = gs->nspec;
     za.fault = c->d_fault;
-    za.engine = tune_len(c, "zconv_engine", sizeof(T), Nz);
+    za.engine = tune_len(c, "zconv_engine", sizeof(T), Nz, ZCONV_PAIRED);
     if (c->test_wait_timeout) {  // test only: waits that must run out quickly
         za.poll_limit = 64;
         za.skip_copies = 1;
@@ -769,6 +769,7 @@ int slab_zpass(osc_ctx *c, const FreeSpaceJob &j, int col0, int ncols, const cpl
     za.ng = gs->nspec;
     for (int i = 0; i < gs->nspec; ++i) za.g[i] = gs->spec[i];
     za.fault = c->d_fault;
+    za.engine = ZCONV_PAIRED;
     za.nbatch = 1;
     Launch L_(c, "fft_z_conv");
     return kerr(c, launch_zconv<float>(in, out, za, twz, c->stream), "z convolution");

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(ZI_WARPS * 32, zi_minb<T, IMG>())
     if (threadIdx.x == 0) {
         const bool ok = mbar_wait_bounded(&gbar, 0, a.poll_limit);
         if (!ok) {
-            report_fault(a.fault, FAULT_BULK_WAIT);
+            report_fault(a.fault, FAULT_BULK_WAIT_PAIRED);
             // let copies in flight land before leaving (bounded as well)
             mbar_wait_bounded(&gbar, 0, a.poll_limit);
         }

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(W * 32, 6) k_zconv_w512(const float2 *__restri
     if (threadIdx.x == 0) {
         const bool ok = mbar_wait_bounded(&gbar, 0, a.poll_limit);
         if (!ok) {
-            report_fault(a.fault, FAULT_BULK_WAIT);
+            report_fault(a.fault, FAULT_BULK_WAIT_EXCHANGE);
             mbar_wait_bounded(&gbar, 0, a.poll_limit);
         }
         gfail = ok ? 0 : 1;

@@ -231,7 +231,7 @@ class Context:
         return int(v.value)
 
     def set_tuning(self, key: str, value: int) -> None:
-        """Launch shape `key` (see osc_ctx_set_tuning); 0 restores the default."""
+        """Launch shape `key` (see osc_ctx_set_tuning); 0 restores the default ("zconv_engine": 2)."""
         self.call("osc_ctx_set_tuning", key.encode(), int(value))
 
     def get_tuning(self, key: str) -> int:
