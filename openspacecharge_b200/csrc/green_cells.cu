@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128) k_cell_series(CellGeom *__restrict__ gs, 
 }
 int launch_cell_series(CellGeom *g, int n, cudaStream_t st) {
     if (n <= 0) return OSC_OK;
-    k_cell_series<<<n, 128, 0, st>>>(g, kSerRatio);
+    k_cell_series<<<n, 128, 0, st>>>(g, ser_ratio<float>());
     return ok();
 }
 

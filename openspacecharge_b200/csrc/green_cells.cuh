@@ -19,10 +19,15 @@ namespace osc {
 constexpr int kSerN = 4;                       // highest degree (order 8 in 1/r)
 constexpr int kSerC = 35;                      // monomials u^i v^j w^k, i + j + k <= 4
 constexpr int kSerP = 36;                      // the same, padded to whole 16-byte pairs
-// Distance, in half cell diagonals, from which the series is used.  There its truncation error (3e-10
-// of the value for the most elongated cells, 7e-12 for cubes, falling as r^-10) meets the round-off
-// that the corner difference has by then; FP32 spectra keep 6e-8.
-constexpr double kSerRatio = 9.0;
+// Distance, in half cell diagonals, from which the series is used, by the type of the stored spectra.
+// The series' truncation falls as r^-10, the corner difference's round-off in FP64 grows as r^3.  Largest
+// errors over the directions, of |E| (series, corners), at 9, 10 and 11: cubes 4.0e-12 1.3e-12, 1.6e-12
+// 1.1e-12, 4.9e-13 1.9e-12; cells 1 x 1 x 10 8.2e-11 9.2e-11, 4.4e-11 3.5e-11, 1.3e-11 6.8e-11;
+// 1 x 10 x 10 2.3e-11 9.7e-12, 8.0e-12 1.8e-11, 3.1e-12 5.2e-11; 1 x 3 x 10 3.9e-11 9.3e-12, 2.1e-11
+// 2.8e-11, 5.5e-12 3.4e-11; 1 x 1 x 50 9.9e-11 7.7e-9 and better from there.  So 11 for FP64: no
+// shape of cell has the series where the corners would be the better one.  FP32 spectra keep 6e-8 of
+// a value, and 9 spares them near tiles.
+template <typename T> constexpr double ser_ratio() { return sizeof(T) == 8 ? 11.0 : 9.0; }
 
 // Position of u^i v^j w^k in Horner order (i, then j, then k), all degrees <= kSerN.
 constexpr __host__ __device__ int ser_idx(int i, int j, int k) {

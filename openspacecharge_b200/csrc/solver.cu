@@ -194,7 +194,7 @@ static int green_sym_set(osc_ctx *c, int nx, int ny, int nz, const double delta[
         ca.hstride = (int64_t)nx * ny * nz;
         Launch L_(c, "green_cells");
         TRY(kerr(c, launch_green_cells<T>(h, ca, cell_geom(delta[0], delta[1], delta[2] * gamma, gamma, 0.0,
-                                                           kSerRatio), c->stream),
+                                                           ser_ratio<T>()), c->stream),
                  "green cells"));
     }
     const int zp = zinner ? green_zpitch(nz + 1, sizeof(T)) : nz + 1;
@@ -260,7 +260,7 @@ static int green_zoff_set(osc_ctx *c, int nx, int ny, int nz, const double delta
         ca.hstride = (int64_t)nx * ny * Nz;
         Launch L_(c, "green_cells");
         TRY(kerr(c, launch_green_cells<double>(h, ca, cell_geom(delta[0], delta[1], delta[2] * gamma, gamma,
-                                                                zoff * gamma, kSerRatio), c->stream),
+                                                                zoff * gamma, ser_ratio<T>()), c->stream),
                  "green cells"));
     }
     int odd[3][2] = {{0, 0}, {0, 0}, {0, 0}};
