@@ -208,10 +208,15 @@ bool zconv_warp_ok(int L, int nz, int elem_bytes);
 // kz-outermost for the CTA one.  staged: all spectra real and even or odd in z (a kernel without an
 // offset, and its images), whose columns the warp kernels stage in shared memory.  The others are read
 // complex and in full from global memory, and at the doubled lengths 32 and 64 a warp per column
-// has too few bytes in flight for that: 128 x 128 x 32 displaced, with images, takes 181 us in FP32 and
-// 340 in FP64 with a warp per column, 92 and 177 with CTAs of eight columns (128 x 128 x 16 132 and 330
-// against 72 and 162; a pipe on 128 x 64 x 32 FP64 73).  Lengths from 96 on keep the warps.
-bool zconv_zinner(int L, int nz, int elem_bytes, bool staged);
+// has too few bytes in flight for that: the z pass of 128 x 128 x 32 displaced, with images, takes 181 us
+// in FP32 and 340 in FP64 with a warp per column, 92 and 177 with CTAs of eight columns.  Few columns
+// leave such CTAs too few to fill the SMs, and the kz-innermost layout serves short y and x lines
+// better: whole solves (warps, CTAs) with B and images on 32 x 32 x 32 (2112 columns) 51.5 and 68.4
+// us in FP32, 68.4 and 77.6 in FP64; 40 x 40 x 32 (3280) 92 103, 113 115; 64 x 32 x 32 (4160) 68 83, 89
+// 82; 48 x 48 x 32 (4704) 73 80, 100 93; 64 x 64 x 32 (8320) 105 92, 159 108; 128 x 128 x 32 (33024) 328
+// 224, 556 356.  So up to 7168 columns in FP32 and half as many in FP64 keep the warps, and so do
+// lengths from 96 on.
+bool zconv_zinner(int L, int nz, int elem_bytes, bool staged, int64_t columns);
 // True when the cathode-image z pass (zconv_img.cuh) covers length L: the warp-per-column
 // lengths whose first-stage butterfly count L/R is a multiple of 32 or below 32.
 bool zconv_img_ok(int L, int nz, int elem_bytes);

@@ -58,8 +58,8 @@ bool zconv_warp_ok(int L, int nz, int elem_bytes) {
     if ((elem_bytes != 4 && elem_bytes != 8) || 2 * nz != L) return false;
     return dispatch_warp_len(L, [](auto eng) -> int { return decltype(eng)::kLen > 0 ? 1 : 0; }) != 0;
 }
-bool zconv_zinner(int L, int nz, int elem_bytes, bool staged) {
-    return zconv_warp_ok(L, nz, elem_bytes) && (staged || L >= 96);
+bool zconv_zinner(int L, int nz, int elem_bytes, bool staged, int64_t columns) {
+    return zconv_warp_ok(L, nz, elem_bytes) && (staged || L >= 96 || columns * elem_bytes <= 28 * 1024);
 }
 bool zconv_img_ok(int L, int nz, int elem_bytes) {
     if (!zconv_warp_ok(L, nz, elem_bytes)) return false;

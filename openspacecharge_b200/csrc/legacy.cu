@@ -341,7 +341,8 @@ template <typename T> static int pipe_comb(osc_ctx *c, const LGeom &g) {
         TRY(kchk(c, launch_green_extract<T>(reinterpret_cast<const double2 *>(p.g[t].p),
                                             reinterpret_cast<char *>(p.comb.p) + t * each, nx, g.period[0],
                                             g.period[1], g.period[1], g.period[2], 0, 0, PIPE_SIGN[t] * factr,
-                                            zconv_zinner(g.period[2], g.n[2], (int)sizeof(T), false)
+                                            zconv_zinner(g.period[2], g.n[2], (int)sizeof(T), false,
+                                                         (int64_t)(g.n[0] + 1) * g.period[1])
                                                 ? green_zpitch(g.period[2], sizeof(cplx<T>))
                                                 : 0,
                                             c->stream),
@@ -441,7 +442,7 @@ static int pipe_phi_opt(osc_ctx *c, const LGeom &g, const double *rho, double *p
         s.par_y = s.par_z = 1;
         s.dimy = Ny;
         s.dimz = Nz;
-        s.zinner = zconv_zinner(Nz, nz, (int)sizeof(T), false) ? 1 : 0;
+        s.zinner = zconv_zinner(Nz, nz, (int)sizeof(T), false, (int64_t)nxh * Ny) ? 1 : 0;
         s.zpitch = s.zinner ? green_zpitch(Nz, sizeof(V)) : Nz;
     }
     {

@@ -410,7 +410,7 @@ static int green_set(osc_ctx *c, const FreeSpaceJob &j, const int *comps, int nc
     gs.key = key;
     const int nsets = j.at_cathode ? 2 : 1;
     const bool displaced = j.offset[0] != 0.0 || j.offset[1] != 0.0 || j.offset[2] != 0.0;
-    const int zinner = zconv_zinner(2 * j.nz, j.nz, (int)sizeof(T), !displaced) ? 1 : 0;
+    const int zinner = zconv_zinner(2 * j.nz, j.nz, (int)sizeof(T), !displaced, (int64_t)(j.nx + 1) * 2 * j.ny) ? 1 : 0;
     for (int s = 0; s < nsets; ++s) {
         double off[3] = {j.offset[0], j.offset[1], j.offset[2]};
         if (s == 1) off[2] = off[2] + j.img_zoff;
