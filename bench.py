@@ -791,7 +791,7 @@ def run_batch(args, ws, rank, local, dist):
     roof = {"kernel": "whole batched step (per-bunch deposit, Green build, field, gather)", "bound": "hbm",
             "achieved": ach, "peak": hbm_peak, "unit": "GB/s", "frac": ach / hbm_peak,
             "peak_source": peak_src, "traffic": None, "alg_bytes_per_step": alg,
-            "note": "the FP64 IGF corner primitives of the Green build are FP64-pipe bound, not HBM bound"}
+            "note": "the FP64 cell integrals of the Green build are FP64-pipe bound, not HBM bound"}
     cpu = None
     if rank == 0 and ws == 1 and not args.no_cpu:
         cpu = cpu_baseline_batch(grids, counts, charges, sb, x, y, z)

@@ -1,5 +1,6 @@
 // fft_kernels_impl.cuh -- batched shared-memory FFT kernels for the IGF convolution (sm_100a).
-// Included by fft_kernels_f32.cu and fft_kernels_f64.cu, which instantiate one precision each.
+// Included by the fft_*_f32.cu and fft_*_f64.cu files, which instantiate one family of kernels in one
+// precision each.
 //
 // The free-space solve runs as five kernels over HBM (FP32 path, G spectra cached):
 //   k_r2c_rows  x: real rho rows -> half spectra (two rows packed per complex line)
