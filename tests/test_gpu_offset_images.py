@@ -1,5 +1,5 @@
 """space_charge_3d with a displaced kernel and cathode images together (the offset adds to the
-image's own displacement, code/open_spacecharge_mod.f90:466-489): neither set of spectra is even
+image's own displacement, code/open_spacecharge_mod.f90:472): neither set of spectra is even
 or odd along z then, at the lengths that have an image z pass and at others, along z alone and along
 every axis, against the FP64 oracle (tolerances as in the other free-space comparisons)."""
 import numpy as np

@@ -1,5 +1,5 @@
 """B of the FP32 pipe step: gathered from FP64 differences of the potential, not from E as it is
-rounded to FP32 for its own gather.  B = beta/c (-E_y, E_x, 0) (code/open_spacecharge_core_mod.f90:456-461),
+rounded to FP32 for its own gather.  B = beta/c (-E_y, E_x, 0) (as in code/open_spacecharge_mod.f90:456-461),
 so B and E of one call differ by E's FP32 rounding and no more: within 2^-23 of the component's
 largest value, and, at most of the particles, by more than FP64 round-off."""
 import numpy as np
